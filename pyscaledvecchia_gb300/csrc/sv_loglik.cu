@@ -16,8 +16,9 @@
 // sv_vecchia_loglik): every block carries its problem index, so one launch of
 // the block kernel processes the blocks of all problems.
 //
-// Kernels: k_prob_params (theta -> per-problem parameters), k_block_warp (one
-// warp per block, K <= 32), k_block_cta (one CTA per block, K > 32),
+// Kernels: k_prob_params (theta -> per-problem parameters), k_block_fix
+// (sv_loglik_fix.cu: nu = 3/2 and 5/2, K <= 32), k_block_warp (one warp per
+// block, K <= 32, what the former does not take), k_block_cta (one CTA per block, K > 32),
 // k_chunk_max / fix-up pass (reference chunk-wide jitter), k_reduce1 /
 // k_final1 (GLS + Fisher sums, beta), k_reduce2 / k_final2 (ll, score,
 // variance penalty).  Reductions are in a fixed order, so results are bitwise
@@ -131,6 +132,20 @@ __global__ void k_prob_params(const sv_prob_desc* descs, const double* theta, in
       if (D.estimate_nu) mf.dtab = (const float4*)(mm.tab + kDtabOff);
     }
     I.mf32 = mf;
+    // fixed-point kernel: nu = 3/2 or 5/2, its sizes, and a scale with room
+    // for its results' exponents
+    I.fix_ek = -1;
+    I.fix_diag = 0;
+    I.fix_sig = I.fix_rsig = 1.0;
+    if ((mm.closed == 1 || mm.closed == 2) && d <= kFixMaxD && d + 2 + D.q <= kFixCols && I.s2 > 1e-200 &&
+        I.s2 < 1e200 && I.tau >= 0.0 && I.tau <= 1e6) {
+      int ek = 0;
+      while ((double)(1ll << ek) < 1.0 + I.tau) ++ek;  // (1 + tau) 2^-ek in (1/2, 1]
+      I.fix_ek = ek;
+      I.fix_diag = (1ll << (58 - ek)) + llrint(ldexp(I.tau, 58 - ek));
+      I.fix_sig = sqrt(ldexp(I.s2, ek));
+      I.fix_rsig = 1.0 / I.fix_sig;
+    }
   }
   for (int l = threadIdx.x; l < d; l += blockDim.x) I.invlam[l] = exp(-th[1 + l]);
 }
@@ -860,6 +875,7 @@ namespace {
 struct EvalShape {
   int64_t nprob, nblk, nx, nblk_max;
   int dmax, qmax, Pmax, kmax, need_grad, any_est, precision;
+  int fix;   // some problem may run on the fixed-point kernel (float64 form)
   int tabs;  // a Matern table per problem (problems of fixed general nu fill theirs)
 };
 
@@ -1041,6 +1057,7 @@ int run_eval(const EvalCall& C, cudaStream_t st, const ShardStage* sh = nullptr)
   A.redo_mode = 0;
   A.rho_min = C.rho_min > 0.0 ? C.rho_min : 1e-4;
   A.xhl = (float2*)(ws + W.xhl);
+  A.qmax = S.qmax;
   A.kcap = S.kmax + 1 < 32 ? (S.kmax + 1 > 0 ? S.kmax + 1 : 1) : 32;
 
   // the blocks of this call: all, or those of the shard's partitions
@@ -1063,6 +1080,11 @@ int run_eval(const EvalCall& C, cudaStream_t st, const ShardStage* sh = nullptr)
   const int lanes = C.team_lanes > 0 ? C.team_lanes : 16;
   if (split && lanes != 4 && lanes != 8 && lanes != 16 && lanes != 32) return SV_EINVAL;
 
+  // float64 form: the fixed-point kernel first where a problem may be its
+  // (10.2 ms against 27.3 ms for the float64 kernels, measured at 200,000
+  // blocks of 31, d = 10), then the float64 kernels over the blocks it flagged
+  const bool fix = !split && S.fix;
+
   // list ranges: the warp-kernel blocks are [0, nwarp) (or wlist), the CTA
   // blocks the rest; a shard (one problem, no lists) takes its part of each
   auto warp_pass = [&](LikArgs B) -> int {
@@ -1073,6 +1095,7 @@ int run_eval(const EvalCall& C, cudaStream_t st, const ShardStage* sh = nullptr)
     if (B.b1 <= B.b0) return SV_OK;
     if (split && !B.redo_mode)
       return S.precision == 1 ? launch_block_split(B, lanes, st) : launch_block_split_df(B, lanes, st);
+    if (fix && !B.redo_mode && !B.fixup) return launch_block_fix(B, max_smem_optin(), st);
     return launch_warp_kernel(B, st);
   };
   auto cta_pass = [&](LikArgs B) -> int {
@@ -1116,6 +1139,11 @@ int run_eval(const EvalCall& C, cudaStream_t st, const ShardStage* sh = nullptr)
       if (rc != SV_OK) return rc;
     }
     if ((rc = warp_pass(A)) != SV_OK) return rc;
+    if (fix && C.nwarp > 0) {
+      LikArgs B = A;
+      B.redo_mode = 1;
+      if ((rc = warp_pass(B)) != SV_OK) return rc;
+    }
     if ((rc = cta_pass(A)) != SV_OK) return rc;
     // the largest jitter level of every chunk (of this call's blocks)
     if (C.chunked && bhi > blo) {
@@ -1213,6 +1241,8 @@ EvalShape single_shape(const sv_loglik_desc* D) {
   // a fixed nu without a closed form, or an estimated nu: its Matern is
   // interpolated from tables (built if the evaluation's nu is in their range)
   S.tabs = (D->estimate_nu || mtab_ok(D->nu)) ? 1 : 0;
+  const int code = D->estimate_nu ? -1 : matern_closed_code(D->nu);
+  S.fix = (code == 1 || code == 2) && D->d <= kFixMaxD && D->d + 2 + D->q <= kFixCols;
   return S;
 }
 
@@ -1230,6 +1260,7 @@ EvalShape batch_shape(const sv_batch_desc* B) {
   S.any_est = B->any_estimate_nu;
   S.precision = B->precision;
   S.tabs = B->general_nu ? 1 : 0;
+  S.fix = 1;  // decided per problem on the device
   return S;
 }
 

@@ -26,6 +26,12 @@ struct ProbInfo {
   double dg, s2t;  // s2 (1 + tau) and s2 tau
   // double-float split form: s2, s2 (1 + tau) and s2 tau as float32 (hi, lo) pairs
   float s2_hi, s2_lo, dg_hi, dg_lo, s2t_hi, s2t_lo;
+  // fixed-point kernel: Sigma = s2 2^fix_ek times a matrix with diagonal
+  // fix_diag (Q58, in (1/2, 1]); fix_sig = sqrt(s2 2^fix_ek).  fix_ek < 0: a
+  // problem it does not take
+  double fix_sig, fix_rsig;
+  int64_t fix_diag;
+  int32_t fix_ek, fix_pad;
   MaternMode mm;
   MaternF32 mf32;  // the split kernels' float32 Matern (code -1: the float64 pass)
   double invlam[kMaxD];
@@ -56,7 +62,8 @@ struct LikArgs {
   int redo_mode;          // float64 kernel: only blocks flagged by the split kernel
   double rho_min;
   float2* xhl;            // split form: x / lambda as float32 (hi, lo) pairs
-  int kcap;               // split form: largest K of the launch (<= 32)
+  int kcap;               // split form, fixed-point kernel: largest K of the launch (<= 32)
+  int qmax;
 };
 
 // The chunk fix-up pass has work only when some block used jitter
@@ -133,6 +140,13 @@ __host__ __device__ inline int split_slot_doubles(int d, int NR, int kc) {
 // launch_block_split_df: double-float factorisation and solves
 int launch_block_split(const LikArgs& A, int lanes, cudaStream_t st);
 int launch_block_split_df(const LikArgs& A, int lanes, cudaStream_t st);
+
+// the fixed-point kernel over list entries [A.b0, A.b1) (float64 form, all
+// K <= 32); blocks it does not take are flagged for the float64 kernels
+// (A.redo).  maxsm: opt-in shared memory of the device
+constexpr int kFixMaxD = 12;   // dimensions, and
+constexpr int kFixCols = 32;   // right-hand sides (d + 2 + q) it takes
+int launch_block_fix(const LikArgs& A, int maxsm, cudaStream_t st);
 
 // split form: fills A.xhl (X's n * d entries as float2) for every problem
 int launch_split_prep(const LikArgs& A, int64_t nx, cudaStream_t st);

@@ -1,0 +1,545 @@
+// The fixed-point block kernel of the Vecchia likelihood / score / Fisher
+// evaluation: the float64 form's kernel for blocks of at most 32 points with
+// Matern smoothness 3/2 or 5/2 (d <= 12, at most 32 right-hand sides).
+//
+// Same per-block record as k_block_warp (likelihood.py:111-144 of the
+// reference), from arithmetic at least as fine as float64's: every quantity
+// with a known bound is a 64-bit integer in units of 2^-58 or so of that bound
+// (sv_fix.cuh). k_block_warp is bound by the float64 pipe (64 cycles per warp
+// instruction and scheduler, 2,310 of them per block of 31); here the pipe is
+// left with the coordinate differences and the conversion of the results, and
+// the work is on the integer multiply-adds (2 cycles each).
+//
+//   * coordinates centred on the block's own point, in units of 2^es, 8 times
+//     the block's largest coordinate: r^2 = n_i + n_j - 2 U_i . U_j with an
+//     absolute error of about 2^-61 of the unit's square;
+//   * the covariance is scaled by its own variance and a power of two,
+//     Sigma = s2 2^ek (M 2^-ek + tau 2^-ek I), so that its diagonal lies in
+//     (1/2, 1] and its Cholesky factor's entries are below 1 whatever the
+//     conditioning: the backward error of the factorisation is about 2^-57 of
+//     the diagonal, where float64's is about K 2^-53;
+//   * the factor's inverse T comes with it (fix_factor): its last row is
+//     a = C^-T e_K, and the solves W = C^-1 V are products with T;
+//   * dSigma_l a as one matrix product with the pairs' g: for every input,
+//     sum_j g_ij (U_i - U_j)^2 a_j = U_i^2 (G a)_i - 2 U_i (G aU)_i +
+//     (G aU^2)_i, U in units of the input's own extent in the block;
+//   * rows of T, right-hand sides and solutions carry power-of-two scales.
+//
+// Measured at n = 200,000, d = 10, m = 30: 10.2 ms, where k_block_warp takes
+// 27.3 ms; the integer multiply pipe is 65 % busy, the float64 pipe 6 %
+// (3 warps per scheduler, one block of 18 KB of shared memory each). Errors
+// against 113-bit arithmetic at n = 500 are those of the float64 form or
+// smaller (tau = 1e-2: log-likelihood 7e-16 against 1.4e-15, beta 2.3e-15
+// against 9.2e-15; tau = 1e-8 at d = 3: 8.5e-10 against 1.4e-9).
+//
+// What has no such bound goes to the float64 kernels: a block with a pivot
+// below 2^-34 of the diagonal (its jitter ladder is theirs), coordinates
+// beyond 32 ranges of the block's own point, non-finite or huge data, another
+// smoothness. The choice depends on the block and its problem alone, so a
+// block has the same bits in every launch that holds it.
+#include "sv_fixblock.cuh"
+
+namespace sv {
+
+constexpr int kFixThreads = 384;
+constexpr int kFixV = 4;  // inputs per pass over the pairs' g
+
+__device__ __forceinline__ double pow2(int n) {
+  return n < -1022 ? 0.0 : __longlong_as_double((long long)(min(n, 1023) + 1023) << 52);
+}
+
+// shared memory of one team, in 8-byte words.  rs: words per point of the
+// coordinates (padded to a multiple of 4 inputs) and of the right-hand sides
+// that replace them; 2 more than a multiple of 4, so that eight lanes' 16-byte
+// loads of the same entries of consecutive points meet all banks once
+__host__ __device__ inline int fix_g_words(int G, int kcap, int ncol) {
+  const int g = kcap * (kcap - 1) / 2, w = (G + 1) * ncol;  // pairs' g, then the solutions
+  return ((g > w ? g : w) + 1) & ~1;
+}
+// products of kFixV inputs with a, then the columns' scales and last rows
+__host__ __device__ inline int fix_p_words(int kcap) {
+  return 2 * kFixV * kcap > 2 * kFixCols ? 2 * kFixV * kcap : 2 * kFixCols;
+}
+__host__ __device__ inline int fix_slot_words(int G, int kcap, int ncol, int rs) {
+  int s = kcap * (G + 2);            // M
+  s += fix_g_words(G, kcap, ncol);
+  s += rs * kcap;                    // coordinates, then right-hand sides
+  s += fix_p_words(kcap);
+  s += 2 * G;                        // a, norms
+  return (s + 1) & ~1;
+}
+
+template <int G>
+struct FixSlot {
+  Fx2* M;
+  Fx2* Gp;   // g of the pairs i > j at i(i-1)/2 + j; then the solutions (column stride kCs)
+  Fx2* cv;   // [point][rs]
+  Fx2* Pm;
+  Fx2* us;
+  int64_t* nrm;
+  int rs;
+};
+
+// Sigma / (s2 2^ek) below the diagonal of M and g: in round r lane i takes
+// the pair (i, i + r mod K), so each unordered pair is met once; two rounds at
+// a time, whose chains of dependent products overlap
+template <int G, int CODE>
+__device__ __forceinline__ void fix_assemble(int K, int d, int tl, int es, int ek, const FixSlot<G>& S,
+                                             const uint64_t* T) {
+  constexpr int St = FixDim<G>::kSt;
+  Fx2 ui[kFixMaxD];
+#pragma unroll
+  for (int g = 0; g < kFixMaxD; g += 4)
+    if (g < d) {
+#pragma unroll
+      for (int l = g; l < g + 4; ++l) ui[l] = S.cv[tl * S.rs + l];
+    }
+  const int64_t ni = S.nrm[tl];
+  for (int r = 1; 2 * r <= K; r += 2) {
+    int jj[2];
+    uint64_t s[2], m[2], g[2];
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      int j = tl + r + t;
+      if (j >= K) j -= K;
+      if (2 * (r + t) > K || (2 * (r + t) == K && tl >= r + t)) j = tl;  // no such pair
+      jj[t] = j;
+      const Fx2* uj = S.cv + j * S.rs;
+      int64_t hh = 0, cr = 0;
+#pragma unroll
+      for (int g4 = 0; g4 < kFixMaxD; g4 += 4)
+        if (g4 < d) {
+          Fx2 v[4];
+          load4(uj + g4, v);
+#pragma unroll
+          for (int l = 0; l < 4; ++l) {
+            hh += (int64_t)ui[g4 + l].h * v[l].h;
+            cr += (int64_t)ui[g4 + l].h * v[l].l;
+            cr += (int64_t)ui[g4 + l].l * v[l].h;
+          }
+        }
+      // in [0, 3) 2^62; what rounds below 0 reads as close to 2^64
+      const uint64_t x = (uint64_t)(ni + S.nrm[j]) - ((uint64_t)hh << 1) - (uint64_t)((cr + (1ll << 28)) >> 29);
+      s[t] = x > ~0xfffffull ? 0 : x;
+    }
+#pragma unroll
+    for (int t = 0; t < 2; ++t) fx_matern<CODE>(s[t], es, T, m[t], g[t]);
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+      if (jj[t] != tl) {
+        const int lo = min(tl, jj[t]), hi = max(tl, jj[t]);
+        *(int64_t*)(S.M + lo * St + hi) = (int64_t)((m[t] + (4ull << ek)) >> (3 + ek));
+        S.Gp[hi * (hi - 1) / 2 + lo] = fx_split((int64_t)((g[t] + 4) >> 3));
+      }
+  }
+}
+
+// a right-hand side (this lane's element x, in units 2^-58, its row of T at
+// scale 2^E): stored as split x 2^(E - f), below 1/2, f being the result
+template <int G>
+__device__ __forceinline__ int fix_put_rhs(int64_t x, int E, bool own, Fx2* p) {
+  const int f = team_max<G>(own ? fx_bits(x) + E : -100000) - 57;
+  if (own) *p = fx_split(fx_scale2(x, E - f));
+  return f;
+}
+
+// dSigma_l a for NV inputs l0 .. l0 + NV - 1, in place of their coordinates;
+// fc[l] their scales. FIRST also takes G a. Returns false when a sum does not
+// fit.
+template <int G, int NV, bool FIRST>
+__device__ __forceinline__ bool fix_dsig(int K, int d, int l0, int tl, int es, int E, const FixSlot<G>& S, Fx2 usi,
+                                         int& fc, int64_t& A0) {
+  const bool own = tl < K;
+  Fx2* cv = S.cv + tl * S.rs;
+  Fx2 U[NV];
+  int ex[NV];
+#pragma unroll
+  for (int t = 0; t < NV; ++t) {
+    const int l = l0 + t;
+    const int64_t x = (own && l < d) ? fx_join(cv[l]) : 0;
+    const int len = team_max<G>(fx_bits(x));
+    const int sh = len > 0 ? 58 - len : 0;  // |x| < 2^59
+    ex[t] = es - 3 - sh;
+    U[t] = fx_split(fx_scale2(x, sh));
+    const Fx2 p1 = fx_split(fx_mul(usi, U[t]));
+    const Fx2 p2 = fx_split(fx_mul(p1, U[t]));
+    if (own) {
+      S.Pm[2 * NV * tl + 2 * t] = p1;
+      S.Pm[2 * NV * tl + 2 * t + 1] = p2;
+    }
+  }
+  __syncwarp();
+  FxAcc a0 = {0, 0}, a[2 * NV];
+#pragma unroll
+  for (int t = 0; t < 2 * NV; ++t) a[t] = {0, 0};
+  const int i = own ? tl : 0;
+  const Fx2* pj = S.Pm;
+  const Fx2* row = S.Gp + i * (i - 1) / 2;
+  int off = 0;  // j (j - 1) / 2
+#pragma unroll 2
+  for (int j = 0; j < K; ++j, pj += 2 * NV) {
+    Fx2 g = j > i ? S.Gp[off + i] : row[j < i ? j : 0];
+    if (j == i) g = {0, 0};
+    off += j;
+    if (FIRST) fx_mac(a0, g, S.us[j]);
+#pragma unroll
+    for (int t = 0; t < 2 * NV; t += 4) {
+      Fx2 p[4];
+      load4(pj + t, p);
+#pragma unroll
+      for (int w = 0; w < 4; ++w) fx_mac(a[t + w], g, p[w]);
+    }
+  }
+  if (FIRST) A0 = fx_val(a0);
+  int64_t mx = A0 < 0 ? -A0 : A0;
+  const Fx2 A0s = fx_split(A0);
+#pragma unroll
+  for (int t = 0; t < NV; ++t)
+    if (l0 + t < kFixMaxD) {
+      const int64_t a1 = fx_val(a[2 * t]), a2 = fx_val(a[2 * t + 1]);
+      mx |= (a1 < 0 ? -a1 : a1) | (a2 < 0 ? -a2 : a2);
+      // U (U A0 - 2 a1) + a2
+      const int64_t in = fx_mul(U[t], A0s) - 2 * a1;
+      const int64_t v = a2 + fx_mul(U[t], fx_split(in));
+      const bool put = own && l0 + t < d;
+      const int f = fix_put_rhs<G>(v, E, put, cv + l0 + t);
+      if (tl == l0 + t) fc = f + 2 * ex[t];
+    }
+  __syncwarp();
+  return !own || mx < (1ll << 59);
+}
+
+template <int G>
+__global__ void __launch_bounds__(kFixThreads, 1) k_block_fix(LikArgs A, int wpc, int ncap, int rs, int kmin) {
+  extern __shared__ double smem[];
+  constexpr int St = FixDim<G>::kSt, Cs = FixDim<G>::kCs, NB = 32 / G;
+  uint64_t* T = (uint64_t*)smem;
+  for (int i = threadIdx.x; i < 256; i += blockDim.x) T[i] = kFxExp2[i];
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tm = lane / G, tl = lane % G;
+  const int kcap = A.kcap < G ? A.kcap : G;
+  FixSlot<G> S;
+  S.M = (Fx2*)(smem + 256 + (int64_t)(warp * NB + tm) * fix_slot_words(G, kcap, ncap, rs));
+  S.Gp = S.M + kcap * St;
+  S.cv = S.Gp + fix_g_words(G, kcap, ncap);
+  S.Pm = S.cv + rs * kcap;
+  S.us = S.Pm + fix_p_words(kcap);
+  S.nrm = (int64_t*)(S.us + G);
+  S.rs = rs;
+  double* scg = (double*)S.Pm;   // column scales and last rows, after dSigma a
+  double* wkd = scg + kFixCols;  // w_K of the parameters, then z_K of y and Z
+
+  const int64_t nb = A.b1 - A.b0;
+  const int64_t stride = (int64_t)gridDim.x * wpc * NB;
+  for (int64_t base = ((int64_t)blockIdx.x * wpc + warp) * NB; base < nb; base += stride) {
+    const int64_t tix = base + tm;
+    bool active = tix < nb;
+    const int64_t b = active ? launch_block(A, A.b0 + tix) : 0;
+    const int pid = active ? block_problem(A, b) : 0;
+    const ProbInfo& PI = A.probs[pid];
+    if (active && PI.skip) active = false;
+    int K = active ? A.kb[b] + 1 : 0;
+    if (K <= kmin) active = false;  // another launch's
+    if (active && K > 32) {
+      if (tl == 0) set_error(A.info + 4 * pid + SV_INFO_STATUS, SV_EINVAL);
+      active = false;
+    }
+    // fix_ek < 0: a problem this kernel does not take
+    if (active && (PI.fix_ek < 0 || K > kcap)) {
+      if (K <= 16 || G == 32 || A.kcap <= 16) {  // else the 32-lane launch's
+        if (tl == 0) {
+          A.level[b] = 0;
+          A.redo[b] = 1;
+          A.flags[1] = 1;
+        }
+      }
+      active = false;
+    }
+    if (!active) K = 0;
+    const int Kw = __reduce_max_sync(kFull, K);
+    if (Kw == 0) continue;
+    const int d = PI.d, q = PI.q, P = PI.P;
+    bool bad = false;  // to the float64 kernels
+    const int ek = PI.fix_ek;
+    const bool own = tl < K;
+
+    // ---- gather: neighbours first, self last; coordinates centred on self,
+    //      a lane takes its own row, all its loads in flight at once
+    int row = 0, exm = 0;
+    if (own) row = (tl < K - 1) ? A.nbr[b * A.ldnbr + tl] : A.rowb[b];
+    {
+      const int self = __shfl_sync(kFull, row, K > 0 ? K - 1 : 0, G);
+      const double* xi = A.X + PI.x_off + (int64_t)row * d;
+      const double* xs = A.X + PI.x_off + (int64_t)self * d;
+      double v[kFixMaxD];
+#pragma unroll
+      for (int l = 0; l < kFixMaxD; ++l) v[l] = (own && l < d) ? xi[l] - xs[l] : 0.0;
+#pragma unroll
+      for (int l = 0; l < kFixMaxD; ++l)
+        if (l < d) {
+          v[l] *= PI.invlam[l];
+          exm = max(exm, (int)((dbits(v[l]) >> 52) & 0x7ff));
+        }
+      exm = team_max<G>(exm);
+      if (exm > 1023 + 4) {  // |u| >= 32, infinities, NaN
+        bad = true;
+        exm = 2046;
+      }
+      // Q61 with |U| < 1/4; n = |U|^2 in Q62
+      int64_t hh = 0, cr = 0, ll = 0;
+#pragma unroll
+      for (int g = 0; g < kFixMaxD; g += 4)
+        if (g < d) {
+#pragma unroll
+          for (int l = g; l < g + 4; ++l) {
+            const Fx2 u = fx_split(fx_from_bits<6>(dbits(v[l]), exm));
+            if (own) S.cv[tl * rs + l] = u;
+            hh += (int64_t)u.h * u.h;
+            cr += (int64_t)u.h * u.l;
+            ll += (int64_t)u.l * u.l;
+          }
+        }
+      S.nrm[tl] = hh + ((2 * cr + (ll >> 30) + (1ll << 29)) >> 30);
+    }
+    const int es = bad ? 0 : exm - 1023 + 3;  // |u| 2^-es < 1/4
+    if (own) *(int64_t*)(S.M + tl * St + tl) = PI.fix_diag;
+    __syncwarp();
+
+    if (own) {
+      if (PI.closed == 1)
+        fix_assemble<G, 1>(K, d, tl, es, ek, S, T);
+      else
+        fix_assemble<G, 2>(K, d, tl, es, ek, S, T);
+    }
+    __syncwarp();
+
+    // ---- C C^T = Sigma / (s2 2^ek), T = C^-1
+    int E, su;
+    int64_t cd;
+    const int64_t dmin = fix_factor<G>(K, Kw, tl, S.M, cd, E);
+    bad |= dmin < (1ll << (58 - kFixPivotShift));
+    Fx2 usi;
+    bad |= !fix_last_row<G>(K, Kw, tl, S.M, cd, E, S.us, su, usi);
+
+    // ---- right-hand sides: d inputs, nugget, y, q trend columns; fc: scale
+    //      of the column tl (fc2: tl + G)
+    int fc = 0, fc2 = 0;
+    Fx2* cv = S.cv + tl * rs;
+    if (A.need_grad) {
+      int64_t A0 = 0;
+      const int dw = __reduce_max_sync(kFull, active ? d : 0);
+      if (!fix_dsig<G, kFixV, true>(K, d, 0, tl, es, E, S, usi, fc, A0)) bad = true;
+      int l0 = kFixV;
+#pragma unroll 1
+      for (; l0 + 2 < dw; l0 += kFixV)
+        if (!fix_dsig<G, kFixV, false>(K, d, l0, tl, es, E, S, usi, fc, A0)) bad = true;
+      if (l0 < dw)
+        if (!fix_dsig<G, 2, false>(K, d, l0, tl, es, E, S, usi, fc, A0)) bad = true;
+      const int f = fix_put_rhs<G>(fx_join(usi), E, own, cv + d);  // nugget: s2 tau a
+      if (tl == d) fc = f;
+    }
+    double* rec = A.cache + b * (int64_t)A.CS;
+    const double rsig = PI.fix_rsig;
+    const int np = d + 1;  // columns before y: parameters 1 .. d + 1
+    double* zk = wkd + np;
+    const int qw = __reduce_max_sync(kFull, active ? q : 0);
+    for (int c = 0; c <= qw; ++c) {
+      const bool in = own && c <= q;
+      int64_t x = 0;
+      if (in) x = dbits(c == 0 ? A.y[PI.y_off + row] : A.Z[PI.z_off + (int64_t)row * q + (c - 1)]);
+      const int em = team_max<G>((int)((x >> 52) & 0x7ff));
+      if (em > 1023 + 600) bad = true;
+      x = fx_from_bits<5>(x, em);  // units 2^(em - 1022 - 58)
+      // a.y, a.Z = (L^-1 y)_K, (L^-1 Z)_K (likelihood.py:129-134)
+      FxAcc p = {0, 0};
+      if (in) fx_mac(p, usi, fx_split(x));
+#pragma unroll
+      for (int o = G / 2; o > 0; o >>= 1) {
+        p.h += __shfl_xor_sync(kFull, (long long)p.h, o, G);
+        p.m += __shfl_xor_sync(kFull, (long long)p.m, o, G);
+      }
+      if (active && c <= q && tl == 0) {
+        const double az = (double)fx_val(p) * (rsig * pow2(em - 1022)) * pow2(su - 58);
+        rec[1 + c] = az;
+        rec[2 + q + c] = az;
+        zk[c] = az;
+      }
+      if (A.need_grad) {
+        const int f = fix_put_rhs<G>(x, E, in, cv + np + c) + em - 1022;
+        if (np + c == tl) fc = f;
+        if (np + c == tl + G) fc2 = f;
+      }
+    }
+    if (own && tl == K - 1) rec[0] = PI.fix_sig * ((double)cd * pow2(-58));  // L_KK
+    __syncwarp();
+    if (A.need_grad) {
+      // ---- W = C^-1 V = T V (likelihood.py:139, 154): lane k its row of T
+      //      and of every column, four columns at a time; kept at the scale
+      //      of the column's largest element
+      const int NR = d + 2 + q;
+      const int NRw = __reduce_max_sync(kFull, active ? NR : 0);
+      const double pu = pow2(su - ek);
+      Fx2* W = S.Gp;
+      const Fx2* tr = S.M + (own ? tl : 0) * St;
+      for (int c0 = 0; c0 < NRw; c0 += 4) {
+        FxAcc acc[4];
+#pragma unroll
+        for (int w = 0; w < 4; ++w) acc[w] = {0, 0};
+        const Fx2* vj = S.cv + c0;
+#pragma unroll 4
+        for (int j = 0; j < K; ++j, vj += rs) {
+          Fx2 v[4];
+          load4(vj, v);
+          const Fx2 t = tr[j];
+#pragma unroll
+          for (int w = 0; w < 4; ++w) fx_mac(acc[w], t, v[w]);
+        }
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          const int c = c0 + w;
+          const int64_t x = own && c < NR ? fx_val(acc[w]) : 0;
+          const int s = team_max<G>(fx_bits(x)) - 57;
+          if (own && c < NR) W[c * Cs + tl] = fx_split(fx_scale2(x, -s));
+          if (c == tl) fc += s;
+          if (c == tl + G) fc2 += s;
+        }
+      }
+      __syncwarp();
+      for (int c = tl; active && c < NR; c += G) {
+        // true value = W 2^-58 sc
+        double sc = pow2(c < G ? fc : fc2);
+        if (c > d)
+          sc *= rsig;
+        else if (c == d)
+          sc *= PI.tau * pu;
+        else
+          sc *= (PI.closed == 1 ? 3.0 : 5.0 / 3.0) * pu;
+        sc *= pow2(-29);
+        scg[c] = sc;
+        const double wk = c < np ? (double)fx_join(W[c * Cs + K - 1]) * sc * pow2(-29) : zk[c - np];
+        if (c < np) wkd[c] = wk;
+        // ---- record: z_K, w_K and what involves W_0 = e_K (parameter 0 is
+        //      Sigma itself); columns c < np are parameters c + 1
+        double* wK = rec + 3 + 2 * q;
+        double* wzy = wK + P;
+        double* wzZ = wzy + P;
+        double* F = wzZ + P * q;
+        if (c < np) {
+          wK[c + 1] = wk;
+          F[tri_off(c + 1, 0)] = 0.5 * wk;
+        } else {
+          if (c == np)
+            wzy[0] = wk;
+          else
+            wzZ[c - np - 1] = wk;
+        }
+        if (c == 0) {
+          wK[0] = 1.0;
+          F[0] = 0.5;
+        }
+      }
+      __syncwarp();
+      if (active) {
+        // ---- record: W z, F = W W^T - w_K w_K^T / 2 (likelihood.py:140-142)
+        //      by 2 x 2 tiles: columns (c2, c2 + 1) of the parameters, rows
+        //      (c1, c1 + 1) from c1 = c2 on
+        double* wzy = rec + 3 + 2 * q + P;
+        double* wzZ = wzy + P;
+        double* F = wzZ + P * q;
+        auto tiles_of = [&](int t) { return (NR - 2 * t + 1) / 2; };
+        int ntile = 0;
+        for (int t = 0; 2 * t < np; ++t) ntile += tiles_of(t);
+        auto put = [&](int c1, int c2, const FxAcc& a) {
+          if (c1 >= NR || c2 >= np || c1 < c2) return;
+          const double v = (double)fx_val(a) * (scg[c1] * scg[c2]);
+          if (c1 < np)
+            F[tri_off(c1 + 1, c2 + 1)] = fma(-0.5 * wkd[c1], wkd[c2], v);
+          else if (c1 == np)
+            wzy[c2 + 1] = v;
+          else
+            wzZ[(c2 + 1) * q + (c1 - np - 1)] = v;
+        };
+        for (int t = tl; t < ntile; t += G) {
+          int pu2 = 0, rem = t;
+          while (rem >= tiles_of(pu2)) {
+            rem -= tiles_of(pu2);
+            ++pu2;
+          }
+          const int c2 = 2 * pu2, c1 = c2 + 2 * rem;
+          const Fx2* xa = W + c1 * Cs;
+          const Fx2* xb = W + min(c1 + 1, NR - 1) * Cs;
+          const Fx2* ya = W + c2 * Cs;
+          const Fx2* yb = W + min(c2 + 1, NR - 1) * Cs;
+          FxAcc g00 = {0, 0}, g01 = {0, 0}, g10 = {0, 0}, g11 = {0, 0};
+#pragma unroll 2
+          for (int i = 0; i < K; ++i) {
+            const Fx2 a0 = xa[i], a1 = xb[i], b0 = ya[i], b1 = yb[i];
+            fx_mac(g00, a0, b0);
+            fx_mac(g01, a0, b1);
+            fx_mac(g10, a1, b0);
+            fx_mac(g11, a1, b1);
+          }
+          put(c1, c2, g00);
+          put(c1, c2 + 1, g01);
+          put(c1 + 1, c2, g10);
+          put(c1 + 1, c2 + 1, g11);
+        }
+      }
+    }
+    const unsigned badm = __ballot_sync(kFull, bad) & (G == 32 ? kFull : 0xffffu << (16 * tm));
+    if (active && tl == 0) {
+      A.level[b] = 0;
+      A.redo[b] = badm ? 1 : 0;
+      if (badm) A.flags[1] = 1;
+    }
+    __syncwarp();
+  }
+}
+
+namespace {
+
+template <int G>
+int launch_fix_g(const LikArgs& A, int kmin, int maxsm, cudaStream_t st) {
+  // columns of the largest problem taken
+  const int dm = A.dmax < kFixMaxD ? A.dmax : kFixMaxD;
+  int ncap = dm + 2 + A.qmax;
+  if (ncap > kFixCols) ncap = kFixCols;
+  const int pad = (dm + 3) & ~3, col4 = (ncap + 3) & ~3;
+  const int rs = (pad > col4 ? pad : col4) + 2;
+  const int kcap = A.kcap < G ? A.kcap : G;
+  const size_t per_warp = (32 / G) * sizeof(double) * (size_t)fix_slot_words(G, kcap, ncap, rs),
+               fixed = 256 * sizeof(double);
+  int wpc = kFixThreads / 32;
+  while (wpc > 1 && fixed + wpc * per_warp > (size_t)maxsm) --wpc;
+  const size_t smem = fixed + wpc * per_warp;
+  if (smem > (size_t)maxsm) return SV_EINVAL;
+  SV_CUDA_TRY(cudaFuncSetAttribute(k_block_fix<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_block_fix<G>, 32 * wpc, smem) != cudaSuccess ||
+      per_sm < 1)
+    per_sm = 1;
+  const int64_t per_cta = (int64_t)wpc * (32 / G);
+  int64_t grid = (A.b1 - A.b0 + per_cta - 1) / per_cta;
+  if (grid > (int64_t)per_sm * sv_num_sms()) grid = (int64_t)per_sm * sv_num_sms();
+  if (grid < 1) grid = 1;
+  k_block_fix<G><<<(unsigned)grid, 32 * wpc, smem, st>>>(A, wpc, ncap, rs, kmin);
+  SV_CUDA_TRY(cudaGetLastError());
+  return SV_OK;
+}
+
+}  // namespace
+
+int launch_block_fix(const LikArgs& A, int maxsm, cudaStream_t st) {
+  if (A.kcap <= 16) return launch_fix_g<16>(A, 0, maxsm, st);
+  // a batch may hold many blocks of at most 16 points: they go two to a warp.
+  // One problem has at most 16 of them, not worth a launch
+  int kmin = 0;
+  if (A.nprob > 1) {
+    const int rc = launch_fix_g<16>(A, 0, maxsm, st);
+    if (rc != SV_OK) return rc;
+    kmin = 16;
+  }
+  return launch_fix_g<32>(A, kmin, maxsm, st);
+}
+
+}  // namespace sv

@@ -250,6 +250,9 @@ class DeviceProblem:
         split = (precision in _SPLIT and split_nu(nu, estimate_nu)
                  and self.d + 3 + self.q <= 32)
         n = (1 if warp else 0) + (1 if cta else 0)
+        if (not split and warp and not estimate_nu and float(nu) in (1.5, 2.5) and self.d <= 12
+                and self.d + 2 + self.q <= 32):
+            n += 1  # the fixed-point kernel, then the float64 kernels over what it flagged
         if estimate_nu or matern_table_nu(nu):
             n += 2 if split else 1  # the Matern tables: float64, and float32 for the split kernels
         if split and warp:

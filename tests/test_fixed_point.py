@@ -1,0 +1,115 @@
+"""The fixed-point block kernel (csrc/sv_fix.cuh, sv_loglik_fix.cu).
+
+On the CPU, the arithmetic compiled as host C++ against long double: limbs
+rejoin exactly, a product is within 2 units of 2^-58, a pivot's reciprocal
+root within 4 relative units and the Matern terms within 4 units (their chain
+of a dozen truncated 64-bit products, each below 2^-60, and the table's and
+polynomial's 2^-62).  On the GPU, the kernel at the edges of its block sizes,
+dimensions and ranges against the oracle; what it hands to the float64 kernels
+must come out the same way."""
+import math
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "pyscaledvecchia_gb300", "csrc")
+
+DRIVER = r"""
+#include "sv_fix.cuh"
+#include <cstdio>
+#include <cmath>
+using namespace sv;
+typedef long double LD;
+static uint64_t st = 88172645463325252ULL;
+static uint64_t rnd() { st ^= st << 13; st ^= st >> 7; st ^= st << 17; return st; }
+static double uni() { return (double)(rnd() >> 11) / 9007199254740992.0; }
+int main() {
+  double em = 0, eg = 0, ep = 0, ex = 0;
+  long bad = 0;
+  for (int it = 0; it < 300000; ++it) {
+    const int code = 1 + (it & 1), es = (int)(rnd() % 10) - 4;
+    const double lg = (it % 3 == 0) ? -8 + 9 * uni() : -60 + 61 * uni();
+    const uint64_t s = (uint64_t)std::ldexp(1.0 + uni(), 62 + (int)std::floor(lg)) ^ (rnd() & 1);
+    uint64_t M, g;
+    if (code == 1) fx_matern<1>(s, es, kFxExp2, M, g); else fx_matern<2>(s, es, kFxExp2, M, g);
+    const LD c = std::sqrt((LD)s * (code == 1 ? 3 : 5)) * std::ldexp((LD)1, es - 31), e = std::exp(-c);
+    const LD Mr = code == 1 ? (1 + c) * e : (1 + c + c * c / 3) * e, gr = code == 1 ? e : (1 + c) * e;
+    em = std::fmax(em, (double)(std::fabs(std::ldexp((LD)M, -61) - Mr) * std::ldexp((LD)1, 58)));
+    eg = std::fmax(eg, (double)(std::fabs(std::ldexp((LD)g, -61) - gr) * std::ldexp((LD)1, 58)));
+    int64_t d = (int64_t)(rnd() >> 6) >> (rnd() % 41);
+    if (d < 65536) d = 65536;
+    int ee;
+    const int64_t Y = fx_rsqrt_pivot(d, ee);
+    bad += Y > (1ll << 58) || Y <= (1ll << 57) - 16 || ee < 0;
+    const LD yr = std::ldexp((LD)Y, ee - 58) * std::sqrt(std::ldexp((LD)d, -58));
+    ep = std::fmax(ep, (double)(std::fabs(yr - 1) * std::ldexp((LD)1, 58)));
+    const int64_t x = ((int64_t)(rnd() >> 5) - (1ll << 58)), y = ((int64_t)(rnd() >> 5) - (1ll << 58));
+    bad += fx_join(fx_split(x)) != x;
+    bad += fx_split(x).l > (1 << 29) || fx_split(x).l < -(1 << 29);
+    const __int128 pr = (__int128)x * y;
+    const __int128 df = ((__int128)fx_mul(fx_split(x), fx_split(y)) << 58) - pr;
+    ex = std::fmax(ex, std::fabs((double)df) * std::ldexp(1.0, -58));
+  }
+  std::printf("%.4f %.4f %.4f %.4f %ld\n", em, eg, ep, ex, bad);
+}
+"""
+
+
+def test_arithmetic(tmp_path):
+    gxx = shutil.which("g++")
+    if gxx is None:
+        pytest.skip("no g++")
+    src, exe = tmp_path / "t.cpp", tmp_path / "t"
+    src.write_text(DRIVER)
+    subprocess.run([gxx, "-O2", "-std=gnu++17", "-I" + CSRC, str(src), "-o", str(exe)], check=True)
+    em, eg, ep, ex, bad = (float(v) for v in
+                           subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split())
+    assert em <= 4 and eg <= 4 and ep <= 4 and ex <= 2 and bad == 0, (em, eg, ep, ex, bad)
+
+
+CASES = [  # n, d, m, nu, trend columns, range lo, scale of y
+    (40, 1, 5, 1.5, 0, 0.2, 1.0),
+    (150, 12, 15, 2.5, 1, 0.5, 1.0),      # blocks of 16: two to a warp
+    (150, 12, 16, 2.5, 1, 0.5, 1e30),     # blocks of 17
+    (150, 4, 31, 1.5, 5, 0.2, 1e-30),     # blocks of 32, a linear trend
+    (150, 2, 30, 2.5, 16, 0.2, 1.0),      # the most trend columns
+    (150, 13, 20, 2.5, 1, 0.5, 1.0),      # d = 13: the float64 kernels
+    (150, 3, 20, 2.5, 1, 0.005, 1.0),     # neighbours 32 ranges away and more
+]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,d,m,nu,q,lo,ys", CASES)
+def test_against_oracle(oracle, n, d, m, nu, q, lo, ys):
+    import pyscaledvecchia_gb300 as sv
+    from pyscaledvecchia_gb300.batched import BatchedLikelihood, BatchProblem
+    from pyscaledvecchia_gb300.likelihood import DeviceProblem
+    from pyscaledvecchia_gb300.ordering import _nn_groups
+    rng = np.random.default_rng(100 * d + m)
+    X = rng.random((n, d))
+    y = ys * rng.standard_normal(n)
+    Z = np.hstack([np.ones((n, 1)), rng.random((n, q - 1))]) if q else None
+    lam = np.exp(rng.uniform(math.log(lo), math.log(20 * lo), d))
+    theta = np.concatenate([[math.log(1.7)], np.log(lam), [math.log(2e-3)]])
+    groups = _nn_groups(sv.find_ordered_nn(X / lam, m), m)
+    ref = oracle.vecchia_loglik(theta, X, y, Z, groups, nu)
+    prob = DeviceProblem(X, y, Z, groups)
+    got = prob.evaluate(theta, nu)
+    # conditioning up to 31 / tau ~ 2e4 times 31 float64 roundings, as the
+    # float64 form's own oracle tests allow
+    assert abs(got[0] - ref[0]) <= 1e-10 * abs(ref[0])
+    for a, b in zip(got[1:], ref[1:]):
+        np.testing.assert_allclose(a, b, rtol=1e-8, atol=1e-8 * (np.abs(b).max() if np.size(b) else 0.0))
+    ll = prob.evaluate(theta, nu, need_grad=False)
+    assert abs(ll[0] - got[0]) <= 1e-12 * abs(got[0])
+    # the same bits in a batch that also holds a problem of another kind
+    other = (X[:40, :1], y[:40], None, _nn_groups(sv.find_ordered_nn(X[:40, :1], 35), 35))
+    BL = BatchedLikelihood([BatchProblem(X, y, Z, groups, nu=nu), BatchProblem(*other, nu=0.5)])
+    r = BL.evaluate([theta, np.array([0.1, math.log(0.3), math.log(0.1)])])[0]
+    assert r[0] == 0 and r[1] == got[0]
+    for a, b in zip(r[2:], got[1:]):
+        np.testing.assert_array_equal(a, b)
