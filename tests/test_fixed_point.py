@@ -113,3 +113,41 @@ def test_against_oracle(oracle, n, d, m, nu, q, lo, ys):
     assert r[0] == 0 and r[1] == got[0]
     for a, b in zip(r[2:], got[1:]):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["float64", "split"])
+@pytest.mark.parametrize("m,d,nu,lo", [(32, 1, 1.5, 0.3), (39, 5, 2.5, 0.3), (40, 12, 2.5, 0.5),
+                                       (144, 3, 1.5, 0.3), (207, 4, 2.5, 0.3), (60, 13, 2.5, 0.5),
+                                       (60, 2, 2.5, 0.004)])
+def test_prediction_against_dense(m, d, nu, lo, precision):
+    """Prediction blocks at the edges of the panels and of the kernel's range
+    (d = 13 and ranges far below the neighbours' distances go elsewhere)
+    against dense solves of the same blocks.  tau = 1e-2: conditioning below
+    m / tau = 2e4, so float64 solves agree to 1e-10; the split form's float32
+    entries to 1e-7 times that."""
+    import pyscaledvecchia_gb300 as sv
+    rng = np.random.default_rng(m + d)
+    n, ns = 400, 9
+    X, Xn = rng.random((n, d)), rng.random((ns, d))
+    y = np.sin(4.0 * X.sum(1)) + 0.1 * rng.standard_normal(n)
+    lam = np.exp(rng.uniform(math.log(lo), math.log(10 * lo), d))
+    gp = sv.ScaledVecchiaGP(m_pred=m, nu=nu, trend="zero", precision=precision)
+    gp.X_, gp.y_, gp.beta_, gp.b_, gp.d_ = X, y, np.zeros(0), 1.0, d
+    gp.theta_ = np.concatenate([[math.log(1.3)], np.log(lam), [math.log(1e-2)]])
+    gp._nu_fit, gp._lo, gp._span, gp._ymu, gp._ysd = nu, np.zeros(d), np.ones(d), 0.0, 1.0
+    mu, var = gp.predict(Xn, return_var=True)
+
+    def corr(r):
+        c = math.sqrt(2.0 * nu) * r
+        return (1.0 + c + (c * c / 3.0 if nu == 2.5 else 0.0)) * np.exp(-c)
+
+    tol = 1e-10 if precision == "float64" else 2e-3
+    for i in range(ns):
+        nb = np.argsort((((X - Xn[i]) / lam) ** 2).sum(1), kind="stable")[:m]
+        U, u = X[nb] / lam, Xn[i] / lam
+        S = 1.3 * (corr(np.sqrt(((U[:, None] - U[None]) ** 2).sum(2))) + 1e-2 * np.eye(m))
+        k = 1.3 * corr(np.sqrt(((U - u) ** 2).sum(1)))
+        w = np.linalg.solve(S, k)
+        assert abs(var[i] - (1.3 - w @ k)) <= tol * 1.3
+        assert abs(mu[i] - w @ y[nb]) <= tol * max(1.0, np.abs(y).max())
