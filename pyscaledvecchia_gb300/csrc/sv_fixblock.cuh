@@ -36,6 +36,16 @@ __device__ __forceinline__ void load4(const Fx2* p, Fx2 (&v)[4]) {
   v[2].h = b.x; v[2].l = b.y; v[3].h = b.z; v[3].l = b.w;
 }
 
+// The products of low limbs that fx_mac leaves out average to nothing in a sum
+// of products of different numbers, but in a row's sum of squares (its pivot)
+// they are all positive, a third of a unit each. fx_sq adds one up (in units
+// of 2^-50 of Q58's), fx_sq_val is their sum in Q58.
+__device__ __forceinline__ void fx_sq(int64_t& s, Fx2 x) {
+  const int t = x.l >> 4;
+  s += (int64_t)t * t;
+}
+__device__ __forceinline__ int64_t fx_sq_val(int64_t s) { return (s + (1ll << 49)) >> 50; }
+
 // x where keep is -1, 0 where it is 0: by a mask the compiler cannot see
 // through (it would otherwise select between whole products)
 __device__ __forceinline__ Fx2 fx_keep(Fx2 x, int keep) {
@@ -65,7 +75,7 @@ __device__ __forceinline__ Fx2 fx_keep(Fx2 x, int keep) {
 template <int G>
 __device__ __forceinline__ int64_t fix_factor(int K, int Kw, int tl, Fx2* M, int64_t& cd, int& E) {
   constexpr int St = FixDim<G>::kSt;
-  int64_t dmin = 1ll << 58;
+  int64_t dmin = 1ll << 58, sq = 0;
   E = 0;
   cd = 0;
   for (int k0 = 0; k0 < Kw; k0 += kFixPanel) {
@@ -90,6 +100,7 @@ __device__ __forceinline__ int64_t fix_factor(int K, int Kw, int tl, Fx2* M, int
       int64_t v = 0;
       if (tl >= k && tl < K) v = *(const int64_t*)ck;
       v -= fx_val(acc[w]);
+      if (tl == k) v -= fx_sq_val(sq);
       int64_t d = __shfl_sync(kFull, (long long)v, k, G);
       if (k < K && d < dmin) dmin = d;
       if (d < (1ll << (58 - kFixPivotShift)) || d > (1ll << 58)) d = 1ll << 58;
@@ -125,6 +136,7 @@ __device__ __forceinline__ int64_t fix_factor(int K, int Kw, int tl, Fx2* M, int
         for (int w2 = w + 1; w2 < kFixPanel; ++w2) acc[w2] = {0, 0};
       }
       const Fx2 c = fx_split(x);
+      if (tl > k) fx_sq(sq, c);
       if (tl < K && k < K) *ck = c;
 #pragma unroll
       for (int w2 = w + 1; w2 < kFixPanel; ++w2) {

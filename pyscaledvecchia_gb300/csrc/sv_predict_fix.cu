@@ -19,7 +19,7 @@
 // panel) while the rows' warps take the next panel's sums over the columns
 // before. Two CTAs of a 141-point block (106 KB) fill an SM.
 //
-// Weights beyond 32, pivots below 2^-34 of the diagonal (split form: below
+// Weights beyond 2^11, pivots below 2^-34 of the diagonal (split form: below
 // rho_min), coordinates beyond 32 ranges of the target and non-finite data: the
 // split form's block is redone as the float64 form's, that one by pred_block
 // in the same CTA.
@@ -29,7 +29,9 @@
 namespace sv {
 
 constexpr int kPfW = 8;     // columns per panel
-constexpr int kPfShift = 6; // weights u = us 2^kPfShift, |us| < 1/2
+// weights |a_j| < 2^(kPfShift - 1) / C_KK, then (where one does not fit)
+// 2^(kPfShift2 - 1) / C_KK
+constexpr int kPfShift = 3, kPfShift2 = 12;
 
 // column j's rows start at row 8 (j / 8); two words of padding keep the
 // columns' 16-byte loads apart
@@ -84,10 +86,12 @@ __device__ __forceinline__ void pf_diag(int K, int k0, int r, bool writer, Fx2* 
 #pragma unroll
   for (int w = 0; w < kPfW; ++w) acc[w] = {0, 0};
   int E = 0;
+  int64_t sq = 0;
 #pragma unroll
   for (int w = 0; w < kPfW; ++w) {
     const int c = k0 + w;
     int64_t v = (r >= w ? *(const int64_t*)(pc + w * Lp + k0 + r) : 0) - fx_val(acc[w]);
+    if (r == w) v -= fx_sq_val(sq);
     const int64_t dv = __shfl_sync(kFull, (long long)v, w, 8);
     if (c < K && writer && r == w && (dv < thr[c] || dv > (1ll << 58))) *bad = 1;
     const int64_t dc = (dv < (1ll << (58 - kFixPivotShift)) || dv > (1ll << 58)) ? 1ll << 58 : dv;
@@ -131,6 +135,7 @@ __device__ __forceinline__ void pf_diag(int K, int k0, int r, bool writer, Fx2* 
       for (int w2 = w + 1; w2 < kPfW; ++w2) acc[w2] = {0, 0};
     }
     const Fx2 cs = fx_split(x);
+    if (r > w) fx_sq(sq, cs);
     if (writer) {
       if (r > w)
         pc[w * Lp + k0 + r] = cs;
@@ -339,6 +344,7 @@ __global__ void __launch_bounds__(NT, MINB) k_pred_fix(PredArgs A) {
 
     // ---- Cholesky factor, panels of 8 columns.  At the start of a panel its
     //      columns hold S less the earlier columns' products
+    int64_t sq = 0;
     for (int k0 = 0; k0 < K8; k0 += kPfW) {
       Fx2* pc = M + pf_col(k0, K8);
       const int Lp = K8 - k0 + 2, k1 = k0 + kPfW;
@@ -378,6 +384,7 @@ __global__ void __launch_bounds__(NT, MINB) k_pred_fix(PredArgs A) {
           for (int u = 0; u < w; ++u) fx_mac(t, c[u], pc[u * Lp + k0 + w]);
           const int64_t v = below ? *(const int64_t*)(pc + w * Lp + i) - fx_val(t) : 0;
           c[w] = fx_split(fx_mul(fx_split((int64_t)((uint64_t)v << ive[k0 + w])), ivy[k0 + w]));
+          fx_sq(sq, c[w]);
           if (below && half == 0) pc[w * Lp + i] = c[w];
         }
       }
@@ -402,7 +409,8 @@ __global__ void __launch_bounds__(NT, MINB) k_pred_fix(PredArgs A) {
         for (int w = 0; w < kPfW; ++w) {
           acc[w].h += __shfl_xor_sync(kFull, (long long)acc[w].h, 16);
           acc[w].m += __shfl_xor_sync(kFull, (long long)acc[w].m, 16);
-          if (half == (w & 1) && i >= k1 + w && i < K8) *(int64_t*)(pn + w * Ln) -= fx_val(acc[w]);
+          if (half == (w & 1) && i >= k1 + w && i < K8)
+            *(int64_t*)(pn + w * Ln) -= fx_val(acc[w]) + (i == k1 + w ? fx_sq_val(sq) : 0);
         }
       }
       __syncthreads();
@@ -416,49 +424,56 @@ __global__ void __launch_bounds__(NT, MINB) k_pred_fix(PredArgs A) {
     // ---- a = C^-T e_K, panels from the last to the first: the panel's 8 rows
     //      by the inverse of its diagonal block, then every earlier row its
     //      terms (the two lanes of a row four each).  a = us 2^sa
-    const int sa = ive[K - 1] + kPfShift;
-    FxAcc acc = {0, 0};
+    int sa = ive[K - 1] + kPfShift;
     Fx2 ui = {0, 0};
-    for (int k0 = K8 - kPfW; k0 >= 0; k0 -= kPfW) {
-      if (!boss && warp == (k0 >> 4)) {
-        const bool mine = i >= k0 && i < k0 + kPfW;
-        FxAcc tot = acc;
-        tot.h += __shfl_xor_sync(kFull, (long long)acc.h, 16);
-        tot.m += __shfl_xor_sync(kFull, (long long)acc.m, 16);
-        int64_t r = mine && own ? -fx_val(tot) : 0;
-        if (mine && i == K - 1) r += 1ll << (58 - sa);
-        const int g = 57 - team_max<32>(fx_bits(r));  // the panel's largest below 2^57
-        const Fx2 rs2 = fx_split(fx_scale2(r, g));
-        const Fx2* t = Tp + 8 * k0 + (i & 7);
-        FxAcc u = {0, 0};
-#pragma unroll
-        for (int w = 0; w < kPfW; ++w) {
-          Fx2 o;
-          o.h = __shfl_sync(kFull, rs2.h, (k0 & 15) + w);
-          o.l = __shfl_sync(kFull, rs2.l, (k0 & 15) + w);
-          if (w >= (i & 7)) fx_mac(u, t[8 * w], o);
-        }
-        if (mine) {
-          const int64_t x = fx_val(u);
-          int sh = Te[i] - g;
-          if (own && fx_bits(x) + sh > 57 && x != 0) {
-            s_bad = 1;
-            sh = 0;
+    for (int wide = 0; wide < 2; ++wide) {
+      FxAcc acc = {0, 0};
+      for (int k0 = K8 - kPfW; k0 >= 0; k0 -= kPfW) {
+        if (!boss && warp == (k0 >> 4)) {
+          const bool mine = i >= k0 && i < k0 + kPfW;
+          FxAcc tot = acc;
+          tot.h += __shfl_xor_sync(kFull, (long long)acc.h, 16);
+          tot.m += __shfl_xor_sync(kFull, (long long)acc.m, 16);
+          int64_t r = mine && own ? -fx_val(tot) : 0;
+          if (mine && i == K - 1) r += 1ll << (58 - sa);
+          const int g = 57 - team_max<32>(fx_bits(r));  // the panel's largest below 2^57
+          const Fx2 rs2 = fx_split(fx_scale2(r, g));
+          const Fx2* t = Tp + 8 * k0 + (i & 7);
+          FxAcc u = {0, 0};
+  #pragma unroll
+          for (int w = 0; w < kPfW; ++w) {
+            Fx2 o;
+            o.h = __shfl_sync(kFull, rs2.h, (k0 & 15) + w);
+            o.l = __shfl_sync(kFull, rs2.l, (k0 & 15) + w);
+            if (w >= (i & 7)) fx_mac(u, t[8 * w], o);
           }
-          ui = fx_split(own ? fx_scale2(x, sh) : 0);
-          if (half == 0) us[i] = ui;
+          if (mine) {
+            const int64_t x = fx_val(u);
+            int sh = Te[i] - g;
+            if (own && fx_bits(x) + sh > 57 && x != 0) {
+              s_bad = 1;
+              sh = 0;
+            }
+            ui = fx_split(own ? fx_scale2(x, sh) : 0);
+            if (half == 0) us[i] = ui;
+          }
+        }
+        __syncthreads();
+        if (!boss && i < k0) {
+          Fx2 c4[4], u4[4];
+          load4(M + pf_col(i, K8) + k0 + 4 * half, c4);
+          load4(us + k0 + 4 * half, u4);
+  #pragma unroll
+          for (int w = 0; w < 4; ++w) fx_mac(acc, c4[w], u4[w]);
         }
       }
       __syncthreads();
-      if (!boss && i < k0) {
-        Fx2 c4[4], u4[4];
-        load4(M + pf_col(i, K8) + k0 + 4 * half, c4);
-        load4(us + k0 + 4 * half, u4);
-#pragma unroll
-        for (int w = 0; w < 4; ++w) fx_mac(acc, c4[w], u4[w]);
-      }
+      if (!s_bad || wide) break;
+      __syncthreads();
+      if (threadIdx.x == 0) s_bad = 0;
+      sa = ive[K - 1] + kPfShift2;
+      __syncthreads();
     }
-    __syncthreads();
     if (s_bad) {
       if (pf_next(A, split, s_bad, s_max)) continue;
       pf_fallback(A, prm, b, region);
