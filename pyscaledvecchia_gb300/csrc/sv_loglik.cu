@@ -24,6 +24,7 @@
 // variance penalty).  Reductions are in a fixed order, so results are bitwise
 // reproducible run to run.  Only kernels and memsets are enqueued, so a
 // batched evaluation can be captured in a CUDA graph.
+#include <cooperative_groups.h>
 #include <stdio.h>
 
 #include <algorithm>
@@ -32,6 +33,8 @@
 #include "sv_loglik.cuh"
 
 namespace sv {
+
+namespace cg = cooperative_groups;
 
 // the central difference step of an estimated nu (_matern_general.py:135, nu_fd_h)
 constexpr double kNuFdH = 1e-3;
@@ -147,7 +150,8 @@ __global__ void k_prob_params(const sv_prob_desc* descs, const double* theta, in
       I.fix_rsig = 1.0 / I.fix_sig;
     }
   }
-  for (int l = threadIdx.x; l < d; l += blockDim.x) I.invlam[l] = exp(-th[1 + l]);
+  // (the second warp, beside the first one's chain of float64 operations)
+  for (int l = (int)threadIdx.x - 32; l >= 0 && l < d; l += 32) I.invlam[l] = exp(-th[1 + l]);
 }
 
 // the Matern tables of the problems that use them (kMtabMaxDoubles each, in
@@ -524,7 +528,7 @@ __global__ void k_block_warp(LikArgs A) {
         set_error(A.info + 4 * block_problem(A, b) + SV_INFO_STATUS, SV_EINVAL);
       continue;
     }
-    if (A.kb[b] + 1 <= 16) continue;
+    if (A.kb[b] + 1 <= 16 && !A.fixup) continue;
     block_pass1<32>(A, b, sm, 32);
     __syncwarp();
   }
@@ -634,8 +638,27 @@ __host__ __device__ inline int red_parts_n(int64_t nblk) {
   return (int)parts;
 }
 
-__global__ void k_reduce1(RedArgs R) {
+// CTAs per partition: a thread-block cluster, its CTAs the partition's blocks
+// in runs, added up through distributed shared memory in CTA order (a
+// partition per CTA leaves all but a few SMs idle below 100,000 blocks:
+// n = 5,000 took 90 us in k_reduce1 and 51 us in k_reduce2)
+constexpr int kRedCl = 8;
+
+// the blocks [b0, b1) of CTA `rank` of partition `part`
+__device__ __forceinline__ void red_range(const ProbInfo& PI, int parts, int part, int rank, int64_t& b0,
+                                          int64_t& b1) {
+  const int64_t per = (PI.nblk + parts - 1) / parts;
+  const int64_t p0 = PI.blk_off + part * per;
+  const int64_t p1 = min(PI.blk_off + PI.nblk, p0 + per);
+  const int64_t run = (per + kRedCl - 1) / kRedCl;
+  b0 = min(p1, p0 + rank * run);
+  b1 = min(p1, b0 + run);
+}
+
+__global__ void __cluster_dims__(kRedCl, 1, 1) k_reduce1(RedArgs R) {
   extern __shared__ double racc[];  // [nwarp][nfmax]
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = (int)cl.block_rank();
   const int p = blockIdx.y;
   const ProbInfo& PI = R.probs[p];
   if (PI.skip) return;
@@ -643,11 +666,10 @@ __global__ void k_reduce1(RedArgs R) {
   const int nf = nfield1(q, P, R.need_grad);
   const int nwarp = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int parts = red_parts_n(PI.nblk);
-  const int part = R.pbeg + (int)blockIdx.x;
+  const int part = R.pbeg + (int)blockIdx.x / kRedCl;
   if (part >= parts) return;
-  const int64_t per = (PI.nblk + parts - 1) / parts;
-  const int64_t b0 = PI.blk_off + part * per;
-  const int64_t b1 = min(PI.blk_off + PI.nblk, b0 + per);
+  int64_t b0, b1;
+  red_range(PI, parts, part, rank, b0, b1);
   double* acc = racc + (int64_t)w * R.nfmax;
   const int foff = 3 + 2 * q + P * (2 + q);
   // the (warp, field) sums, one owner lane each: fields lane + 32 r < 128 in
@@ -706,13 +728,25 @@ __global__ void k_reduce1(RedArgs R) {
   for (int r = 0; r < kFr; ++r)
     if (lane + 32 * r < nf) acc[lane + 32 * r] = a[r];
   __syncthreads();
-  double* partv = R.part1 + ((int64_t)p * R.parts + part) * R.nfmax;
   for (int f = threadIdx.x; f < nf; f += blockDim.x) {
     double s = 0.0;
     for (int k = 0; k < nwarp; ++k) s += racc[(int64_t)k * R.nfmax + f];
-    partv[f] = s;
+    racc[f] = s;
   }
+  cl.sync();
+  if (rank == 0) {
+    double* partv = R.part1 + ((int64_t)p * R.parts + part) * R.nfmax;
+    for (int f = threadIdx.x; f < nf; f += blockDim.x) {
+      double s = 0.0;
+#pragma unroll
+      for (int c = 0; c < kRedCl; ++c) s += cl.map_shared_rank(racc, c)[f];
+      partv[f] = s;
+    }
+  }
+  cl.sync();  // the others' shared memory stays until it has been read
 }
+
+constexpr int kFinSl = 8;  // slices of the partitions summed side by side
 
 __global__ void k_final1(RedArgs R) {
   const int p = blockIdx.x;
@@ -722,14 +756,28 @@ __global__ void k_final1(RedArgs R) {
   const int nf = nfield1(q, P, R.need_grad);
   double* sums = R.sums + (int64_t)p * R.nfmax;
   const int parts = red_parts_n(PI.nblk);
-  for (int f = threadIdx.x; f < nf; f += blockDim.x) {
+  // kFinSl slices of the partitions side by side, added in slice order
+  __shared__ double sl[kFinSl][kRedThreads / kFinSl];
+  constexpr int kF = kRedThreads / kFinSl;
+  const int ps = (parts + kFinSl - 1) / kFinSl;
+  for (int f0 = 0; f0 < nf; f0 += kF) {
+    const int f = f0 + threadIdx.x % kF, z = threadIdx.x / kF;
     double s = 0.0;
-    const double* src = R.part1 + (int64_t)p * R.parts * R.nfmax + f;
+    if (f < nf) {
+      const double* src = R.part1 + (int64_t)p * R.parts * R.nfmax + f;
+      const int c1 = min(parts, (z + 1) * ps);
 #pragma unroll 8
-    for (int c = 0; c < parts; ++c) s += src[(int64_t)c * R.nfmax];
-    sums[f] = s;
+      for (int c = z * ps; c < c1; ++c) s += src[(int64_t)c * R.nfmax];
+    }
+    sl[z][threadIdx.x % kF] = s;
+    __syncthreads();
+    if (z == 0 && f < nf) {
+#pragma unroll
+      for (int k = 1; k < kFinSl; ++k) s += sl[k][threadIdx.x];
+      sums[f] = s;
+    }
+    __syncthreads();
   }
-  __syncthreads();
   if (threadIdx.x == 0) {
     // beta = solve(XtX + 1e-12 I, Zty): Gaussian elimination, partial pivoting
     double* beta = R.beta + (int64_t)p * (R.qmax + 1);
@@ -761,9 +809,16 @@ __global__ void k_final1(RedArgs R) {
   }
 }
 
-__global__ void k_reduce2(RedArgs R) {
+// Pass-2 sums of one partition: z_K^2 and the score terms, a thread per block.
+// PR: parameters whose sums are held in registers (a runtime count puts them
+// into local memory: 131 us instead of 111 at 200,000 blocks)
+template <int PR>
+__global__ void __cluster_dims__(kRedCl, 1, 1) k_reduce2(RedArgs R) {
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = (int)cl.block_rank();
   __shared__ double sbeta[kMaxQ];
-  __shared__ double red[kRedThreads / 32][kMaxP + 1];
+  __shared__ double tot[kMaxP + 1];
+  __shared__ double red[kRedThreads / 32][PR + 1];
   const int p = blockIdx.y;
   const ProbInfo& PI = R.probs[p];
   if (PI.skip) return;
@@ -771,42 +826,56 @@ __global__ void k_reduce2(RedArgs R) {
   for (int i = threadIdx.x; i < q; i += blockDim.x) sbeta[i] = R.beta[(int64_t)p * (R.qmax + 1) + i];
   __syncthreads();
   const int parts = red_parts_n(PI.nblk);
-  const int part = R.pbeg + (int)blockIdx.x;
+  const int part = R.pbeg + (int)blockIdx.x / kRedCl;
   if (part >= parts) return;
-  const int64_t per = (PI.nblk + parts - 1) / parts;
-  const int64_t b0 = PI.blk_off + part * per;
-  const int64_t b1 = min(PI.blk_off + PI.nblk, b0 + per);
-  double acc[kMaxP + 1];
-  for (int i = 0; i <= np; ++i) acc[i] = 0.0;
+  int64_t b0, b1;
+  red_range(PI, parts, part, rank, b0, b1);
+  double acc[PR + 1];
+#pragma unroll
+  for (int i = 0; i <= PR; ++i) acc[i] = 0.0;
   for (int64_t b = b0 + threadIdx.x; b < b1; b += blockDim.x) {
     const double* c = R.cache + b * R.CS;
     double zK = c[2 + q];
     for (int i = 0; i < q; ++i) zK -= c[3 + q + i] * sbeta[i];
-    acc[0] -= 0.5 * (2.0 * log(c[0]) + zK * zK);
+    const double zz = zK * zK;
+    acc[0] += zz;
     if (R.need_grad) {
       const double* wK = c + 3 + 2 * q;
       const double* wzy = wK + P;
       const double* wzZ = wzy + P;
-      for (int pp = 0; pp < P; ++pp) {
-        double wz = wzy[pp];
-        for (int i = 0; i < q; ++i) wz -= wzZ[pp * q + i] * sbeta[i];
-        acc[1 + pp] -= 0.5 * (wK[pp] * (1.0 + zK * zK) - 2.0 * zK * wz);
-      }
+#pragma unroll
+      for (int pp = 0; pp < PR; ++pp)
+        if (pp < P) {
+          double wz = wzy[pp];
+          for (int i = 0; i < q; ++i) wz -= wzZ[pp * q + i] * sbeta[i];
+          acc[1 + pp] -= 0.5 * (wK[pp] * (1.0 + zz) - 2.0 * zK * wz);
+        }
     }
   }
   // fixed-order block reduction
   const int w = threadIdx.x >> 5, ln = threadIdx.x & 31;
-  for (int i = 0; i <= np; ++i) {
-    double v = acc[i];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (ln == 0) red[w][i] = v;
-  }
+#pragma unroll
+  for (int i = 0; i <= PR; ++i)
+    if (i <= np) {
+      double v = acc[i];
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+      if (ln == 0) red[w][i] = v;
+    }
   __syncthreads();
   for (int i = threadIdx.x; i <= np; i += blockDim.x) {
     double s = 0.0;
     for (int k = 0; k < (int)(blockDim.x >> 5); ++k) s += red[k][i];
-    R.part2[((int64_t)p * R.parts + part) * (R.Pmax + 1) + i] = s;
+    tot[i] = s;
   }
+  cl.sync();
+  if (rank == 0)
+    for (int i = threadIdx.x; i <= np; i += blockDim.x) {
+      double s = 0.0;
+#pragma unroll
+      for (int c = 0; c < kRedCl; ++c) s += cl.map_shared_rank(tot, c)[i];
+      R.part2[((int64_t)p * R.parts + part) * (R.Pmax + 1) + i] = s;
+    }
+  cl.sync();  // the others' shared memory stays until it has been read
 }
 
 __global__ void k_final2(RedArgs R) {
@@ -816,49 +885,49 @@ __global__ void k_final2(RedArgs R) {
   const int P = PI.P, q = PI.q, np = R.need_grad ? P : 0;
   __shared__ double tot[kMaxP + 1];
   const int parts = red_parts_n(PI.nblk);
-  for (int i = threadIdx.x; i <= np; i += blockDim.x) {
+  // a warp per entry at a time, a lane every 32nd partition, added up in lane
+  // order
+  const int nw = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int i = w; i <= np; i += nw) {
     double s = 0.0;
     const double* src = R.part2 + (int64_t)p * R.parts * (R.Pmax + 1) + i;
-#pragma unroll 8
-    for (int c = 0; c < parts; ++c) s += src[(int64_t)c * (R.Pmax + 1)];
-    tot[i] = s;
+#pragma unroll 4
+    for (int c = lane; c < parts; c += 32) s += src[(int64_t)c * (R.Pmax + 1)];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) tot[i] = s;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double* out = R.out + (int64_t)p * R.ostride;
-    const double* sums = R.sums + (int64_t)p * R.nfmax;
-    const double* th = R.theta + (int64_t)p * R.tstride;
-    // ll = -n/2 log(2pi) - sum_b (log L_KK + z_K^2 / 2)  (likelihood.py:149-156)
-    double ll = -0.5 * (double)PI.n * 1.8378770664093453 + tot[0];
-    double g0 = np ? tot[1] : 0.0;
-    double f00_add = 0.0;
-    if (PI.var_penalty > 0.0) {  // likelihood.py:165-171
-      double excess = th[0] - PI.log_var_target;
-      if (excess < 0.0) excess = 0.0;
-      ll -= 0.5 * PI.var_penalty * excess * excess;
-      g0 -= PI.var_penalty * excess;
-      if (excess > 0.0) f00_add = PI.var_penalty;
-    }
-    out[0] = ll;
-    if (np) {
-      out[1] = g0;
-      for (int pp = 1; pp < P; ++pp) out[1 + pp] = tot[1 + pp];
-      // Fisher: sums hold the packed lower triangle
-      double* fish = out + 1 + P;
-      const int foff = 1 + q + q * q;
-      for (int i = 0; i < P; ++i)
-        for (int j = 0; j <= i; ++j) {
-          const double v = sums[foff + i * (i + 1) / 2 + j];
-          fish[i * P + j] = v;
-          fish[j * P + i] = v;
-        }
-      fish[0] += f00_add;
-    } else {
-      for (int i = 0; i < P + P * P; ++i) out[1 + i] = 0.0;
-    }
-    double* bo = out + 1 + P + P * P;
-    for (int i = 0; i < q; ++i) bo[i] = R.beta[(int64_t)p * (R.qmax + 1) + i];
+  double* out = R.out + (int64_t)p * R.ostride;
+  const double* th = R.theta + (int64_t)p * R.tstride;
+  // variance penalty (likelihood.py:165-171)
+  double ll_pen = 0.0, g0_pen = 0.0, f00_add = 0.0;
+  if (PI.var_penalty > 0.0) {
+    double excess = th[0] - PI.log_var_target;
+    if (excess < 0.0) excess = 0.0;
+    ll_pen = 0.5 * PI.var_penalty * excess * excess;
+    g0_pen = PI.var_penalty * excess;
+    if (excess > 0.0) f00_add = PI.var_penalty;
   }
+  if (threadIdx.x == 0) {
+    // ll = -n/2 log(2pi) - sum_b (log L_KK + z_K^2 / 2)  (likelihood.py:149-156)
+    out[0] = -0.5 * (double)PI.n * 1.8378770664093453 - (R.sums[(int64_t)p * R.nfmax] + 0.5 * tot[0]) - ll_pen;
+  }
+  if (np) {
+    const double* sums = R.sums + (int64_t)p * R.nfmax;
+    for (int pp = threadIdx.x; pp < P; pp += blockDim.x) out[1 + pp] = tot[1 + pp] - (pp == 0 ? g0_pen : 0.0);
+    // Fisher: sums hold the packed lower triangle
+    double* fish = out + 1 + P;
+    const int foff = 1 + q + q * q;
+    for (int t = threadIdx.x; t < P * P; t += blockDim.x) {
+      const int i = t / P, j = t - (t / P) * P;
+      const int hi = i > j ? i : j, lo = i > j ? j : i;
+      fish[t] = sums[foff + hi * (hi + 1) / 2 + lo] + (t == 0 ? f00_add : 0.0);
+    }
+  } else {
+    for (int i = threadIdx.x; i < P + P * P; i += blockDim.x) out[1 + i] = 0.0;
+  }
+  double* bo = out + 1 + P + P * P;
+  for (int i = threadIdx.x; i < q; i += blockDim.x) bo[i] = R.beta[(int64_t)p * (R.qmax + 1) + i];
 }
 
 }  // namespace sv
@@ -987,6 +1056,9 @@ int launch_team_kernel(Kern kern, LikArgs A, int kt, int tw, int max_teams, cuda
 }
 
 int launch_warp_kernel(LikArgs A, cudaStream_t st) {
+  // (the jitter fix-up, seldom with work, in one launch: a block's bits do not
+  // depend on its team's width)
+  if (A.fixup) return launch_team_kernel(k_block_warp, A, 32, 32, 16, st);
   int rc = launch_team_kernel(k_block_half, A, 16, 16, 32, st);
   if (rc != SV_OK) return rc;
   return launch_team_kernel(k_block_warp, A, 32, 32, 16, st);
@@ -1194,7 +1266,7 @@ int run_eval(const EvalCall& C, cudaStream_t st, const ShardStage* sh = nullptr)
   R.parts = parts;
   R.pbeg = sh ? sh->pb : 0;
   const int npart = sh ? sh->pe - sh->pb : parts;
-  const dim3 rgrid((unsigned)(npart > 0 ? npart : 1), (unsigned)S.nprob);
+  const dim3 rgrid((unsigned)(npart > 0 ? npart * kRedCl : 1), (unsigned)S.nprob);
   if (stage == 0 || stage == 2) {
     int rwarps = kRedThreads / 32;
     while (rwarps > 1 && sizeof(double) * (size_t)rwarps * W.nfmax > (size_t)max_smem_optin()) --rwarps;
@@ -1210,12 +1282,24 @@ int run_eval(const EvalCall& C, cudaStream_t st, const ShardStage* sh = nullptr)
     k_final1<<<(unsigned)S.nprob, kRedThreads, 0, st>>>(R);
     SV_CUDA_TRY(cudaGetLastError());
     if (npart > 0) {
-      k_reduce2<<<rgrid, kRedThreads, 0, st>>>(R);
+      // a thread per block of a CTA's run while the CTAs do not fill the SMs;
+      // beyond that one warp, four blocks a thread: the sums over a warp are
+      // most of the float64 work
+      const int64_t per = (S.nblk_max + parts - 1) / parts;
+      const int64_t run = (per + kRedCl - 1) / kRedCl;
+      int thr = (int64_t)npart * kRedCl * S.nprob > 2 * sv_num_sms() ? 32 : (int)((run + 31) / 32 * 32);
+      thr = std::max(32, std::min(thr, kRedThreads));
+      if (S.Pmax <= 8)
+        k_reduce2<8><<<rgrid, thr, 0, st>>>(R);
+      else if (S.Pmax <= 16)
+        k_reduce2<16><<<rgrid, thr, 0, st>>>(R);
+      else
+        k_reduce2<kMaxP><<<rgrid, thr, 0, st>>>(R);
       SV_CUDA_TRY(cudaGetLastError());
     }
   }
   if (stage == 0 || stage == 4) {
-    k_final2<<<(unsigned)S.nprob, 64, 0, st>>>(R);
+    k_final2<<<(unsigned)S.nprob, 256, 0, st>>>(R);
     SV_CUDA_TRY(cudaGetLastError());
   }
   return SV_OK;

@@ -28,9 +28,10 @@
 // Measured at n = 200,000, d = 10, m = 30: 10.2 ms, where k_block_warp takes
 // 27.3 ms; the integer multiply pipe is 65 % busy, the float64 pipe 6 %
 // (3 warps per scheduler, one block of 18 KB of shared memory each). Errors
-// against 113-bit arithmetic at n = 500 are those of the float64 form or
-// smaller (tau = 1e-2: log-likelihood 7e-16 against 1.4e-15, beta 2.3e-15
-// against 9.2e-15; tau = 1e-8 at d = 3: 8.5e-10 against 1.4e-9).
+// against 113-bit arithmetic at n = 500, m = 30 (float64 kernels in brackets):
+// tau = 1e-4, d = 8: log-likelihood 1e-17 (1.9e-14), score 2e-15 (3e-14),
+// Fisher 3e-16 (5e-15); tau = 1e-8, d = 3: 9e-11 (1.4e-9), 1.2e-10 (1.6e-9),
+// 1.3e-11 (1.4e-10).
 //
 // What has no such bound goes to the float64 kernels: a block with a pivot
 // below 2^-34 of the diagonal (its jitter ladder is theirs), coordinates
@@ -511,6 +512,11 @@ int launch_fix_g(const LikArgs& A, int kmin, int maxsm, cudaStream_t st) {
                fixed = 256 * sizeof(double);
   int wpc = kFixThreads / 32;
   while (wpc > 1 && fixed + wpc * per_warp > (size_t)maxsm) --wpc;
+  // no more warps per CTA than the fewest rounds over the SMs need: a block is
+  // a long chain, and 500 of them on 42 SMs take 107 us, on all SMs less
+  const int64_t share = (A.b1 - A.b0 + (int64_t)(32 / G) * sv_num_sms() - 1) / ((int64_t)(32 / G) * sv_num_sms());
+  const int64_t rounds = (share + wpc - 1) / wpc;
+  if (rounds > 0) wpc = (int)((share + rounds - 1) / rounds);
   const size_t smem = fixed + wpc * per_warp;
   if (smem > (size_t)maxsm) return SV_EINVAL;
   SV_CUDA_TRY(cudaFuncSetAttribute(k_block_fix<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
