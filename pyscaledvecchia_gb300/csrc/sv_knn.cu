@@ -352,44 +352,38 @@ __device__ __forceinline__ void wq_exact_sort(const WqSmem& S, int w, int n, con
     }
 }
 
-// One tile of nw = blockDim.x / 32 query rows: rows [qt nw, qt nw + nw), a
-// warp each.
-template <int DP>
-__device__ __forceinline__ void knn_wq_tile(const KnnArgs& A, int64_t qt, unsigned char* smraw) {
-  const int nw = blockDim.x >> 5;
-  const int cap = A.wq_cap, sortw = A.wq_sort;
+// A query's superset (shared by the warp): bounds and indices in the warp's
+// part of S, cnt entries; Tq = tau' + B_q, +inf until the first filter.
+struct WqList {
   WqSmem S;
-  S.tv = (float*)smraw;
-  S.tB = S.tv + (size_t)kWqC * DP;
-  S.bh = S.tB + kWqC;
-  S.bl = S.bh + (size_t)nw * cap;
-  S.bi = (int*)(S.bl + (size_t)nw * cap);
-  S.bs = (double*)(S.bi + (size_t)nw * cap);  // 8-byte aligned: cap is a multiple of 32
-  S.bsi = (int*)(S.bs + (size_t)nw * sortw);
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float* bh = S.bh + (size_t)w * cap;
-  float* bl = S.bl + (size_t)w * cap;
-  int* bi = S.bi + (size_t)w * cap;
-  const int64_t i = qt * nw + w;
-  const bool valid = i < A.nq;
-  int kq = A.k;
-  if (A.ordered) kq = (int)min((int64_t)A.m, i);
-  bool active = valid && kq > 0;
-  if (A.ordered && i < A.start) active = false;
+  float *bh, *bl;
+  int* bi;
+  const double *xq, *Xr;
+  int w, cap, sortw, kq, d, cnt;
+  float Bi, Tq;
 
-  float qv[DP];
-  float Bi = 0.0f;
-#pragma unroll
-  for (int l = 0; l < DP; ++l) qv[l] = valid ? A.vq[i * DP + l] : 0.0f;
-  if (valid) Bi = A.Bq[i];
-  const double* xq = A.Xq + (valid ? i : 0) * A.d;
-  int cnt = 0;
-  float Tq = __int_as_float(0x7f800000);  // tau' + B_q: +inf until a filter
-  const float g = A.growth;
+  __device__ __forceinline__ void init(const WqSmem& S_, int w_, int cap_, int sortw_, int kq_, float Bi_,
+                                       const double* xq_, const double* Xr_, int d_) {
+    S = S_;
+    w = w_;
+    cap = cap_;
+    sortw = sortw_;
+    kq = kq_;
+    Bi = Bi_;
+    xq = xq_;
+    Xr = Xr_;
+    d = d_;
+    bh = S.bh + (size_t)w * cap;
+    bl = S.bl + (size_t)w * cap;
+    bi = S.bi + (size_t)w * cap;
+    cnt = 0;
+    Tq = __int_as_float(0x7f800000);
+  }
 
   // filter the superset against tau (the kq-th smallest hi); if ties keep it
   // nearly full, keep the kq first by exact (key, index)
-  auto compact = [&]() {
+  __device__ __forceinline__ void compact() {
+    const int lane = threadIdx.x & 31;
     const float tau = wq_kth(bh, cnt, kq);
     const float taum = __fmul_ru(tau, 1.0f + 0x1p-20f);
     int nc = 0;
@@ -418,7 +412,7 @@ __device__ __forceinline__ void knn_wq_tile(const KnnArgs& A, int64_t qt, unsign
     cnt = nc;
     Tq = __fadd_ru(taum, Bi);
     if (cnt > cap - 2 * 32) {
-      wq_exact_sort(S, w, cnt, xq, A.Xr, A.d, cap, sortw);
+      wq_exact_sort(S, w, cnt, xq, Xr, d, cap, sortw);
       const double* bs = S.bs + (size_t)w * sortw;
       const int* bsi = S.bsi + (size_t)w * sortw;
       for (int e = lane; e < kq; e += 32) {
@@ -432,7 +426,68 @@ __device__ __forceinline__ void knn_wq_tile(const KnnArgs& A, int64_t qt, unsign
       const float tau2 = bh[kq - 1];  // the kq-th exact root, rounded up
       Tq = __fadd_ru(__fmul_ru(tau2, 1.0f + 0x1p-20f), Bi);
     }
-  };
+  }
+
+  // one candidate per lane (in: it has one): kept unless lo > tau', i.e.
+  // sqrt(s32 / g) > Tq + B_c
+  __device__ __forceinline__ void add(bool in, float s32, float Bc, int id, float g) {
+    const int lane = threadIdx.x & 31;
+    auto keep_of = [&]() {
+      if (!in) return false;
+      const float tb = __fadd_ru(Tq, Bc);
+      return !(s32 > __fmul_ru(__fmul_ru(tb, tb), g));
+    };
+    bool keep = keep_of();
+    unsigned km = __ballot_sync(0xffffffffu, keep);
+    if (!km) return;
+    if (cnt + __popc(km) > cap) {
+      compact();
+      keep = keep_of();
+      km = __ballot_sync(0xffffffffu, keep);
+    }
+    if (keep) {
+      const int p = cnt + __popc(km & ((1u << lane) - 1));
+      const float bsum = __fadd_ru(Bi, Bc);
+      bh[p] = __fadd_ru(__fsqrt_ru(__fmul_ru(s32, g)), bsum);
+      bl[p] = __fsub_rd(__fsqrt_rd(__fdiv_rd(s32, g)), bsum);
+      bi[p] = id;
+    }
+    cnt += __popc(km);
+    __syncwarp();
+  }
+};
+
+// One tile of nw = blockDim.x / 32 query rows: rows [qt nw, qt nw + nw), a
+// warp each.
+template <int DP>
+__device__ __forceinline__ void knn_wq_tile(const KnnArgs& A, int64_t qt, unsigned char* smraw) {
+  const int nw = blockDim.x >> 5;
+  const int cap = A.wq_cap, sortw = A.wq_sort;
+  WqSmem S;
+  S.tv = (float*)smraw;
+  S.tB = S.tv + (size_t)kWqC * DP;
+  S.bh = S.tB + kWqC;
+  S.bl = S.bh + (size_t)nw * cap;
+  S.bi = (int*)(S.bl + (size_t)nw * cap);
+  S.bs = (double*)(S.bi + (size_t)nw * cap);  // 8-byte aligned: cap is a multiple of 32
+  S.bsi = (int*)(S.bs + (size_t)nw * sortw);
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t i = qt * nw + w;
+  const bool valid = i < A.nq;
+  int kq = A.k;
+  if (A.ordered) kq = (int)min((int64_t)A.m, i);
+  bool active = valid && kq > 0;
+  if (A.ordered && i < A.start) active = false;
+
+  float qv[DP];
+  float Bi = 0.0f;
+#pragma unroll
+  for (int l = 0; l < DP; ++l) qv[l] = valid ? A.vq[i * DP + l] : 0.0f;
+  if (valid) Bi = A.Bq[i];
+  const double* xq = A.Xq + (valid ? i : 0) * A.d;
+  WqList L;
+  L.init(S, w, cap, sortw, kq, Bi, xq, A.Xr, A.d);
+  const float g = A.growth;
 
   int64_t cend = A.nr;
   if (A.ordered) cend = min(A.nq, (qt + 1) * nw);  // rows < last query of the tile
@@ -469,36 +524,14 @@ __device__ __forceinline__ void knn_wq_tile(const KnnArgs& A, int64_t qt, unsign
         }
         Bc = S.tB[cc];
       }
-      // keep unless lo > tau': sqrt(s32 / g) > Tq + B_c
-      auto keep_of = [&]() {
-        if (!in) return false;
-        const float tb = __fadd_ru(Tq, Bc);
-        return !(s32 > __fmul_ru(__fmul_ru(tb, tb), g));
-      };
-      bool keep = keep_of();
-      unsigned km = __ballot_sync(0xffffffffu, keep);
-      if (!km) continue;
-      if (cnt + __popc(km) > cap) {
-        compact();
-        keep = keep_of();
-        km = __ballot_sync(0xffffffffu, keep);
-      }
-      if (keep) {
-        const int p = cnt + __popc(km & ((1u << lane) - 1));
-        const float bsum = __fadd_ru(Bi, Bc);
-        bh[p] = __fadd_ru(__fsqrt_ru(__fmul_ru(s32, g)), bsum);
-        bl[p] = __fsub_rd(__fsqrt_rd(__fdiv_rd(s32, g)), bsum);
-        bi[p] = (int)(c0 + cc);
-      }
-      cnt += __popc(km);
-      __syncwarp();
+      L.add(in, s32, Bc, (int)(c0 + cc), g);
     }
   }
   if (!valid) return;
   int nout = 0;
-  if (active && cnt > 0) {
-    wq_exact_sort(S, w, cnt, xq, A.Xr, A.d, cap, sortw);
-    nout = min(cnt, kq);
+  if (active && L.cnt > 0) {
+    wq_exact_sort(S, w, L.cnt, xq, A.Xr, A.d, cap, sortw);
+    nout = min(L.cnt, kq);
   }
   const int* bsi = S.bsi + (size_t)w * sortw;
   if (A.nbr) {
@@ -557,6 +590,242 @@ __global__ void __launch_bounds__(256) k_knn_wq_batched(const KnnBatchProb* prob
   knn_wq_tile<DP>(A, te.y, smraw);
 }
 
+// ---------------------------------------------------------------------------
+// Large sets: the warp-per-query search over a box tree.
+//
+// The screens above visit every reference row (n = 200,000, m = 30: 133 ms,
+// most of it float64 work of single lanes, one insertion at a time). Here the
+// rows are put in k-d order once, at most 64 to a tile (a segment of the order)
+// and 32 tiles to a super-tile, each with the bounding box of its float32
+// images. A warp owns a query and
+// takes the super-tiles nearest first, within one its tiles nearest first,
+// leaving out a box whose lower bound (gaps and their squares rounded down)
+// passes the screen against the current threshold: every row inside it would.
+// What it keeps, filters and sorts at the end is the superset of the search
+// above, so the result is the same exact (distance, index) order whatever the
+// order of the visits. An ordered search (row i among rows j < i) drops rows
+// j >= i one by one and boxes without an earlier row as a whole.
+// ---------------------------------------------------------------------------
+constexpr int kKtTile = 64;
+constexpr int kKtSuper = 32;        // tiles per super-tile
+constexpr int kKtHead = 4096;       // ordered: rows before this one take the screens above
+
+struct KnnTree {
+  const float* v;      // reference images in tree order [n][DP]
+  const float* B;      // their bounds
+  const int* id;       // their rows
+  const float *lo, *hi, *tB;   // tiles: boxes, largest bound,
+  const int* tmin;             // smallest row
+  const float *slo, *shi, *sB; // super-tiles
+  const int* smin;
+  int64_t n;
+  int ntile, nsuper;   // a power of two
+};
+
+// tile boxes from the rows (leaf = 1), super-tile boxes from the tiles; a NaN
+// image opens its box to everything
+template <int DP>
+__global__ void k_kt_boxes(const float* clo, const float* chi, const float* cB, const int* cid, int64_t nc,
+                           int per, int64_t nn, float* lo, float* hi, float* Bm, int* imin) {
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nn * DP;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t j = e / DP;
+    const int l = (int)(e - j * DP);
+    // per = 0: the tiles' segments of the rows
+    const int64_t c0 = per ? j * per : j * nc / nn, c1 = per ? min(c0 + per, nc) : (j + 1) * nc / nn;
+    const float inf = __int_as_float(0x7f800000);
+    float a = inf, b = -inf, bm = 0.0f;
+    int im = 0x7fffffff;
+    bool nan = false;
+    for (int64_t c = c0; c < c1; ++c) {
+      const float x = clo[c * DP + l], y = chi[c * DP + l];
+      nan = nan || x != x || y != y;
+      a = fminf(a, x);
+      b = fmaxf(b, y);
+      if (l == 0) {
+        const float t = cB[c];
+        bm = (t > bm || t != t) ? t : bm;
+        im = min(im, cid[c]);
+      }
+    }
+    lo[e] = nan ? -inf : a;
+    hi[e] = nan ? inf : b;
+    if (l == 0) {
+      Bm[j] = bm;
+      imin[j] = im;
+    }
+  }
+}
+
+template <int DP>
+__global__ void k_kt_gather(const float* v0, const float* B0, const int* ids, int64_t n, float* v, float* B) {
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n * DP;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t p = e / DP;
+    v[e] = v0[(int64_t)ids[p] * DP + (e - p * DP)];
+    if (e == p * DP) B[p] = B0[ids[p]];
+  }
+}
+
+__global__ void k_kt_iota(int* ids, int64_t n) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    ids[i] = (int)i;
+}
+
+// squared distance of the image qv to a box, rounded down
+template <int DP>
+__device__ __forceinline__ float kt_box2(const float (&qv)[DP], const float* lo, const float* hi) {
+  float s = 0.0f;
+#pragma unroll
+  for (int l = 0; l < DP; l += 4) {
+    const float4 a = *reinterpret_cast<const float4*>(lo + l), b = *reinterpret_cast<const float4*>(hi + l);
+    auto add = [&](float q, float x, float y) {
+      const float g = fmaxf(fmaxf(__fsub_rd(x, q), __fsub_rd(q, y)), 0.0f);
+      s = __fadd_rd(s, __fmul_rd(g, g));
+    };
+    add(qv[l], a.x, b.x);
+    add(qv[l + 1], a.y, b.y);
+    add(qv[l + 2], a.z, b.z);
+    add(qv[l + 3], a.w, b.w);
+  }
+  return s;
+}
+
+template <int DP>
+__global__ void __launch_bounds__(256) k_knn_tree(KnnArgs A, KnnTree R) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int nw = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned full = 0xffffffffu;
+  WqSmem S;
+  S.tv = S.tB = nullptr;
+  S.bs = (double*)smraw;
+  S.bsi = (int*)(S.bs + (size_t)nw * A.wq_sort);
+  S.bh = (float*)(S.bsi + (size_t)nw * A.wq_sort);
+  S.bl = S.bh + (size_t)nw * A.wq_cap;
+  S.bi = (int*)(S.bl + (size_t)nw * A.wq_cap);
+  const int64_t pos = (int64_t)blockIdx.x * nw + w;
+  if (pos >= A.nq) return;
+  // an ordered search takes its queries in tree order (neighbouring warps
+  // visit the same tiles)
+  const int64_t i = A.ordered ? (int64_t)R.id[pos] : pos;
+  if (A.ordered && i < kKtHead) return;
+  if (A.ordered && i < A.start) {  // not asked for: no neighbours
+    int64_t* row = A.out + i * (int64_t)(A.m + 1);
+    for (int c = lane; c <= A.m; c += 32) row[c] = c == 0 ? i : -1;
+    return;
+  }
+  const int kq = A.ordered ? (int)min((int64_t)A.m, i) : A.k;
+  const float* vp = A.ordered ? R.v + pos * DP : A.vq + pos * DP;
+  float qv[DP];
+#pragma unroll
+  for (int l = 0; l < DP; ++l) qv[l] = vp[l];
+  const float Bi = A.ordered ? R.B[pos] : A.Bq[pos];
+  WqList L;
+  L.init(S, w, A.wq_cap, A.wq_sort, kq, Bi, A.Xq + i * A.d, A.Xr, A.d);
+  const float g = A.growth;
+  const int before = A.ordered ? (int)i : 0x7fffffff;  // rows j < before
+  // whether a box at squared distance s with bound Bm is beyond the threshold
+  auto beyond = [&](float s, float Bm) {
+    const float tb = __fadd_ru(L.Tq, Bm);
+    return s > __fmul_ru(__fmul_ru(tb, tb), g);
+  };
+  auto visit = [&](int64_t t) {
+    const int64_t p0 = t * R.n / R.ntile, p1 = (t + 1) * R.n / R.ntile;
+#pragma unroll
+    for (int h = 0; h < kKtTile; h += 32) {
+      const int64_t p = p0 + h + lane;
+      const int id = p < p1 ? R.id[p] : 0x7fffffff;
+      const bool in = p < p1 && id < before;
+      float s32 = 0.0f, Bc = 0.0f;
+      if (in) {
+        const float* tv = R.v + p * DP;
+#pragma unroll
+        for (int l = 0; l < DP; l += 4) {
+          const float4 t4 = *reinterpret_cast<const float4*>(tv + l);
+          float df = __fsub_rn(qv[l], t4.x);
+          s32 = __fmaf_rn(df, df, s32);
+          df = __fsub_rn(qv[l + 1], t4.y);
+          s32 = __fmaf_rn(df, df, s32);
+          df = __fsub_rn(qv[l + 2], t4.z);
+          s32 = __fmaf_rn(df, df, s32);
+          df = __fsub_rn(qv[l + 3], t4.w);
+          s32 = __fmaf_rn(df, df, s32);
+        }
+        Bc = R.B[p];
+      }
+      L.add(in, s32, Bc, id, g);
+    }
+  };
+  // the tiles of super-tile s, nearest first
+  auto super = [&](int s) {
+    const int t = s * kKtSuper + lane;
+    float dt = 0.0f, Bt = 0.0f;
+    bool left = t < R.ntile && R.tmin[t] < before;
+    if (left) {
+      dt = kt_box2<DP>(qv, R.lo + (int64_t)t * DP, R.hi + (int64_t)t * DP);
+      Bt = R.tB[t];
+    }
+    while (true) {
+      left = left && !beyond(dt, Bt);
+      const unsigned key = left ? __float_as_uint(dt) : 0xffffffffu;
+      const unsigned mk = __reduce_min_sync(full, key);
+      if (mk == 0xffffffffu) break;
+      const int src = __ffs(__ballot_sync(full, key == mk)) - 1;
+      visit(s * kKtSuper + src);
+      if (lane == src) left = false;
+    }
+  };
+  // the super-tiles, 32 at a time, nearest first; those of the query's own
+  // neighbourhood before all others
+  int home = A.ordered ? (int)((((pos + 1) * R.ntile - 1) / R.n) / kKtSuper) : 0;
+  if (!A.ordered) {
+    unsigned best = 0xffffffffu;
+    for (int s0 = 0; s0 < R.nsuper; s0 += 32) {
+      const int s = s0 + lane;
+      const unsigned key = s < R.nsuper
+          ? __float_as_uint(kt_box2<DP>(qv, R.slo + (int64_t)s * DP, R.shi + (int64_t)s * DP)) : 0xffffffffu;
+      const unsigned mk = __reduce_min_sync(full, key);
+      if (mk < best) {
+        best = mk;
+        home = s0 + __ffs(__ballot_sync(full, key == mk)) - 1;
+      }
+    }
+  }
+  super(home);
+  for (int s0 = 0; s0 < R.nsuper; s0 += 32) {
+    const int s = s0 + lane;
+    bool left = s < R.nsuper && s != home && R.smin[s] < before;
+    float ds = 0.0f, Bs = 0.0f;
+    if (left) {
+      ds = kt_box2<DP>(qv, R.slo + (int64_t)s * DP, R.shi + (int64_t)s * DP);
+      Bs = R.sB[s];
+    }
+    while (true) {
+      left = left && !beyond(ds, Bs);
+      const unsigned key = left ? __float_as_uint(ds) : 0xffffffffu;
+      const unsigned mk = __reduce_min_sync(full, key);
+      if (mk == 0xffffffffu) break;
+      const int src = __ffs(__ballot_sync(full, key == mk)) - 1;
+      super(s0 + src);
+      if (lane == src) left = false;
+    }
+  }
+  int nout = 0;
+  if (L.cnt > 0) {
+    wq_exact_sort(S, w, L.cnt, L.xq, A.Xr, A.d, A.wq_cap, A.wq_sort);
+    nout = min(L.cnt, kq);
+  }
+  const int* bsi = S.bsi + (size_t)w * A.wq_sort;
+  if (A.ordered) {
+    int64_t* row = A.out + i * (int64_t)(A.m + 1);
+    if (lane == 0) row[0] = i;
+    for (int c = lane; c < A.m; c += 32) row[1 + c] = c < nout ? (int64_t)bsi[c] : -1;
+  } else {
+    int64_t* row = A.out + i * (int64_t)A.k;
+    for (int c = lane; c < A.k; c += 32) row[c] = c < nout ? (int64_t)bsi[c] : -1;
+  }
+}
+
 static int pad_dim(int d) {
   if (d <= 4) return 4;
   if (d <= 8) return 8;
@@ -599,7 +868,7 @@ static bool wq_plan(int k, int DP, int* warps, size_t* smem) {
 // the warp-per-query search: for large k, and for moderate k while the
 // candidate sets are small enough that list insertions, not the screen,
 // dominate the per-thread search (measured: 4x faster at n = 20k, m = 20;
-// 15 % slower at n = 200k, m = 30)
+// 15 % slower at n = 200k, m = 30, which the tree search below now takes)
 static bool use_wq(int k, int64_t nr, int DP) {
   if (!wq_plan(k, DP, nullptr, nullptr)) return false;
   return k >= kKnnHeapMin || (k >= 16 && nr <= 65536);
@@ -656,7 +925,107 @@ static int launch_knn(const KnnArgs& A, int DP, int64_t grid, size_t smem, cudaS
   return SV_OK;
 }
 
+// ---- tree search: scratch, build and launch
 static size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
+
+// rows from which the tree search is taken (below, the screens of all rows
+// take less than building the tree)
+constexpr int64_t kKtMinRows = 16384;
+
+static int kt_levels(int64_t n) {
+  int L = 5;  // at least one super-tile of 32 tiles
+  while (((n + ((int64_t)1 << L) - 1) >> L) > kKtTile) ++L;
+  return L;
+}
+// and the queries from which it is, for smaller sets: the screens take one pass
+// over the rows while every query has a warp of its own (16 to an SM). Measured
+// at d = 6, k = 140: 1,500 queries of 60,000 rows 1.33 ms by the tree, 1.36 by
+// the screens (of 30,000: 1.04, 0.85), 4,000 queries 1.35, 2.60 (1.11, 1.60);
+// 50 of 100,000 1.45, 1.81. 200,000 ordered rows, d = 10, m = 30: 8.4, 134 ms;
+// 20,000 queries of 100,000: 2.2, 15.8 ms; no slower where every input counts
+// (100,000 ordered rows, d = 10, no range above 0.1: 25.7, 55 ms)
+static bool kt_use(int k, int64_t n, int64_t nq, int DP) {
+  return n >= kKtMinRows && n <= 0x7fffffffLL && (n >= 65536 || nq > 16LL * sv_num_sms()) &&
+         wq_plan(k, DP, nullptr, nullptr);
+}
+static size_t kt_bytes(int64_t n, int d, int DP) {
+  if (n < kKtMinRows || DP > 16) return 0;
+  const size_t S = (size_t)1 << kt_levels(n), N = (size_t)n;
+  return 2 * al256(8 * N) + 2 * al256(4 * N) + 2 * al256(4 * S * d) + al256(kd_sort_reserve(n)) +
+         al256(4 * N * DP) + al256(4 * N) + 2 * al256(4 * S * DP) + 2 * al256(4 * S) +
+         2 * al256(4 * (S / kKtSuper) * DP) + 2 * al256(4 * (S / kKtSuper));
+}
+
+// superset capacity of the tree search: the first tiles are the nearest, so
+// little beyond k is worth keeping before a filter
+static int kt_cap(int k) { return ((k + 96 + 31) / 32) * 32; }
+
+template <int DP>
+static int kt_run(const KnnArgs& A0, int warps, char* ws, cudaStream_t st) {
+  const int64_t n = A0.nr;
+  const int L = kt_levels(n), S = 1 << L;
+  auto take = [&](size_t bytes) -> char* {
+    char* p = ws;
+    ws += al256(bytes);
+    return p;
+  };
+  unsigned long long* keys0 = (unsigned long long*)take(8 * (size_t)n);
+  unsigned long long* keys1 = (unsigned long long*)take(8 * (size_t)n);
+  int* ids0 = (int*)take(4 * (size_t)n);
+  int* ids1 = (int*)take(4 * (size_t)n);
+  unsigned* mn = (unsigned*)take(4 * (size_t)S * A0.d);
+  unsigned* mx = (unsigned*)take(4 * (size_t)S * A0.d);
+  const size_t sort_bytes = kd_sort_reserve(n);
+  void* tmp = take(sort_bytes);
+  float* v = (float*)take(4 * (size_t)n * DP);
+  float* B = (float*)take(4 * (size_t)n);
+  float* lo = (float*)take(4 * (size_t)S * DP);
+  float* hi = (float*)take(4 * (size_t)S * DP);
+  float* tB = (float*)take(4 * (size_t)S);
+  int* tmin = (int*)take(4 * (size_t)S);
+  const int ns = S / kKtSuper;
+  float* slo = (float*)take(4 * (size_t)ns * DP);
+  float* shi = (float*)take(4 * (size_t)ns * DP);
+  float* sB = (float*)take(4 * (size_t)ns);
+  int* smin = (int*)take(4 * (size_t)ns);
+  const unsigned grid = (unsigned)min(8LL * sv_num_sms(), (long long)((n * DP + 255) / 256));
+  k_kt_iota<<<grid, 256, 0, st>>>(ids0, n);
+  SV_CUDA_TRY(cudaGetLastError());
+  int* ids = nullptr;
+  const int rc = kd_order(A0.vr, n, A0.d, DP, L, keys0, keys1, ids0, ids1, mn, mx, tmp, sort_bytes, &ids, st);
+  if (rc != SV_OK) return rc;
+  k_kt_gather<DP><<<grid, 256, 0, st>>>(A0.vr, A0.Br, ids, n, v, B);
+  SV_CUDA_TRY(cudaGetLastError());
+  k_kt_boxes<DP><<<(unsigned)((S * DP + 255) / 256), 256, 0, st>>>(v, v, B, ids, n, 0, S, lo, hi, tB, tmin);
+  SV_CUDA_TRY(cudaGetLastError());
+  k_kt_boxes<DP><<<(unsigned)((ns * DP + 255) / 256), 256, 0, st>>>(lo, hi, tB, tmin, S, kKtSuper, ns, slo, shi,
+                                                                   sB, smin);
+  SV_CUDA_TRY(cudaGetLastError());
+  KnnTree R = {v, B, ids, lo, hi, tB, tmin, slo, shi, sB, smin, n, S, ns};
+  KnnArgs A = A0;
+  A.wq_cap = kt_cap(A.k);
+  A.wq_sort = wq_sort(A.wq_cap);
+  size_t smem = 0;
+  for (; warps > 1; --warps) {
+    smem = (size_t)warps * 12 * ((size_t)A.wq_cap + A.wq_sort);
+    if (smem <= (size_t)knn_max_smem() / 2) break;
+  }
+  smem = (size_t)warps * 12 * ((size_t)A.wq_cap + A.wq_sort);
+  SV_CUDA_TRY(cudaFuncSetAttribute(k_knn_tree<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  k_knn_tree<DP><<<(unsigned)((A.nq + warps - 1) / warps), 32 * warps, smem, st>>>(A, R);
+  SV_CUDA_TRY(cudaGetLastError());
+  return SV_OK;
+}
+
+static int launch_knn_tree(const KnnArgs& A, int DP, char* ws, cudaStream_t st) {
+  switch (DP) {
+    case 4: return kt_run<4>(A, 8, ws, st);
+    case 8: return kt_run<8>(A, 8, ws, st);
+    case 12: return kt_run<12>(A, 8, ws, st);
+    case 16: return kt_run<16>(A, 8, ws, st);
+    default: return SV_EINVAL;
+  }
+}
 
 // batched ordered search: entry t of the tile table is (problem, query tile)
 template <int DP>
@@ -763,7 +1132,7 @@ using namespace sv;
 extern "C" size_t sv_ordered_knn_workspace_bytes(int64_t n, int32_t d) {
   const int DP = pad_dim(d > 0 ? d : 1);
   return al256(sizeof(double) * 64) + al256(sizeof(float) * (size_t)(n > 0 ? n : 1) * DP) +
-         al256(sizeof(float) * (size_t)(n > 0 ? n : 1));
+         al256(sizeof(float) * (size_t)(n > 0 ? n : 1)) + kt_bytes(n, d > 0 ? d : 1, DP);
 }
 
 extern "C" size_t sv_knn_query_workspace_bytes(int64_t nref, int64_t nq, int32_t d) {
@@ -823,6 +1192,15 @@ extern "C" int sv_ordered_knn(const double* X, int64_t n, int32_t d, int32_t m, 
   A.nbr = nullptr;
   A.b0 = 0;
   A.ldnbr = 0;
+  const bool tree = m > 0 && kt_use(m, n, n - A.start, DP);
+  if (tree) {
+    // the first rows have few earlier ones, spread over all of the tree
+    A.nq = A.nr = kKtHead;
+    const int rc = launch_knn(A, DP, (kKtHead + kKnnQ - 1) / kKnnQ, smem, st);
+    if (rc != SV_OK) return rc;
+    A.nq = A.nr = n;
+    return launch_knn_tree(A, DP, (char*)B + al256(sizeof(float) * (size_t)n), st);
+  }
   const int64_t ntile = (n + kKnnQ - 1) / kKnnQ;
   return launch_knn(A, DP, ntile, smem, st);
 }
@@ -882,6 +1260,7 @@ extern "C" int sv_knn_query(const double* Xref, int64_t nref, const double* Xq, 
   A.nbr = nullptr;
   A.b0 = 0;
   A.ldnbr = 0;
+  if (kt_use(k, nref, nq, DP)) return launch_knn_tree(A, DP, (char*)Br + al256(sizeof(float) * (size_t)nref), st);
   const int64_t ntile = (nq + kKnnQ - 1) / kKnnQ;
   return launch_knn(A, DP, ntile, smem, st);
 }

@@ -895,6 +895,36 @@ static int mt_kd_levels(int64_t n) {
 // buffers; checked at run time
 static size_t mt_sort_reserve(int64_t n) { return ((size_t)32 << 20) + 16 * (size_t)n; }
 
+size_t kd_sort_reserve(int64_t n) { return mt_sort_reserve(n); }
+
+// k-d order of n rows of float32 images (DV words each, d of them used): ids0
+// holds 0 .. n-1, L levels of halving segments along their widest coordinate;
+// *ids is the buffer that holds the result
+int kd_order(const float* v0, int64_t n, int d, int DV, int L, unsigned long long* keys0,
+             unsigned long long* keys1, int* ids0, int* ids1, unsigned* mn, unsigned* mx, void* sort_tmp,
+             size_t sort_bytes, int** ids, cudaStream_t st) {
+  const unsigned grid = (unsigned)std::min<int64_t>(8LL * sv_num_sms(), (n * DV + 255) / 256 + 1);
+  cub::DoubleBuffer<unsigned long long> kbuf(keys0, keys1);
+  cub::DoubleBuffer<int> ibuf(ids0, ids1);
+  size_t tmp_need = 0;
+  SV_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmp_need, kbuf, ibuf, (int)n, 0, 64, st));
+  if (tmp_need > sort_bytes) return SV_ENOSPC;
+  for (int lev = 0; lev < L; ++lev) {
+    const int64_t S = (int64_t)1 << lev;
+    k_mt_fill_u32<<<grid, 256, 0, st>>>(mn, S * d, 0xffffffffu);
+    k_mt_fill_u32<<<grid, 256, 0, st>>>(mx, S * d, 0u);
+    k_mt_seg_minmax<<<grid, 256, 0, st>>>(v0, ibuf.Current(), n, d, DV, S, mn, mx);
+    k_mt_keys<<<grid, 256, 0, st>>>(v0, ibuf.Current(), n, d, DV, S, mn, mx, kbuf.Current());
+    SV_CUDA_TRY(cudaGetLastError());
+    int end_bit = 32;
+    while (((int64_t)1 << (end_bit - 32)) < S) ++end_bit;
+    size_t tb = sort_bytes;
+    SV_CUDA_TRY(cub::DeviceRadixSort::SortPairs(sort_tmp, tb, kbuf, ibuf, (int)n, 0, end_bit, st));
+  }
+  *ids = ibuf.Current();
+  return SV_OK;
+}
+
 size_t maximin_tree_workspace_bytes(int64_t n, int d) {
   if (n < 1) n = 1;
   const int DV = d <= 4 ? 4 : d <= 8 ? 8 : d <= 16 ? 16 : d <= 32 ? 32 : 64;
@@ -1007,26 +1037,11 @@ int maximin_tree_single(const double* X, int64_t n, int d, int64_t first, int64_
   const unsigned grid = (unsigned)std::min<int64_t>(8LL * nsm, (n * DV + 255) / 256 + 1);
   k_mt_images<<<grid, 256, 0, st>>>(X, n, d, DV, first, v0, ids0);
   SV_CUDA_TRY(cudaGetLastError());
-  // k-d order: L levels of halving
-  cub::DoubleBuffer<unsigned long long> kbuf(keys0, keys1);
-  cub::DoubleBuffer<int> ibuf(ids0, ids1);
-  size_t tmp_need = 0;
-  SV_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmp_need, kbuf, ibuf, (int)n, 0, 64, st));
-  if (tmp_need > sort_bytes) return SV_ENOSPC;
-  for (int lev = 0; lev < L; ++lev) {
-    const int64_t S = (int64_t)1 << lev;
-    k_mt_fill_u32<<<grid, 256, 0, st>>>(mn, S * d, 0xffffffffu);
-    k_mt_fill_u32<<<grid, 256, 0, st>>>(mx, S * d, 0u);
-    k_mt_seg_minmax<<<grid, 256, 0, st>>>(v0, ibuf.Current(), n, d, DV, S, mn, mx);
-    k_mt_keys<<<grid, 256, 0, st>>>(v0, ibuf.Current(), n, d, DV, S, mn, mx, kbuf.Current());
-    SV_CUDA_TRY(cudaGetLastError());
-    int end_bit = 32;
-    while (((int64_t)1 << (end_bit - 32)) < S) ++end_bit;
-    size_t tb = sort_bytes;
-    SV_CUDA_TRY(cub::DeviceRadixSort::SortPairs(sort_tmp, tb, kbuf, ibuf, (int)n, 0, end_bit, st));
-  }
+  int* ids = nullptr;
+  const int rc = kd_order(v0, n, d, DV, L, keys0, keys1, ids0, ids1, mn, mx, sort_tmp, sort_bytes, &ids, st);
+  if (rc != SV_OK) return rc;
   SV_CUDA_TRY(cudaMemsetAsync(Q.lmask, 0, 4 * (size_t)Q.nn[1], st));
-  k_mt_gather<<<grid, 256, 0, st>>>(X, v0, ibuf.Current(), n, d, DV, first, xs, v, Bp, gidx, posof, dist,
+  k_mt_gather<<<grid, 256, 0, st>>>(X, v0, ids, n, d, DV, first, xs, v, Bp, gidx, posof, dist,
                                     thr, first_pos);
   SV_CUDA_TRY(cudaGetLastError());
   for (int h = 1; h <= H; ++h) {

@@ -43,4 +43,11 @@ int maximin_tree_single(const double* X, int64_t n, int d, int64_t first, int64_
                         int32_t* info, char* ws, size_t ws_bytes, int flags, cudaStream_t st);
 size_t maximin_tree_workspace_bytes(int64_t n, int d);
 
+// k-d order of float32 images (sv_maximin_tree.cu), and the scratch its sort
+// may ask for
+size_t kd_sort_reserve(int64_t n);
+int kd_order(const float* v0, int64_t n, int d, int DV, int L, unsigned long long* keys0,
+             unsigned long long* keys1, int* ids0, int* ids1, unsigned* mn, unsigned* mx, void* sort_tmp,
+             size_t sort_bytes, int** ids, cudaStream_t st);
+
 }  // namespace sv
