@@ -15,8 +15,9 @@
 // split the problem's points; each keeps, in shared memory, the squared
 // float64 distances, float32 skip thresholds, exact coordinates and float32
 // coordinates centred on the first row.  Every decision is the reference's:
-//  * screening: a rigorous float32 bound skips a point only when the
-//    reference would not update it;
+//  * screening: a rigorous bound from bf16 images on the tensor cores, then
+//    one from float32 images, skip a point only when the reference would not
+//    update it;
 //  * update: the squared distance s_new is computed in IEEE sequential
 //    float64 exactly as ordering.py:52-57 does before its square root; the
 //    point is updated when s_new < s_stored (bit compare).  With a correctly
@@ -50,7 +51,7 @@ namespace sv {
 constexpr int kMcThreads = 512;
 constexpr int kMcWarps = kMcThreads / 32;
 constexpr int kMcSlots = 32;  // candidate slots; slot 31 holds a pivot found by a full scan
-// static shared memory of k_maximin_cluster (about 1.3 KB), rounded up: the
+// static shared memory of k_maximin_cluster (about 1.8 KB), rounded up: the
 // capacity of a cluster is computed from what is left of 227 KB
 constexpr int kMcStaticSmem = 4096;
 constexpr int kMcMaxCluster = 16;
@@ -70,12 +71,10 @@ struct RoProb {
 __host__ __device__ inline int64_t mc_point_bytes(int d, bool grid = false) {
   return 16 + (grid ? 4 : 12) * (int64_t)d;
 }
-// width of the pivot images held in registers (zero padded)
-__host__ __device__ inline int mc_dv(int d) { return d <= 4 ? 4 : d <= 8 ? 8 : d <= 16 ? 16 : d <= 32 ? 32 : 64; }
 // per-CTA shared memory before the points: candidate slots (exact and float32
-// coordinates, squared bits, index, bound), the pivot images and the work area
+// coordinates, squared bits, index, bound) and the work area
 __host__ __device__ inline int64_t mc_fixed_bytes(int d) {
-  return (int64_t)kMcSlots * (12 * d + 16) + (int64_t)kMcSlots * 4 * mc_dv(d) + kMcWorkBytes;
+  return (int64_t)kMcSlots * (12 * d + 16) + kMcWorkBytes;
 }
 
 __global__ void k_ro_info_init(int32_t* info, int nprob) {
@@ -107,7 +106,6 @@ struct McSmem {
   long long* Ub;   // [32] squared-distance bits at the start of the selection
   int* Ui;         // [32] row index
   float* UB;       // [32] float32 rounding bound of the image
-  float* Pv;       // [32][DV] images of this pass's pivots, zero padded to DV
   double* pairS;   // [31][31] exact squared distances between candidates (work area)
   long long* wlb;  // [warps][32] candidate lists (work area)
   int* wli;
@@ -127,8 +125,7 @@ __device__ __forceinline__ McSmem mc_layout(unsigned char* base, int d, int Sc, 
   L.Ub = (long long*)(base + (size_t)kMcSlots * 12 * d);
   L.Ui = (int*)(L.Ub + kMcSlots);
   L.UB = (float*)(L.Ui + kMcSlots);
-  L.Pv = (float*)(base + (size_t)kMcSlots * (12 * d + 16));
-  unsigned char* work = (unsigned char*)(L.Pv + kMcSlots * mc_dv(d));
+  unsigned char* work = base + (size_t)kMcSlots * (12 * d + 16);
   L.pairS = (double*)work;
   L.wlb = (long long*)work;
   L.wli = (int*)(work + kMcWarps * 32 * 8);
@@ -141,159 +138,182 @@ __device__ __forceinline__ McSmem mc_layout(unsigned char* base, int d, int Sc, 
   return L;
 }
 
-// exact squared distances (ordering.py:52-57) of the pivots in `mask`, in
-// pivot order, lower point p's distance; its threshold follows
-__device__ __forceinline__ void mc_exact(const McSmem& M, const int* Ps, int p, int d, unsigned mask) {
-  const double* xp = M.xs + (size_t)p * d;
-  double dp = M.dist[p];
-  const long long b0 = __double_as_longlong(dp);
-  do {
-    const int t = __ffs(mask) - 1;
-    mask &= mask - 1;
-    const double sn = sqdist_exact(xp, M.Ux + Ps[t] * d, d);
-    if (__double_as_longlong(sn) < __double_as_longlong(dp)) dp = sn;
-  } while (mask);
-  if (__double_as_longlong(dp) != b0) {
-    M.dist[p] = dp;
-    M.thr[p] = thr_sq(dp, M.Bp[p]);
-  }
-}
+// queue of (point << 5 | pivot) for the exact distances, in the work area
+constexpr int kMcQueue = kMcWorkBytes / 4;
 
-// float32 squared distance of a register image to pivot image t
-template <int DV>
-__device__ __forceinline__ float mc_s32(const float (&vp)[DV], const float4* pv) {
+// pivot e & 31 against point e >> 5: the float32 screen, then the exact
+// squared distance (ordering.py:52-57), which lowers the point's distance and
+// threshold.  The result of a pass is the smallest of its distances, so the
+// order in which the pivots are taken is free; an ordered point's -1 is below
+// any distance, and stays.
+__device__ __forceinline__ void mc_update(const McSmem& M, const int* slot, unsigned e, int Sc, int d,
+                                          float growth) {
+  const int p = (int)(e >> 5), u = slot[e & 31];
   float s32 = 0.0f;
-#pragma unroll
-  for (int q = 0; q < DV / 4; ++q) {
-    const float4 f = pv[q];
-    float df = __fsub_rn(vp[4 * q], f.x);
-    s32 = __fmaf_rn(df, df, s32);
-    df = __fsub_rn(vp[4 * q + 1], f.y);
-    s32 = __fmaf_rn(df, df, s32);
-    df = __fsub_rn(vp[4 * q + 2], f.z);
-    s32 = __fmaf_rn(df, df, s32);
-    df = __fsub_rn(vp[4 * q + 3], f.w);
+  for (int l = 0; l < d; ++l) {
+    const float df = __fsub_rn(M.v[(size_t)l * Sc + p], M.Uv[u * d + l]);
     s32 = __fmaf_rn(df, df, s32);
   }
-  return s32;
+  if (!mc_may_update(s32, *(volatile float*)(M.thr + p), M.UB[u], growth)) return;
+  const double sn = sqdist_exact(M.xs + (size_t)p * d, M.Ux + u * d, d);
+  const long long b = __double_as_longlong(sn);
+  if (atomicMin((long long*)(M.dist + p), b) > b)
+    atomicMin((int*)(M.thr + p), __float_as_int(thr_sq(sn, M.Bp[p])));  // thresholds of live points are >= 0
 }
 
-// queue of (point, pivot mask) for the exact distances, in the work area
-constexpr int kMcQueue = kMcWorkBytes / 8;
+__device__ __forceinline__ uint32_t mc_bf16x2(float a, float b, float& sq) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+  const float fa = __uint_as_float(r << 16), fb = __uint_as_float(r & 0xffff0000u);
+  sq = fmaf(fa, fa, fmaf(fb, fb, sq));
+  return r;
+}
 
-// after the screen of point p: ordered if it is a pivot of this pass
-// (ordering.py:58); else the pivots in `mask` go to the queue (processed by
-// dense warps: a float64 warp instruction costs the same with one lane
-// active as with 32), or are applied here when the queue is full
-__device__ __forceinline__ void mc_screened(const McSmem& M, const int* Ps, int* qn, int p, int d,
-                                            bool hit, unsigned mask) {
-  if (hit) {
-    M.dist[p] = -1.0;
-    mask = 0;
-  }
-  const unsigned act = __activemask();
-  const unsigned want = __ballot_sync(act, mask != 0);
-  if (!want) return;
-  const int leader = __ffs(want) - 1;
-  const int lane = threadIdx.x & 31;
-  int base = 0;
-  if (lane == leader) base = atomicAdd(qn, __popc(want));
-  base = __shfl_sync(act, base, leader);
-  if (mask) {
-    const int slot = base + __popc(want & ((1u << lane) - 1));
-    if (slot < kMcQueue) {
-      int2* q = reinterpret_cast<int2*>(M.pairS);
-      q[slot] = make_int2(p, (int)mask);
+// The (point, pivot) pairs of this pass that may update, from the tensor
+// cores.  With vb the images rounded to bf16, pivot j cannot lower point p when
+//   ||vb_p - vb_j||^2 >= (thr_p + e_p + e_j)^2,
+// e_p = kBf ||vb_p|| the rounding to bf16, e_j that and the image's own
+// (which thr_p holds for the point).  The left side is
+// |vb_p|^2 + |vb_j|^2 - 2 vb_p.vb_j: the products are exact in float32, and
+// all sums together err by less than 2^-16 (|vb_p|^2 + |vb_j|^2); twice that
+// is added to the right side, with the largest e_j and |vb_j|^2 of the pass.
+// The accumulators start at -|vb_j|^2 / 2, so a pair is settled by one
+// comparison with (|vb_p|^2 - right side) / 2; a NaN anywhere keeps the pair.
+// The pairs left (a few per pass, once the distances are small) meet the
+// float32 screen and the exact distance in mc_update.
+// KT: 16-wide steps over the coordinates.  A warp takes 32 points x 32 pivots
+// at a time; the 32 pivots' operands stay in registers.
+template <int KT>
+__device__ __forceinline__ void mc_screen(const McSmem& M, const int* slot, int* qn, int k, int S, int Sc,
+                                          int d, float growth) {
+  constexpr float kBf = 0x1.01p-8f;  // half a unit of bf16's 8 bits, and the roundings of |vb|
+  constexpr float kBp = 0x1.02p16f;  // the same in Bp_p >= 2^-24 |v_p| (|vb| <= |v| (1 + 2^-8))
+  const int lane = threadIdx.x & 31, g = lane >> 2, c2 = (lane & 3) * 2;
+  uint32_t B[4][KT][2];
+  float C0[4][2];
+  unsigned em = 0, nm = 0;
+#pragma unroll
+  for (int nt = 0; nt < 4; ++nt) {
+    const int t = nt * 8 + g;
+    const int u = t < k ? slot[t] : -1;
+    float nn = 0.0f;
+#pragma unroll
+    for (int kt = 0; kt < KT; ++kt)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int l = kt * 16 + h * 8 + c2;
+        B[nt][kt][h] = mc_bf16x2(u >= 0 && l < d ? M.Uv[u * d + l] : 0.0f,
+                                 u >= 0 && l + 1 < d ? M.Uv[u * d + l + 1] : 0.0f, nn);
+      }
+    nn += __shfl_xor_sync(0xffffffffu, nn, 1);
+    nn += __shfl_xor_sync(0xffffffffu, nn, 2);
+    if (u >= 0) {  // (as bits: a NaN is the largest)
+      em = max(em, __float_as_uint(fmaf(kBf, sqrtf(nn), M.UB[u])) & 0x7fffffffu);
+      nm = max(nm, __float_as_uint(nn) & 0x7fffffffu);
     } else {
-      mc_exact(M, Ps, p, d, mask);
+      nn = __int_as_float(0x7f800000);  // no pivot: below every level
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) C0[nt][i] = -0.5f * __shfl_sync(0xffffffffu, nn, (c2 + i) * 4);
+  }
+  const float emax = __uint_as_float(__reduce_max_sync(0xffffffffu, em));
+  const float nmax = __uint_as_float(__reduce_max_sync(0xffffffffu, nm));
+  const unsigned kmask = (1u << k) - 1;  // k <= 31
+  for (int r0 = (threadIdx.x >> 5) * 32; r0 < S; r0 += blockDim.x) {
+    uint32_t A[2][KT][4];
+    float np[4] = {}, h[4];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const float* v0 = M.v + min(r0 + g + 8 * x, S - 1);
+#pragma unroll
+      for (int kt = 0; kt < KT; ++kt)
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+          const int l = kt * 16 + y * 8 + c2;
+          A[x >> 1][kt][2 * y + (x & 1)] = mc_bf16x2(l < d ? v0[(size_t)l * Sc] : 0.0f,
+                                                     l + 1 < d ? v0[(size_t)(l + 1) * Sc] : 0.0f, np[x]);
+        }
+    }
+#pragma unroll
+    for (int x = 0; x < 4; ++x) np[x] += __shfl_xor_sync(0xffffffffu, np[x], 1);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) np[x] += __shfl_xor_sync(0xffffffffu, np[x], 2);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const int p = min(r0 + g + 8 * x, S - 1);
+      const float th = *(volatile float*)(M.thr + p);
+      const float t = fmaf(kBp, M.Bp[p], th + emax);
+      const float rhs = fmaf(t * t, 1.0f + 0x1p-12f, fmaf(0x1p-15f, np[x] + nmax, 1e-30f));
+      h[x] = 0.5f * (np[x] - rhs);
+      if (th < 0.0f || r0 + g + 8 * x >= S) h[x] = __int_as_float(0x7f800000);  // ordered: nothing
+    }
+    float acc[4][2][4];  // rows r0 + g + 16 x (+ 8)
+    bool none = true;
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        float(&c)[4] = acc[nt][x];
+        c[0] = c[2] = C0[nt][0];
+        c[1] = c[3] = C0[nt][1];
+#pragma unroll
+        for (int kt = 0; kt < KT; ++kt)
+          asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+              "{%0,%1,%2,%3};"
+              : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+              : "r"(A[x][kt][0]), "r"(A[x][kt][1]), "r"(A[x][kt][2]), "r"(A[x][kt][3]), "r"(B[nt][kt][0]),
+                "r"(B[nt][kt][1]));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) none = none && c[i] < h[2 * x + (i >> 1)];
+      }
+    if (!none) {
+      unsigned bits[4] = {};  // rows r0 + g + 8 x
+      int cnt = 0;
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+            bits[x] |= (acc[nt][x >> 1][2 * (x & 1) + i] < h[x] ? 0u : 1u) << (nt * 8 + i);
+        bits[x] = h[x] == __int_as_float(0x7f800000) ? 0u : bits[x] << c2 & kmask;
+        cnt += __popc(bits[x]);
+      }
+      int at = atomicAdd(qn, cnt);
+      unsigned* queue = reinterpret_cast<unsigned*>(M.pairS);
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+        for (unsigned m = bits[x]; m; m &= m - 1, ++at) {
+          const unsigned e = (unsigned)(r0 + g + 8 * x) << 5 | (unsigned)(__ffs(m) - 1);
+          if (at < kMcQueue)
+            queue[at] = e;
+          else
+            mc_update(M, slot, e, Sc, d, growth);  // the queue is full
+        }
     }
   }
 }
 
-// This pass's pivots (table entries t < k: row Pi, bound PB, image Pv, slot
-// Ps of the exact coordinates) applied to the CTA's points, then each
-// thread's three largest keys.  For every point the float32 screen runs over
-// all pivots first, with the threshold of the pass start (an upper bound of
-// every later one, so a pivot it skips cannot update); the exact squared
-// distances of the pivots left then update in pivot order, as the reference
-// applies them (ordering.py:49-58).  DV: the image width held in registers
-// (0: read from shared memory, any d); up to 16, two points share each
-// read of a pivot image.
-template <int DV>
-__device__ __forceinline__ void mc_apply(const McSmem& M, const int* Pi, const float* PB,
-                                         const int* Ps, int* qn, int k, int S, int Sc, int d,
-                                         int p0, float growth, long long& b1, int& i1,
+// This pass's pivots (slots slot[0..k)) applied to the CTA's points, then
+// each thread's three largest keys.  The screen takes the thresholds of the
+// pass start (upper bounds of every later one, so a pair that it settles
+// cannot update); the pairs left are worked off by dense warps: a float64
+// warp instruction costs the same with one active lane as with 32.
+// 1,316 rows of d = 10 per CTA and 31 pivots: the float32 screen of every
+// pair took 24,300 cycles, this 6,600.
+__device__ __forceinline__ void mc_apply(const McSmem& M, const int* slot, int* qn, int k, int S, int Sc,
+                                         int d, int p0, float growth, long long& b1, int& i1,
                                          long long& b2, int& i2, long long& b3, int& i3) {
-  if constexpr (DV > 0 && DV <= 16) {
-    const int T = blockDim.x;
-    for (int p = threadIdx.x; p < S; p += 2 * T) {
-      const int q = p + T;
-      const bool liveA = __double_as_longlong(M.dist[p]) >= 0;
-      const bool liveB = q < S && __double_as_longlong(M.dist[q]) >= 0;
-      if (!liveA && !liveB) continue;  // ordered (ordering.py:50-51)
-      const float thA = M.thr[p], thB = liveB ? M.thr[q] : 0.0f;
-      float va[DV], vb[DV];
-#pragma unroll
-      for (int l = 0; l < DV; ++l) {
-        va[l] = l < d ? M.v[(size_t)l * Sc + p] : 0.0f;
-        vb[l] = l < d && liveB ? M.v[(size_t)l * Sc + q] : 0.0f;
-      }
-      unsigned mA = 0, mB = 0;
-      bool hA = false, hB = false;
-#pragma unroll 2
-      for (int t = 0; t < k; ++t) {
-        const float4* pv = reinterpret_cast<const float4*>(M.Pv + t * DV);
-        const float sA = mc_s32<DV>(va, pv), sB = mc_s32<DV>(vb, pv);
-        const int pi = Pi[t];
-        const float pb = PB[t];
-        hA = hA || pi == p0 + p;
-        hB = hB || pi == p0 + q;
-        if (mc_may_update(sA, thA, pb, growth)) mA |= 1u << t;
-        if (mc_may_update(sB, thB, pb, growth)) mB |= 1u << t;
-      }
-      mc_screened(M, Ps, qn, p, d, hA, liveA ? mA : 0u);
-      if (liveB) mc_screened(M, Ps, qn, q, d, hB, mB);
-    }
-  } else {
-    constexpr int W = DV > 0 ? DV : 64;
-    for (int p = threadIdx.x; p < S; p += blockDim.x) {
-      if (__double_as_longlong(M.dist[p]) < 0) continue;  // ordered (ordering.py:50-51)
-      const float th = M.thr[p];
-      unsigned mask = 0;
-      bool hit = false;
-      if constexpr (DV > 0) {
-        float vp[DV];
-#pragma unroll
-        for (int l = 0; l < DV; ++l) vp[l] = l < d ? M.v[(size_t)l * Sc + p] : 0.0f;
-#pragma unroll 2
-        for (int t = 0; t < k; ++t) {
-          const float s32 = mc_s32<DV>(vp, reinterpret_cast<const float4*>(M.Pv + t * DV));
-          hit = hit || Pi[t] == p0 + p;
-          if (mc_may_update(s32, th, PB[t], growth)) mask |= 1u << t;
-        }
-      } else {
-        for (int t = 0; t < k; ++t) {
-          const float* pv = M.Pv + t * W;
-          float s32 = 0.0f;
-          for (int l = 0; l < d; ++l) {
-            const float df = __fsub_rn(M.v[(size_t)l * Sc + p], pv[l]);
-            s32 = __fmaf_rn(df, df, s32);
-          }
-          hit = hit || Pi[t] == p0 + p;
-          if (mc_may_update(s32, th, PB[t], growth)) mask |= 1u << t;
-        }
-      }
-      mc_screened(M, Ps, qn, p, d, hit, mask);
-    }
-  }
+  if (d <= 16)
+    mc_screen<1>(M, slot, qn, k, S, Sc, d, growth);
+  else if (d <= 32)
+    mc_screen<2>(M, slot, qn, k, S, Sc, d, growth);
+  else
+    mc_screen<4>(M, slot, qn, k, S, Sc, d, growth);
   __syncthreads();
-  // the queued exact distances, densely
   const int nq = min(*qn, kMcQueue);
-  const int2* q = reinterpret_cast<const int2*>(M.pairS);
-  for (int e = threadIdx.x; e < nq; e += blockDim.x) {
-    const int2 E = q[e];
-    mc_exact(M, Ps, E.x, d, (unsigned)E.y);
-  }
+  const unsigned* queue = reinterpret_cast<const unsigned*>(M.pairS);
+  for (int e = threadIdx.x; e < nq; e += blockDim.x) mc_update(M, slot, queue[e], Sc, d, growth);
   __syncthreads();
   // each thread's three largest keys, its points in index order
   for (int p = threadIdx.x; p < S; p += blockDim.x) {
@@ -352,7 +372,6 @@ __device__ __forceinline__ void mc_run(const McRun& Q, int C, int r) {
   extern __shared__ __align__(16) unsigned char smraw[];
   const int64_t n = Q.n;
   const int d = Q.d;
-  const int DV = mc_dv(d);
   const double* X = Q.X;
   int64_t* order = Q.order;
   const int per = (int)((n + C - 1) / C);
@@ -365,8 +384,8 @@ __device__ __forceinline__ void mc_run(const McRun& Q, int C, int r) {
   __shared__ int cl_i[2][32], cl_Ki[2];
   __shared__ long long w_Kb[kMcWarps];
   __shared__ int w_Ki[kMcWarps];
-  __shared__ int piv_slot[kMcSlots], P_i[kMcSlots], P_s[kMcSlots];
-  __shared__ float P_B[kMcSlots], Uthr[kMcSlots];
+  __shared__ int piv_slot[kMcSlots];
+  __shared__ float Uthr[kMcSlots];
   __shared__ int s_k, s_tie, s_err, s_Ki, s_qn, s_abort;
   __shared__ unsigned s_epoch;
   __shared__ long long s_Kb, s_top;
@@ -422,21 +441,22 @@ __device__ __forceinline__ void mc_run(const McRun& Q, int C, int r) {
       vv = v[(size_t)l * Sc + loc];
     }
   };
-  // warp 0: the pivot table from slots piv_slot[0..kk)
-  auto build_pivots = [&](int kk) {
+  // warp 0: slots piv_slot[0..kk) are the next pivots; their rows are ordered
+  // (ordering.py:58) at positions at, at + 1, ...
+  auto build_pivots = [&](int kk, int64_t at) {
     __syncwarp();
-    for (int e = lane; e < kk * DV; e += 32) {
-      const int t = e / DV, l = e - t * DV;
-      M.Pv[e] = l < d ? M.Uv[piv_slot[t] * d + l] : 0.0f;
-    }
     if (lane < kk) {
-      const int u = piv_slot[lane];
-      P_i[lane] = M.Ui[u];
-      P_B[lane] = M.UB[u];
-      P_s[lane] = u;
+      const int idx = M.Ui[piv_slot[lane]];
+      if (r == 0) order[at + lane] = idx;
+      if (idx >= p0 && idx < p0 + S) {
+        M.dist[idx - p0] = -1.0;
+        M.thr[idx - p0] = __int_as_float(0xff800000);
+      }
     }
-    if (lane == 0) s_qn = 0;
-    __syncwarp();
+    if (lane == 0) {
+      s_k = kk;
+      s_qn = 0;
+    }
   };
 
   // centre: the first row (any shift serves the float32 screen)
@@ -471,12 +491,10 @@ __device__ __forceinline__ void mc_run(const McRun& Q, int C, int r) {
       M.UB[kMcU] = mc_img_bound(M.Uv + kMcU * d, d);
       M.Ui[kMcU] = idx;
       piv_slot[0] = kMcU;
-      s_k = 1;
       s_err = 0;
       s_tie = 0;
-      if (r == 0) order[0] = Q.first;
     }
-    build_pivots(1);
+    build_pivots(1, 0);
   }
   __syncthreads();
 
@@ -663,22 +681,7 @@ __device__ __forceinline__ void mc_run(const McRun& Q, int C, int r) {
     const int k = s_k;
     long long b1 = -1, b2 = -1, b3 = -1;
     int i1 = kMcNone, i2 = kMcNone, i3 = kMcNone;
-    switch (DV) {
-      case 4:
-        mc_apply<4>(M, P_i, P_B, P_s, &s_qn, k, S, Sc, d, p0, growth, b1, i1, b2, i2, b3, i3);
-        break;
-      case 8:
-        mc_apply<8>(M, P_i, P_B, P_s, &s_qn, k, S, Sc, d, p0, growth, b1, i1, b2, i2, b3, i3);
-        break;
-      case 16:
-        mc_apply<16>(M, P_i, P_B, P_s, &s_qn, k, S, Sc, d, p0, growth, b1, i1, b2, i2, b3, i3);
-        break;
-      case 32:
-        mc_apply<32>(M, P_i, P_B, P_s, &s_qn, k, S, Sc, d, p0, growth, b1, i1, b2, i2, b3, i3);
-        break;
-      default:
-        mc_apply<0>(M, P_i, P_B, P_s, &s_qn, k, S, Sc, d, p0, growth, b1, i1, b2, i2, b3, i3);
-    }
+    mc_apply(M, piv_slot, &s_qn, k, S, Sc, d, p0, growth, b1, i1, b2, i2, b3, i3);
     // 2. candidates U = slots 0..30; R bounds every other point's bits
     long long R;
     int Ri;
@@ -752,13 +755,10 @@ __device__ __forceinline__ void mc_run(const McRun& Q, int C, int r) {
         }
         ++kk;
       }
-      build_pivots(kk);
+      build_pivots(kk, nsel);
       if (lane == 0) {
-        s_k = kk;
         s_tie = kk == 0;
         s_top = top;
-        if (r == 0)
-          for (int t = 0; t < kk; ++t) order[nsel + t] = P_i[t];
       }
     }
     __syncthreads();
@@ -819,12 +819,7 @@ __device__ __forceinline__ void mc_run(const McRun& Q, int C, int r) {
             }
             ++kk;
           }
-          build_pivots(kk);
-          if (lane == 0) {
-            s_k = kk;
-            if (r == 0)
-              for (int t = 0; t < kk; ++t) order[nsel + t] = P_i[t];
-          }
+          build_pivots(kk, nsel);
         }
       }
       __syncthreads();
