@@ -51,12 +51,19 @@ namespace sv {
 constexpr int kMcThreads = 512;
 constexpr int kMcWarps = kMcThreads / 32;
 constexpr int kMcSlots = 32;  // candidate slots; slot 31 holds a pivot found by a full scan
-// static shared memory of k_maximin_cluster (about 1.8 KB), rounded up: the
+// static shared memory of k_maximin_cluster (about 3.4 KB), rounded up: the
 // capacity of a cluster is computed from what is left of 227 KB
 constexpr int kMcStaticSmem = 4096;
 constexpr int kMcMaxCluster = 16;
 // work area: the warps' candidate lists (bits + index) or the pair distances
 constexpr int kMcWorkBytes = ((kMcU * kMcU * 8 > kMcWarps * 32 * 12 ? kMcU * kMcU * 8 : kMcWarps * 32 * 12) + 15) & ~15;
+
+// candidates of a pass from a level: the room of a CTA's list and of all
+// lists, and the number of keys that the next level is set for
+constexpr int kMcList = 96;
+constexpr int kMcGather = 256;
+constexpr int kMcTarget = 48;
+static_assert(kMcGather <= kMcThreads && kMcGather * 12 <= kMcWorkBytes, "the gathered keys");
 
 struct RoProb {
   int64_t n, xe_off, ye_off, ze_off, x_off, y_off, z_off, blk_off, first;
@@ -294,16 +301,14 @@ __device__ __forceinline__ void mc_screen(const McSmem& M, const int* slot, int*
   }
 }
 
-// This pass's pivots (slots slot[0..k)) applied to the CTA's points, then
-// each thread's three largest keys.  The screen takes the thresholds of the
+// This pass's pivots (slots slot[0..k)) applied to the CTA's points.  The screen takes the thresholds of the
 // pass start (upper bounds of every later one, so a pair that it settles
 // cannot update); the pairs left are worked off by dense warps: a float64
 // warp instruction costs the same with one active lane as with 32.
 // 1,316 rows of d = 10 per CTA and 31 pivots: the float32 screen of every
 // pair took 24,300 cycles, this 6,600.
 __device__ __forceinline__ void mc_apply(const McSmem& M, const int* slot, int* qn, int k, int S, int Sc,
-                                         int d, int p0, float growth, long long& b1, int& i1,
-                                         long long& b2, int& i2, long long& b3, int& i3) {
+                                         int d, float growth) {
   if (d <= 16)
     mc_screen<1>(M, slot, qn, k, S, Sc, d, growth);
   else if (d <= 32)
@@ -315,12 +320,6 @@ __device__ __forceinline__ void mc_apply(const McSmem& M, const int* slot, int* 
   const unsigned* queue = reinterpret_cast<const unsigned*>(M.pairS);
   for (int e = threadIdx.x; e < nq; e += blockDim.x) mc_update(M, slot, queue[e], Sc, d, growth);
   __syncthreads();
-  // each thread's three largest keys, its points in index order
-  for (int p = threadIdx.x; p < S; p += blockDim.x) {
-    const long long b = __double_as_longlong(M.dist[p]);
-    if (b < 0 || b >= 0x7ff0000000000000LL) continue;  // ordered, or not finite
-    mc_insert3(b, p0 + p, b1, i1, b2, i2, b3, i3);
-  }
 }
 
 // One problem of the pass maximin.
@@ -342,6 +341,10 @@ struct McRun {
   long long* gl_Kb;
   int* gl_Ki;
   unsigned* arrive;
+  // grid form: the keys above the level [3][kMcGather] and their counts [3]
+  long long* gl_gb;
+  int* gl_gi;
+  unsigned* gl_gn;
 };
 
 // Maximin in passes.  A pass applies a batch of pivots, in order, to every
@@ -380,15 +383,15 @@ __device__ __forceinline__ void mc_run(const McRun& Q, int C, int r) {
   const int Sc = per;
   const McSmem M = mc_layout(smraw, d, Sc, kGrid ? X + (size_t)p0 * d : nullptr);
   __shared__ double cen[64];
-  __shared__ long long cl_b[2][32], cl_Kb[2];
-  __shared__ int cl_i[2][32], cl_Ki[2];
+  __shared__ long long cl_b[2][kMcList], cl_Kb[2];
+  __shared__ int cl_i[2][kMcList], cl_Ki[2], cl_n[2];
   __shared__ long long w_Kb[kMcWarps];
   __shared__ int w_Ki[kMcWarps];
   __shared__ int piv_slot[kMcSlots];
   __shared__ float Uthr[kMcSlots];
-  __shared__ int s_k, s_tie, s_err, s_Ki, s_qn, s_abort;
+  __shared__ int s_k, s_tie, s_err, s_Ki, s_qn, s_abort, s_cnt, s_all, s_hold;
   __shared__ unsigned s_epoch;
-  __shared__ long long s_Kb, s_top;
+  __shared__ long long s_Kb, s_top, s_level;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nwarp = blockDim.x >> 5;
   const float growth = mc_growth(d);
@@ -455,7 +458,7 @@ __device__ __forceinline__ void mc_run(const McRun& Q, int C, int r) {
     }
     if (lane == 0) {
       s_k = kk;
-      s_qn = 0;
+      s_qn = s_cnt = s_all = 0;
     }
   };
 
@@ -493,6 +496,8 @@ __device__ __forceinline__ void mc_run(const McRun& Q, int C, int r) {
       piv_slot[0] = kMcU;
       s_err = 0;
       s_tie = 0;
+      s_level = -1;
+      s_hold = 0;
     }
     build_pivots(1, 0);
   }
@@ -637,6 +642,119 @@ __device__ __forceinline__ void mc_run(const McRun& Q, int C, int r) {
     par ^= 1;
     return true;
   };
+  // The same from a level, in the common case: the keys at or above it, some
+  // 48 of all CTAs, are listed and every CTA ranks them by counting.  Slots
+  // 0..30 and (Kb, Ki) are as from collect (with fewer than 32 keys, the level
+  // bounds the others).  The level only decides how many candidates a pass
+  // sees, not which order results; it is set from the keys' density in the
+  // pass before.  found: the number of keys; none, or more than the lists
+  // hold, and collect has to do it.  False once a grid wait gave up.
+  // Sorting every thread's keys and merging all CTAs' lists took 20,000
+  // cycles of a pass over 152 CTAs (11,400 over 4), this 3,700 (4,900).
+  int tri = 0;  // grid form: the buffer of three; the one after next is cleared
+  auto gather = [&](long long level, int& found, long long& Kb, int& Ki) -> bool {
+    long long* gb = M.wlb;
+    int* gi = (int*)(gb + kMcGather);
+    for (int p = threadIdx.x; p < S; p += blockDim.x) {
+      const long long b = __double_as_longlong(M.dist[p]);
+      if (b < level || b >= 0x7ff0000000000000LL) continue;
+      const int at = atomicAdd(&s_cnt, 1);
+      if (at < kMcList) {
+        cl_b[par][at] = b;
+        cl_i[par][at] = p0 + p;
+      }
+    }
+    __syncthreads();
+    const int cnt = s_cnt, add = cnt > kMcList ? kMcGather + 1 : cnt;
+    if constexpr (kGrid) {
+      long long* kb = Q.gl_gb + tri * kMcGather;
+      int* ki = Q.gl_gi + tri * kMcGather;
+      if (warp == 0 && cnt > 0) {
+        int base = lane == 0 ? (int)atomicAdd(Q.gl_gn + tri, (unsigned)add) : 0;
+        base = __shfl_sync(0xffffffffu, base, 0);
+        for (int e = lane; e < min(cnt, kMcList) && base + e < kMcGather; e += 32) {
+          kb[base + e] = cl_b[par][e];
+          ki[base + e] = cl_i[par][e];
+        }
+      }
+      if (!all_sync()) return false;
+      found = (int)__ldcg(Q.gl_gn + tri);
+      if (threadIdx.x < kMcGather) {
+        gb[threadIdx.x] = __ldcg(kb + threadIdx.x);
+        gi[threadIdx.x] = __ldcg(ki + threadIdx.x);
+      }
+      // all read this buffer before the next barrier, and write the cleared
+      // one after it
+      if (r == 0 && threadIdx.x == 0) Q.gl_gn[tri == 0 ? 2 : tri - 1] = 0;
+      tri = tri == 2 ? 0 : tri + 1;
+      __syncthreads();
+    } else {
+      if (C > 1) {
+        cg::cluster_group cluster = cg::this_cluster();
+        if (threadIdx.x == 0) cl_n[par] = cnt;
+        cluster.sync();
+        if (warp < C) {
+          const long long* kb = cluster.map_shared_rank(&cl_b[par][0], warp);
+          const int* ki = cluster.map_shared_rank(&cl_i[par][0], warp);
+          const int nc = *cluster.map_shared_rank(&cl_n[par], warp);
+          long long b = kb[lane];  // (one remote round trip for all three)
+          int i = ki[lane];
+          int base = lane == 0 ? atomicAdd(&s_all, nc > kMcList ? kMcGather + 1 : nc) : 0;
+          base = __shfl_sync(0xffffffffu, base, 0);
+          for (int e = lane; e < min(nc, kMcList) && base + e < kMcGather; e += 32) {
+            if (e >= 32) {
+              b = kb[e];
+              i = ki[e];
+            }
+            gb[base + e] = b;
+            gi[base + e] = i;
+          }
+        }
+        __syncthreads();
+        found = s_all;
+      } else {
+        if (threadIdx.x < min(cnt, kMcList)) {
+          gb[threadIdx.x] = cl_b[par][threadIdx.x];
+          gi[threadIdx.x] = cl_i[par][threadIdx.x];
+        }
+        __syncthreads();
+        found = add;
+      }
+    }
+    par ^= 1;
+    if (found < 1 || found > kMcGather) return true;
+    // a key's slot is the number of keys above it: eight threads a key
+    for (int t0 = 0; t0 < found; t0 += kMcThreads / 8) {
+      const int t = t0 + (threadIdx.x >> 3);
+      const long long b = t < found ? gb[t] : -1LL;
+      const int i = t < found ? gi[t] : kMcNone;
+      int above = 0;
+      for (int j = threadIdx.x & 7; j < found; j += 8) above += mc_greater(gb[j], gi[j], b, i) ? 1 : 0;
+      above += __shfl_xor_sync(0xffffffffu, above, 1);
+      above += __shfl_xor_sync(0xffffffffu, above, 2);
+      above += __shfl_xor_sync(0xffffffffu, above, 4);
+      if (t < found && (threadIdx.x & 7) == 0 && above < 32) {
+        M.Ub[above] = b;
+        M.Ui[above] = i;
+        if (above == 31) {
+          s_Kb = b;
+          s_Ki = i;
+        }
+      }
+    }
+    if (threadIdx.x < 32 && threadIdx.x >= found) {
+      M.Ub[threadIdx.x] = -1LL;
+      M.Ui[threadIdx.x] = kMcNone;
+      if (threadIdx.x == 31) {
+        s_Kb = level - 1;
+        s_Ki = kMcNone;
+      }
+    }
+    __syncthreads();
+    Kb = s_Kb;
+    Ki = s_Ki;
+    return true;
+  };
   // the candidates' rows, then their pairwise exact squared distances
   // (float32-screened: +inf where neither can lower the other; -1 where a
   // float32 upper bound already puts either below R once the other is a pivot)
@@ -676,16 +794,27 @@ __device__ __forceinline__ void mc_run(const McRun& Q, int C, int r) {
 
   int64_t nsel = 1;
   while (nsel < n) {
-    // 1. apply the pivots to this CTA's points; keep each thread's three
-    //    largest keys
-    const int k = s_k;
-    long long b1 = -1, b2 = -1, b3 = -1;
-    int i1 = kMcNone, i2 = kMcNone, i3 = kMcNone;
-    mc_apply(M, piv_slot, &s_qn, k, S, Sc, d, p0, growth, b1, i1, b2, i2, b3, i3);
+    // 1. apply the pivots to this CTA's points
+    const long long level = s_level;
+    mc_apply(M, piv_slot, &s_qn, s_k, S, Sc, d, growth);
     // 2. candidates U = slots 0..30; R bounds every other point's bits
-    long long R;
-    int Ri;
-    if (!collect(b1, i1, b2, i2, b3, i3, R, Ri)) return;  // a grid wait gave up
+    long long R = -1LL, low = level;
+    int Ri = kMcNone, found = 0;
+    if (level >= 0 && !gather(level, found, R, Ri)) return;  // a grid wait gave up
+    const bool listed = found >= 1 && found <= kMcGather;
+    if (!listed) {
+      // from each thread's three largest keys, its points in index order
+      long long b1 = -1, b2 = -1, b3 = -1;
+      int i1 = kMcNone, i2 = kMcNone, i3 = kMcNone;
+      for (int p = threadIdx.x; p < S; p += blockDim.x) {
+        const long long b = __double_as_longlong(M.dist[p]);
+        if (b < 0 || b >= 0x7ff0000000000000LL) continue;  // ordered, or not finite
+        mc_insert3(b, p0 + p, b1, i1, b2, i2, b3, i3);
+      }
+      if (!collect(b1, i1, b2, i2, b3, i3, R, Ri)) return;
+      low = R;
+      found = 32;
+    }
     fetch_pairs(R >= 0 ? __longlong_as_double(R) : -1.0);
     // 3. pivots from the candidates (warp 0, one candidate per lane)
     if (warp == 0) {
@@ -759,6 +888,16 @@ __device__ __forceinline__ void mc_run(const McRun& Q, int C, int r) {
       if (lane == 0) {
         s_tie = kk == 0;
         s_top = top;
+        // The next level: as far below R as kMcTarget keys at this pass's
+        // density (in bits, so near enough in logarithms).  None after many
+        // equal keys, and for a few passes after a level that failed.
+        s_hold = level >= 0 && !listed ? 4 : max(0, s_hold - 1);
+        long long next = -1LL;
+        if (R < 0)
+          next = top < 0 ? -1LL : 0LL;
+        else if (top > low && s_hold == 0)
+          next = max(0LL, R - ((top - low) / found + 1) * kMcTarget);
+        s_level = next;
       }
     }
     __syncthreads();
@@ -781,8 +920,8 @@ __device__ __forceinline__ void mc_run(const McRun& Q, int C, int r) {
         }
       } else {
         const long long rmax = __double_as_longlong(__dsqrt_rn(__longlong_as_double(top)));
-        b1 = b2 = b3 = -1;
-        i1 = i2 = i3 = kMcNone;
+        long long b1 = -1, b2 = -1, b3 = -1;
+        int i1 = kMcNone, i2 = kMcNone, i3 = kMcNone;
         for (int p = threadIdx.x; p < S; p += blockDim.x) {
           const double dp = M.dist[p];
           const long long bits = __double_as_longlong(dp);
@@ -1126,7 +1265,8 @@ static int mg_plan(int64_t n, int d, int& G, int& per, size_t& smem) {
 
 size_t maximin_grid_workspace_bytes() {
   const size_t g2 = 2 * (size_t)sv_num_sms();
-  return ro_align(g2 * 32 * 8) + ro_align(g2 * 32 * 4) + ro_align(g2 * 8) + ro_align(g2 * 4) + 256;
+  return ro_align(g2 * 32 * 8) + ro_align(g2 * 32 * 4) + ro_align(g2 * 8) + ro_align(g2 * 4) +
+         ro_align(3 * kMcGather * 8) + ro_align(3 * kMcGather * 4) + 256;
 }
 
 int64_t maximin_grid_max_rows(int d) {
@@ -1166,8 +1306,13 @@ int maximin_grid_single(const double* X, int64_t n, int d, int64_t first, int64_
   off += ro_align(g2 * 8);
   Q.gl_Ki = (int*)(ws + off);
   off += ro_align(g2 * 4);
+  Q.gl_gb = (long long*)(ws + off);
+  off += ro_align(3 * kMcGather * 8);
+  Q.gl_gi = (int*)(ws + off);
+  off += ro_align(3 * kMcGather * 4);
   Q.arrive = (unsigned*)(ws + off);
-  SV_CUDA_TRY(cudaMemsetAsync(Q.arrive, 0, sizeof(unsigned), st));
+  Q.gl_gn = Q.arrive + 32;  // a line of its own
+  SV_CUDA_TRY(cudaMemsetAsync(Q.arrive, 0, 256, st));
   void* args[] = {&Q};
   SV_CUDA_TRY(cudaLaunchCooperativeKernel((void*)k_maximin_grid, dim3((unsigned)G), dim3(kMcThreads), args,
                                           smem, st));
