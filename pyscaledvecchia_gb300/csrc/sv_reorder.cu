@@ -32,9 +32,9 @@
 //    lists meet through distributed shared memory after one hardware cluster
 //    barrier per pass (double-buffered by pass parity), so there is no
 //    spin-wait at all.
-// Problems are grouped by cluster size (1, 2, 4, 8 or 16 CTAs, the smallest
-// whose shared memory holds the problem), one launch per group, largest
-// problems first.
+// Problems are grouped by cluster size (1, 2, 4, 8 or 16 CTAs: the smallest
+// whose shared memory holds the problem, or more when the SMs have room for
+// all problems side by side), one launch per group, largest problems first.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -78,10 +78,12 @@ struct RoProb {
 __host__ __device__ inline int64_t mc_point_bytes(int d, bool grid = false) {
   return 16 + (grid ? 4 : 12) * (int64_t)d;
 }
-// per-CTA shared memory before the points: candidate slots (exact and float32
-// coordinates, squared bits, index, bound) and the work area
+// coordinates of the bf16 images, zero padded to whole steps of the screen
+__host__ __device__ inline int mc_d16(int d) { return d <= 16 ? 16 : d <= 32 ? 32 : 64; }
+// per-CTA shared memory before the points: candidate slots (exact, float32 and
+// bf16 coordinates, squared bits, index, bound) and the work area
 __host__ __device__ inline int64_t mc_fixed_bytes(int d) {
-  return (int64_t)kMcSlots * (12 * d + 16) + kMcWorkBytes;
+  return (int64_t)kMcSlots * (12 * d + 16 + 2 * mc_d16(d)) + kMcWorkBytes;
 }
 
 __global__ void k_ro_info_init(int32_t* info, int nprob) {
@@ -113,6 +115,7 @@ struct McSmem {
   long long* Ub;   // [32] squared-distance bits at the start of the selection
   int* Ui;         // [32] row index
   float* UB;       // [32] float32 rounding bound of the image
+  uint32_t* Uh;    // [32][d16 / 2] the images rounded to bf16
   double* pairS;   // [31][31] exact squared distances between candidates (work area)
   long long* wlb;  // [warps][32] candidate lists (work area)
   int* wli;
@@ -132,7 +135,8 @@ __device__ __forceinline__ McSmem mc_layout(unsigned char* base, int d, int Sc, 
   L.Ub = (long long*)(base + (size_t)kMcSlots * 12 * d);
   L.Ui = (int*)(L.Ub + kMcSlots);
   L.UB = (float*)(L.Ui + kMcSlots);
-  unsigned char* work = base + (size_t)kMcSlots * (12 * d + 16);
+  L.Uh = (uint32_t*)(base + (size_t)kMcSlots * (12 * d + 16));
+  unsigned char* work = (unsigned char*)(L.Uh + kMcSlots * (mc_d16(d) / 2));
   L.pairS = (double*)work;
   L.wlb = (long long*)work;
   L.wli = (int*)(work + kMcWarps * 32 * 8);
@@ -190,38 +194,31 @@ __device__ __forceinline__ uint32_t mc_bf16x2(float a, float b, float& sq) {
 // float32 screen and the exact distance in mc_update.
 // KT: 16-wide steps over the coordinates.  A warp takes 32 points x 32 pivots
 // at a time; the 32 pivots' operands stay in registers.
+constexpr float kBf = 0x1.01p-8f;  // half a unit of bf16's 8 bits, and the roundings of |vb|
+constexpr float kBp = 0x1.02p16f;  // the same in Bp_p >= 2^-24 |v_p| (|vb| <= |v| (1 + 2^-8))
 template <int KT>
-__device__ __forceinline__ void mc_screen(const McSmem& M, const int* slot, int* qn, int k, int S, int Sc,
-                                          int d, float growth) {
-  constexpr float kBf = 0x1.01p-8f;  // half a unit of bf16's 8 bits, and the roundings of |vb|
-  constexpr float kBp = 0x1.02p16f;  // the same in Bp_p >= 2^-24 |v_p| (|vb| <= |v| (1 + 2^-8))
+__device__ __forceinline__ void mc_screen(const McSmem& M, const float* Un, const float* Ue, const int* slot,
+                                          int* qn, int k, int S, int Sc, int d, float growth) {
   const int lane = threadIdx.x & 31, g = lane >> 2, c2 = (lane & 3) * 2;
   uint32_t B[4][KT][2];
   float C0[4][2];
-  unsigned em = 0, nm = 0;
 #pragma unroll
   for (int nt = 0; nt < 4; ++nt) {
     const int t = nt * 8 + g;
-    const int u = t < k ? slot[t] : -1;
-    float nn = 0.0f;
+    const uint32_t* w = M.Uh + (t < k ? slot[t] : 0) * (KT * 8) + (lane & 3);
 #pragma unroll
-    for (int kt = 0; kt < KT; ++kt)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int l = kt * 16 + h * 8 + c2;
-        B[nt][kt][h] = mc_bf16x2(u >= 0 && l < d ? M.Uv[u * d + l] : 0.0f,
-                                 u >= 0 && l + 1 < d ? M.Uv[u * d + l + 1] : 0.0f, nn);
-      }
-    nn += __shfl_xor_sync(0xffffffffu, nn, 1);
-    nn += __shfl_xor_sync(0xffffffffu, nn, 2);
-    if (u >= 0) {  // (as bits: a NaN is the largest)
-      em = max(em, __float_as_uint(fmaf(kBf, sqrtf(nn), M.UB[u])) & 0x7fffffffu);
-      nm = max(nm, __float_as_uint(nn) & 0x7fffffffu);
-    } else {
-      nn = __int_as_float(0x7f800000);  // no pivot: below every level
+    for (int kt = 0; kt < KT; ++kt) {
+      B[nt][kt][0] = t < k ? w[kt * 8] : 0u;
+      B[nt][kt][1] = t < k ? w[kt * 8 + 4] : 0u;
     }
 #pragma unroll
-    for (int i = 0; i < 2; ++i) C0[nt][i] = -0.5f * __shfl_sync(0xffffffffu, nn, (c2 + i) * 4);
+    for (int i = 0; i < 2; ++i)  // no pivot: below every level
+      C0[nt][i] = nt * 8 + c2 + i < k ? -0.5f * Un[slot[nt * 8 + c2 + i]] : __int_as_float(0xff800000);
+  }
+  unsigned em = 0, nm = 0;  // as bits: a NaN is the largest
+  if (lane < k) {
+    em = __float_as_uint(Ue[slot[lane]]) & 0x7fffffffu;
+    nm = __float_as_uint(Un[slot[lane]]) & 0x7fffffffu;
   }
   const float emax = __uint_as_float(__reduce_max_sync(0xffffffffu, em));
   const float nmax = __uint_as_float(__reduce_max_sync(0xffffffffu, nm));
@@ -307,14 +304,14 @@ __device__ __forceinline__ void mc_screen(const McSmem& M, const int* slot, int*
 // warp instruction costs the same with one active lane as with 32.
 // 1,316 rows of d = 10 per CTA and 31 pivots: the float32 screen of every
 // pair took 24,300 cycles, this 6,600.
-__device__ __forceinline__ void mc_apply(const McSmem& M, const int* slot, int* qn, int k, int S, int Sc,
-                                         int d, float growth) {
+__device__ __forceinline__ void mc_apply(const McSmem& M, const float* Un, const float* Ue, const int* slot,
+                                         int* qn, int k, int S, int Sc, int d, float growth) {
   if (d <= 16)
-    mc_screen<1>(M, slot, qn, k, S, Sc, d, growth);
+    mc_screen<1>(M, Un, Ue, slot, qn, k, S, Sc, d, growth);
   else if (d <= 32)
-    mc_screen<2>(M, slot, qn, k, S, Sc, d, growth);
+    mc_screen<2>(M, Un, Ue, slot, qn, k, S, Sc, d, growth);
   else
-    mc_screen<4>(M, slot, qn, k, S, Sc, d, growth);
+    mc_screen<4>(M, Un, Ue, slot, qn, k, S, Sc, d, growth);
   __syncthreads();
   const int nq = min(*qn, kMcQueue);
   const unsigned* queue = reinterpret_cast<const unsigned*>(M.pairS);
@@ -388,7 +385,8 @@ __device__ __forceinline__ void mc_run(const McRun& Q, int C, int r) {
   __shared__ long long w_Kb[kMcWarps];
   __shared__ int w_Ki[kMcWarps];
   __shared__ int piv_slot[kMcSlots];
-  __shared__ float Uthr[kMcSlots];
+  __shared__ float Uthr[kMcSlots], Un[kMcSlots], Ue[kMcSlots];
+  __shared__ unsigned near_m[kMcSlots], s_red;
   __shared__ int s_k, s_tie, s_err, s_Ki, s_qn, s_abort, s_cnt, s_all, s_hold;
   __shared__ unsigned s_epoch;
   __shared__ long long s_Kb, s_top, s_level;
@@ -444,6 +442,44 @@ __device__ __forceinline__ void mc_run(const McRun& Q, int C, int r) {
       vv = v[(size_t)l * Sc + loc];
     }
   };
+  // W lanes (16 for d <= 16, so that one float64 instruction serves two
+  // slots, else a warp) bring the row of slot u (below 0: none): the exact
+  // row, its float32 image and rounding bound, its bf16 image, that one's
+  // squared norm and bound.  The whole warp calls it.
+  const int W = d <= 16 ? 16 : 32;
+  auto fetch_slot = [&](int u) {
+    const int l0 = lane & (W - 1), D16 = mc_d16(d);
+    float e2 = 0.0f, n2 = 0.0f;
+    for (int l = l0; l < D16; l += W) {
+      const bool on = u >= 0 && l < d;
+      double x;
+      float f;
+      row_elem(on ? M.Ui[u] : (int)Q.first, on ? l : 0, x, f);
+      if (!on) f = 0.0f;
+      float sq = 0.0f;
+      const uint32_t h = mc_bf16x2(f, __shfl_down_sync(0xffffffffu, f, 1), sq);
+      e2 = __fmaf_ru(f, f, e2);
+      if ((lane & 1) == 0) {
+        n2 += sq;
+        if (u >= 0) M.Uh[(u * D16 + l) >> 1] = h;
+      }
+      if (on) {
+        M.Ux[u * d + l] = x;
+        M.Uv[u * d + l] = f;
+      }
+    }
+    for (int o = W >> 1; o > 0; o >>= 1) {
+      e2 = __fadd_ru(e2, __shfl_xor_sync(0xffffffffu, e2, o));
+      n2 += __shfl_xor_sync(0xffffffffu, n2, o);
+    }
+    if (l0 == 0 && u >= 0) {
+      const float Bu = __fmul_ru(__fsqrt_ru(e2), 1.01f * 0x1p-24f);
+      M.UB[u] = Bu;
+      Un[u] = n2;
+      Ue[u] = fmaf(kBf, sqrtf(n2), Bu);
+      if (u < kMcU) Uthr[u] = thr_sq(__longlong_as_double(M.Ub[u]), Bu);
+    }
+  };
   // warp 0: slots piv_slot[0..kk) are the next pivots; their rows are ordered
   // (ordering.py:58) at positions at, at + 1, ...
   auto build_pivots = [&](int kk, int64_t at) {
@@ -487,12 +523,10 @@ __device__ __forceinline__ void mc_run(const McRun& Q, int C, int r) {
   if (!all_sync()) return;
   // the first pivot: row `first` (ordering.py:38-39) in slot 31
   if (warp == 0) {
-    const int idx = (int)Q.first;
-    for (int l = lane; l < d; l += 32) row_elem(idx, l, M.Ux[kMcU * d + l], M.Uv[kMcU * d + l]);
+    if (lane == 0) M.Ui[kMcU] = (int)Q.first;
     __syncwarp();
+    fetch_slot(lane < W ? kMcU : -1);
     if (lane == 0) {
-      M.UB[kMcU] = mc_img_bound(M.Uv + kMcU * d, d);
-      M.Ui[kMcU] = idx;
       piv_slot[0] = kMcU;
       s_err = 0;
       s_tie = 0;
@@ -755,39 +789,41 @@ __device__ __forceinline__ void mc_run(const McRun& Q, int C, int r) {
     Ki = s_Ki;
     return true;
   };
-  // the candidates' rows, then their pairwise exact squared distances
-  // (float32-screened: +inf where neither can lower the other; -1 where a
-  // float32 upper bound already puts either below R once the other is a pivot)
+  // the candidates' rows, then the exact squared distances of the pairs of
+  // them where either can lower the other: bit b of near_m[a] for such a
+  // pair, its distance in pairS; -1 where a float32 upper bound already puts
+  // either below R once the other is a pivot.  s_red: the slots that a slot
+  // before them lowers.
   auto fetch_pairs = [&](double Rv) {
-    for (int e = threadIdx.x; e < kMcU * d; e += blockDim.x) {
-      const int u = e / d, l = e - u * d;
-      if (M.Ub[u] >= 0) row_elem(M.Ui[u], l, M.Ux[u * d + l], M.Uv[u * d + l]);
+    for (int g = warp * (32 / W); g < kMcU; g += nwarp * (32 / W)) {
+      const int u = g + lane / W;
+      fetch_slot(u < kMcU && M.Ub[u] >= 0 ? u : -1);
     }
+    if (threadIdx.x < kMcSlots) near_m[threadIdx.x] = 0;
+    if (threadIdx.x == 0) s_red = 0;
     __syncthreads();
-    if (threadIdx.x < kMcU && M.Ub[threadIdx.x] >= 0) {
-      const int u = threadIdx.x;
-      const float B = mc_img_bound(M.Uv + u * d, d);
-      M.UB[u] = B;
-      Uthr[u] = thr_sq(__longlong_as_double(M.Ub[u]), B);
-    }
-    __syncthreads();
-    for (int t = threadIdx.x; t < kMcU * kMcU; t += blockDim.x) {
-      const int a = t / kMcU, b = t - a * kMcU;
-      if (a >= b || M.Ub[a] < 0 || M.Ub[b] < 0) continue;
+    // pair t: slots x and x + 1 + y (mod 31), each pair once
+    for (int t = threadIdx.x; t < kMcU * (kMcU / 2); t += blockDim.x) {
+      const int x = t / (kMcU / 2);
+      int y = x + 1 + (t - x * (kMcU / 2));
+      y -= y >= kMcU ? kMcU : 0;
+      const int a = min(x, y), b = max(x, y);
+      if (M.Ub[b] < 0) continue;  // (the slots are filled in order)
       float s32 = 0.0f;
       for (int l = 0; l < d; ++l) {
         const float df = __fsub_rn(M.Uv[a * d + l], M.Uv[b * d + l]);
         s32 = __fmaf_rn(df, df, s32);
       }
-      double sp = __longlong_as_double(0x7ff0000000000000LL);  // cannot update
-      if (mc_may_update(s32, Uthr[a], M.UB[b], growth) || mc_may_update(s32, Uthr[b], M.UB[a], growth)) {
-        if (Rv >= 0.0 && (double)mc_sq_upper(s32, M.UB[a], M.UB[b], growth) < Rv)
-          sp = -1.0;  // either, once the other is a pivot, falls below R: out of this pass
-        else
-          sp = sqdist_exact(M.Ux + a * d, M.Ux + b * d, d);  // (x_a - x_b)^2 = (x_b - x_a)^2
-      }
+      if (!mc_may_update(s32, Uthr[a], M.UB[b], growth) && !mc_may_update(s32, Uthr[b], M.UB[a], growth))
+        continue;  // neither can lower the other
+      double sp = -1.0;  // either, once the other is a pivot, falls below R: out of this pass
+      if (!(Rv >= 0.0 && (double)mc_sq_upper(s32, M.UB[a], M.UB[b], growth) < Rv))
+        sp = sqdist_exact(M.Ux + a * d, M.Ux + b * d, d);  // (x_a - x_b)^2 = (x_b - x_a)^2
       M.pairS[a * kMcU + b] = sp;
       M.pairS[b * kMcU + a] = sp;
+      atomicOr(&near_m[a], 1u << b);
+      atomicOr(&near_m[b], 1u << a);
+      if (__double_as_longlong(sp) < M.Ub[b]) atomicOr(&s_red, 1u << b);
     }
     __syncthreads();
   };
@@ -796,7 +832,7 @@ __device__ __forceinline__ void mc_run(const McRun& Q, int C, int r) {
   while (nsel < n) {
     // 1. apply the pivots to this CTA's points
     const long long level = s_level;
-    mc_apply(M, piv_slot, &s_qn, s_k, S, Sc, d, growth);
+    mc_apply(M, Un, Ue, piv_slot, &s_qn, s_k, S, Sc, d, growth);
     // 2. candidates U = slots 0..30; R bounds every other point's bits
     long long R = -1LL, low = level;
     int Ri = kMcNone, found = 0;
@@ -820,6 +856,7 @@ __device__ __forceinline__ void mc_run(const McRun& Q, int C, int r) {
     if (warp == 0) {
       long long sb = lane < kMcU ? M.Ub[lane] : -1LL;
       const int si = lane < kMcU ? M.Ui[lane] : kMcNone;
+      const unsigned nearby = lane < kMcU ? near_m[lane] : 0u;
       bool alive = sb >= 0;
       const long long top = __shfl_sync(0xffffffffu, sb, 0);  // the largest square
       int kk = 0;
@@ -827,9 +864,7 @@ __device__ __forceinline__ void mc_run(const McRun& Q, int C, int r) {
         // the leading run of slots that are certain in list order: each is
         // above R + 4 ulps, more than 4 ulps above the next slot (no equal
         // root below it) and not lowered by a slot before it
-        bool red = false;
-        for (int i = 0; i < lane && i < kMcU; ++i)
-          red = red || __double_as_longlong(M.pairS[lane * kMcU + i]) < sb;  // (knock-outs are < 0)
+        const bool red = (s_red >> lane & 1) != 0;  // (knock-outs are < 0)
         const long long nb = __shfl_down_sync(0xffffffffu, sb, 1);
         const bool near = lane + 1 < kMcU && nb >= 0 && nb >= sb - 4;
         const bool bad = lane >= kMcU || !alive || red || near || !(R < 0 || sb > R + 4);
@@ -839,8 +874,8 @@ __device__ __forceinline__ void mc_run(const McRun& Q, int C, int r) {
             piv_slot[lane] = lane;
             alive = false;
           }
-          for (int i = 0; alive && i < m; ++i) {
-            const long long sn = __double_as_longlong(M.pairS[lane * kMcU + i]);
+          for (unsigned w = nearby & ((1u << m) - 1); alive && w; w &= w - 1) {
+            const long long sn = __double_as_longlong(M.pairS[lane * kMcU + __ffs(w) - 1]);
             if (sn < 0)
               alive = false;  // below R: cannot be chosen in this pass
             else if (sn < sb)
@@ -875,7 +910,7 @@ __device__ __forceinline__ void mc_run(const McRun& Q, int C, int r) {
         const int ws = __ffs(__ballot_sync(0xffffffffu, alive && si == mi)) - 1;
         if (lane == 0) piv_slot[kk] = ws;
         if (lane == ws) alive = false;
-        if (alive) {
+        if (alive && (nearby >> ws & 1)) {
           const long long sn = __double_as_longlong(M.pairS[lane * kMcU + ws]);
           if (sn < 0)
             alive = false;  // below R after this pivot: cannot be chosen in this pass
@@ -941,6 +976,7 @@ __device__ __forceinline__ void mc_run(const McRun& Q, int C, int r) {
         if (warp == 0) {
           long long sb = lane < kMcU ? M.Ub[lane] : -1LL;
           const int si = lane < kMcU ? M.Ui[lane] : kMcNone;
+          const unsigned nearby = lane < kMcU ? near_m[lane] : 0u;
           bool alive = sb >= 0, tied = alive;
           int kk = 0;
           while (kk < kMcU && nsel + kk < n) {
@@ -949,7 +985,7 @@ __device__ __forceinline__ void mc_run(const McRun& Q, int C, int r) {
             const int ws = __ffs(__ballot_sync(0xffffffffu, alive && si == mi)) - 1;
             if (lane == 0) piv_slot[kk] = ws;
             if (lane == ws) alive = false;
-            if (alive) {
+            if (alive && (nearby >> ws & 1)) {
               const double sn = M.pairS[lane * kMcU + ws];
               if (__double_as_longlong(sn) < sb) {
                 sb = __double_as_longlong(sn);
@@ -1094,6 +1130,16 @@ static int mc_cluster_size(int64_t n, int d, int maxsm) {
   return 0;
 }
 
+// the same for a problem that has the SMs to itself: up to 16 CTAs while one
+// has more rows than threads.  A pass's screen and scans shrink with a CTA's
+// rows, its exchange hardly grows: 5,000 rows of d = 8 take 2.65 ms on 4
+// CTAs (all that their memory needs), 2.30 on 16; 60,000 of d = 1 55.9 and
+// 36.6; but 300 rows 0.39 on one and 0.44 on two.
+static int mc_spread(int64_t n, int C) {
+  while (C > 0 && C < mc_max_cluster() && n > (int64_t)C * kMcThreads) C *= 2;
+  return C;
+}
+
 struct RoPlan {
   std::vector<RoProb> probs;
   std::vector<KnnBatchProb> kprobs;
@@ -1113,6 +1159,7 @@ static int ro_plan(const sv_reorder_desc* D, const sv_reorder_prob* hp, RoPlan& 
   const int64_t np = D->nprob;
   L.probs.resize(np);
   L.kprobs.resize(np);
+  int64_t spread = 0;
   for (int64_t i = 0; i < np; ++i) {
     const sv_reorder_prob& U = hp[i];
     if (U.n < 0 || U.d < 1 || U.d > D->dmax || U.d > 64 || U.q < 0 || U.m < 0 || U.m > D->ldnbr ||
@@ -1135,6 +1182,7 @@ static int ro_plan(const sv_reorder_desc* D, const sv_reorder_prob* hp, RoPlan& 
     R.DP = knn_pad_dim(U.d);
     R.C = mc_cluster_size(U.n, U.d, maxsm);
     if (R.C == 0) return SV_EINVAL;
+    spread += mc_spread(U.n, R.C);
     R.xs_off = L.nxs;
     L.nxs += 2 * U.n * U.d;  // scaled rows, then the same rows in maximin order
     R.v_off = L.nv;
@@ -1150,6 +1198,8 @@ static int ro_plan(const sv_reorder_desc* D, const sv_reorder_prob* hp, RoPlan& 
     K.d = U.d;
     K.m = U.m;
   }
+  if (spread <= sv_num_sms())  // room for all of them at once
+    for (RoProb& R : L.probs) R.C = mc_spread(R.n, R.C);
   // largest problems first in every launch
   std::vector<int32_t> byn(np);
   for (int64_t i = 0; i < np; ++i) byn[i] = (int32_t)i;
@@ -1234,7 +1284,7 @@ static int launch_maximin_cluster(int C, size_t smem, unsigned nclusters, const 
 // one cluster).  ws: 256 bytes of device scratch.
 int maximin_cluster_single(const double* X, int64_t n, int d, int64_t first, int64_t* order,
                            int32_t* info, char* ws, int flags, cudaStream_t st) {
-  const int C = mc_cluster_size(n, d, ro_max_smem());
+  const int C = mc_spread(n, mc_cluster_size(n, d, ro_max_smem()));
   if (C == 0) return SV_EINVAL;
   struct {
     RoProb p;

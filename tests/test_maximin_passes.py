@@ -43,3 +43,19 @@ def test_order(oracle, kind, n, d, flags):
         return
     assert int(info[0]) == 0
     np.testing.assert_array_equal(order.cpu().numpy(), oracle.maximin_order(X, first=n // 3))
+
+
+def test_cluster_sizes_of_a_batch():
+    """A problem takes more CTAs when the whole batch has room on the SMs: the
+    same orders from a batch that has none (90 problems) and one by one."""
+    import math
+    from pyscaledvecchia_gb300.batched import BatchedLikelihood, BatchProblem, ordered_groups
+    rng = np.random.default_rng(8)
+    n, d, m, nprob = 600, 3, 5, 90
+    raw = [(rng.random((n, d)), rng.standard_normal(n)) for _ in range(nprob)]
+    thetas = [np.concatenate([[0.1], rng.uniform(-2.0, 2.0, d), [math.log(1e-3)]]) for _ in range(nprob)]
+    BL = BatchedLikelihood([BatchProblem(X, y, None, ordered_groups(n, m)) for X, y in raw])
+    BL.set_sources([r[0] for r in raw], [r[1] for r in raw], [None] * nprob, [m] * nprob)
+    together = BL.reorder(list(range(nprob)), thetas, return_orders=True)
+    for i in range(0, nprob, 30):
+        np.testing.assert_array_equal(BL.reorder([i], [thetas[i]], return_orders=True)[0], together[i])
