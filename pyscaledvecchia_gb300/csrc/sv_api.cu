@@ -112,7 +112,7 @@ __global__ void k_matern_eval32(const double* r, int64_t n, double nu, int which
 // (interval) of kMtabN threads
 __global__ void k_matern_table1(double nu, double* tab) {
   __shared__ double fm[kMtabN], fg[kMtabN];
-  mtab_build_interval(nu, blockIdx.x, fm, fg, tab);
+  mtab_build_interval(nu, blockIdx.x, fm, fg, tab + (size_t)blockIdx.x * 2 * kMtabN);
 }
 
 // its float32 part (the split prediction blocks): CTA (interval) of kFtabN

@@ -43,6 +43,7 @@ struct MaternMode {
   double lc_p, lc_m;   // log_coef at nu +- h
   double inv2h;        // 1 / (2h)
   const double* tab;   // general nu: the table of M and g (or null)
+  int tab_fixed;       // its rows (and those of nu +- h) are in fixed point
   int tab_elo;         // its first octave
   double s2n;          // sqrt(2 nu)
   // estimated nu with tables: those of nu + h and nu - h
@@ -59,17 +60,22 @@ __device__ __forceinline__ void matern_eval(const MaternMode& mm, double r, doub
     dMnu = 0.0;
     return;
   }
-  if (mm.tab) {
-    matern_table_Mg(mm.tab, mm.tab_elo, mm.s2n, mm.nu, mm.log_coef, r, M, g, want_g);
+  if (mm.tab && mm.tab_fixed) {
+    matern_table_fixed(mm.tab, mm.tab_elo, mm.s2n, mm.nu, mm.log_coef, r, M, g, want_g);
     dMnu = 0.0;
     if (mm.estimate_nu) {
       // _matern_general.py:170-176 (central difference in nu), M at nu +- h
       // from their tables
       double Mp, Mm, gx;
-      matern_table_Mg(mm.tab_p, mm.elo_p, mm.s2n_p, mm.nu_p, mm.lc_p, r, Mp, gx, false);
-      matern_table_Mg(mm.tab_m, mm.elo_m, mm.s2n_m, mm.nu_m, mm.lc_m, r, Mm, gx, false);
+      matern_table_fixed(mm.tab_p, mm.elo_p, mm.s2n_p, mm.nu_p, mm.lc_p, r, Mp, gx, false);
+      matern_table_fixed(mm.tab_m, mm.elo_m, mm.s2n_m, mm.nu_m, mm.lc_m, r, Mm, gx, false);
       dMnu = (Mp - Mm) * mm.inv2h;
     }
+    return;
+  }
+  if (mm.tab) {
+    matern_table_Mg(mm.tab, mm.tab_elo, mm.s2n, mm.nu, mm.log_coef, r, M, g, want_g);
+    dMnu = 0.0;  // (prediction: no derivative)
     return;
   }
   if (want_g) {

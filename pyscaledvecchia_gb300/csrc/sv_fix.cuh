@@ -17,6 +17,7 @@
 #include <stdint.h>
 #if !defined(__CUDACC__)
 #include <math.h>
+#include <string.h>
 #endif
 
 #ifndef SV_FX
@@ -207,6 +208,18 @@ SV_FX int64_t fx_rsqrt_pivot(int64_t d, int& e) {
   return ((int64_t)y0 << 28) + ((add + (1 << 16)) >> 17);
 }
 
+// e^-z (Q63) for z < 2^-8 ln 2 (Q70): the Taylor polynomial of degree 5
+SV_FX uint64_t fx_exp_tail(uint64_t z) {
+  const uint32_t zt = (uint32_t)(z >> 30);  // Q40
+  // z^2 from the top 32 bits and their cross product with the rest: Q80
+  const uint64_t z2 = (uint64_t)zt * zt + (((uint64_t)zt * (uint32_t)(((uint32_t)z & 0x3fffffffu) << 2)) >> 31);
+  const uint32_t z2t = (uint32_t)(z2 >> 32);   // Q48
+  const uint32_t z3 = fx_mulhi32(z2t, zt);     // Q56
+  // 1/6 - z/24 + z^2/120, Q34
+  const uint32_t c3 = 2863311531u - fx_mulhi32(zt, 2796203u) + fx_mulhi32(z2t, 2185u);
+  return (1ull << 63) - (z >> 7) + (z2 >> 18) - (((uint64_t)z3 * c3) >> 27);
+}
+
 // Matern 3/2 (code 1) and 5/2 (code 2) of a squared distance s (Q62) in units
 // of 2^(2 es): the correlation M, and the factor of its
 // derivative, g = e^-c (3/2: M'(r)/r = -3 g) or (1 + c) e^-c (5/2:
@@ -232,16 +245,7 @@ SV_FX void fx_matern(uint64_t s, int es, const uint64_t* T, uint64_t& M, uint64_
   const uint32_t th = (uint32_t)(t >> 32);
   const int n = E > 5 ? 128 : (int)(th >> 25);
   const uint64_t rem = t & ((1ull << 49) - 1);
-  const uint64_t z = fx_mulhi(rem << 14, kFxLn2);  // Q70
-  const uint32_t zt = (uint32_t)(z >> 30);         // Q40
-  // z^2 from the top 32 bits and their cross product with the rest: Q80
-  const uint64_t z2 = (uint64_t)zt * zt + (((uint64_t)zt * (uint32_t)(((uint32_t)z & 0x3fffffffu) << 2)) >> 31);
-  const uint32_t z2t = (uint32_t)(z2 >> 32);   // Q48
-  const uint32_t z3 = fx_mulhi32(z2t, zt);     // Q56
-  // 1/6 - z/24 + z^2/120, Q34
-  const uint32_t c3 = 2863311531u - fx_mulhi32(zt, 2796203u) + fx_mulhi32(z2t, 2185u);
-  const uint64_t em = (1ull << 63) - (z >> 7) + (z2 >> 18) - (((uint64_t)z3 * c3) >> 27);  // Q63
-  const uint64_t e = fx_mulhi(em, T[(th >> 17) & 255]);                                    // Q62
+  const uint64_t e = fx_mulhi(fx_exp_tail(fx_mulhi(rem << 14, kFxLn2)), T[(th >> 17) & 255]);  // Q62
   const uint64_t c = fx_mulhi(q << 1, CODE == 1 ? kFxA3 : kFxA5);  // c = this 2^E, Q60
   const uint64_t F = fx_mulhi(c << 1, e << 1);                     // c e^-c, Q60 before the shift
   const uint64_t e0 = fx_shr(e, n + 1);
@@ -264,6 +268,51 @@ SV_FX int64_t fx_scale2(int64_t x, int n) {
   return n < -62 ? 0 : (x + (1ll << (-n - 1))) >> -n;
 }
 SV_FX int fx_bits(int64_t x) { return 64 - fx_clz((uint64_t)(x < 0 ? -x : x)); }
+
+// v 2^ex as float64, rounded to nearest (ties up); no subnormal results
+SV_FX double fx_to_double(uint64_t v, int ex) {
+  if (v == 0) return 0.0;
+  const int lz = fx_clz(v);
+  v <<= lz;
+  const uint64_t b = ((uint64_t)(ex + 63 - lz + 1022) << 52) + (v >> 11) + ((v >> 10) & 1);
+#if defined(__CUDA_ARCH__)
+  return __longlong_as_double((long long)b);
+#else
+  double r;
+  memcpy(&r, &b, 8);
+  return r;
+#endif
+}
+
+// General Matern from tables in fixed point (a row: sv_matern.cuh's intervals
+// as polynomials, see mtab_fix_interval).  The polynomial's 16 coefficients
+// are Q58 of 2^ex (the top 16 bits of the last word; the sum of their
+// magnitudes is below 2), by Horner's rule in t (Q58): value (Q58) of 2^ex.
+constexpr uint64_t kFxTabS0 = 0x4d413cccfe779921ull;  // 2 (1 + sqrt 2), Q60
+constexpr uint64_t kFxTabS1 = 0x36a09e667f3bcc90ull;  // 2 + sqrt 2, Q60
+constexpr int64_t kFxTabO1 = 0x09a827999fcef324ll;    // 1 + sqrt 2, Q58
+constexpr uint64_t kFxLog2e = 0x5c551d94ae0bf85dull;  // log2 e, Q62
+// t in [-1, 1] (Q58) of the mantissa fraction f (52 bits) on the lower
+// ([1, sqrt2)) or upper ([sqrt2, 2)) half of an octave
+SV_FX int64_t fx_tab_t(uint64_t f, bool upper) {
+  const uint64_t p = fx_mulhi(f << 11, upper ? kFxTabS1 : kFxTabS0);  // Q59
+  return (int64_t)(p >> 1) - (upper ? kFxTabO1 : 1ll << 58);
+}
+// e^-c for c = (1 + f 2^-52) 2^e, e < 9: the result (Q62) times 2^-n.  t = c log2 e
+// in Q54 here, for c up to 2^9.
+SV_FX uint64_t fx_exp_neg(uint64_t f, int e, const uint64_t* T, int& n) {
+  const uint64_t m = (1ull << 62) + (f << 10);
+#if defined(__CUDA_ARCH__)
+  const uint64_t p = __umul64hi(m, kFxLog2e), pl = m * kFxLog2e;  // Q124 before 2^e
+#else
+  const unsigned __int128 q = (unsigned __int128)m * kFxLog2e;
+  const uint64_t p = (uint64_t)(q >> 64), pl = (uint64_t)q;
+#endif
+  const uint64_t t = e > 6 ? p << (e - 6) | pl >> (70 - e) : fx_shr(p + (e < 6 ? fx_shr(1ull << 5, e) : 0), 6 - e);
+  n = (int)(t >> 54);
+  const uint64_t rem = t & ((1ull << 46) - 1);
+  return fx_mulhi(fx_exp_tail(fx_mulhi(rem << 17, kFxLn2)), T[(t >> 46) & 255]);
+}
 
 // mantissa and sign of a float64 (bits) as an integer in units of the power
 // of two that puts the largest biased exponent exm of a group below 2^(53 + UP)

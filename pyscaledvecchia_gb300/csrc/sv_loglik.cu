@@ -111,6 +111,7 @@ __global__ void k_prob_params(const sv_prob_desc* descs, const double* theta, in
     // nu also M at nu +- h)
     mm.tab = (mtabs && uses_matern_table(D, nu)) ? mtabs + (size_t)p * kMtabSlotDoubles : nullptr;
     mm.tab_elo = mm.tab ? mtab_elo(nu) : 0;
+    mm.tab_fixed = 1;
     mm.s2n = sqrt(2.0 * nu);
     const bool est_tab = mm.tab && D.estimate_nu;
     mm.tab_p = est_tab ? mm.tab + kMtabOffP : nullptr;
@@ -161,7 +162,7 @@ __global__ void k_prob_params(const sv_prob_desc* descs, const double* theta, in
 // coefficients ([16 of M, 16 of G] per interval)
 __global__ void k_matern_tables(const sv_prob_desc* descs, const double* theta, int tstride,
                                 double* tabs) {
-  __shared__ double fm[kMtabN], fg[kMtabN];
+  __shared__ double fm[kMtabN], fg[kMtabN], cf[2 * kMtabN];
   const sv_prob_desc& D = descs[blockIdx.y];
   const double nu0 = problem_nu(D, theta + (int64_t)blockIdx.y * tstride);
   if (!uses_matern_table(D, nu0)) return;
@@ -170,7 +171,11 @@ __global__ void k_matern_tables(const sv_prob_desc* descs, const double* theta, 
   const double nu = z == 0 ? nu0 : z == 1 ? nu0 + kNuFdH : nu0 - kNuFdH;
   if ((int)blockIdx.x >= mtab_intervals(mtab_elo(nu))) return;
   double* tab = tabs + (size_t)blockIdx.y * kMtabSlotDoubles + (z == 0 ? 0 : z == 1 ? kMtabOffP : kMtabOffM);
-  mtab_build_interval(nu, blockIdx.x, fm, fg, tab);
+  mtab_build_interval(nu, blockIdx.x, fm, fg, cf);
+  __syncthreads();
+  int64_t* row = (int64_t*)tab + (size_t)blockIdx.x * 2 * kMtabN;
+  mtab_fix_interval(cf, 1.0, fm, row);
+  mtab_fix_interval(cf + kMtabN, -1.0, fg, row + kMtabN);
 }
 
 // the float32 tables of the split kernels (after the float64 tables in each

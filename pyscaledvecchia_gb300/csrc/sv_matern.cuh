@@ -19,6 +19,8 @@
 #pragma once
 #include <math.h>
 
+#include "sv_fix.cuh"
+
 #ifndef SV_HD
 #define SV_HD __host__ __device__ __forceinline__
 #endif
@@ -285,14 +287,14 @@ __device__ inline double mtab_coef(const double* f, int j) {
   return a * ((j == 0 ? 1.0 : 2.0) / kMtabN);
 }
 
-// interval iv of the float64 table of nu into tab (a CTA of kMtabN threads,
+// interval iv of the float64 table of nu into row (a CTA of kMtabN threads,
 // thread j; fm, fg shared arrays of kMtabN)
-__device__ inline void mtab_build_interval(double nu, int iv, double* fm, double* fg, double* tab) {
+__device__ inline void mtab_build_interval(double nu, int iv, double* fm, double* fg, double* row) {
   const int j = threadIdx.x;
   mtab_node(nu, mtab_elo(nu), iv, j, fm[j], fg[j]);
   __syncthreads();
-  tab[(size_t)iv * 2 * kMtabN + j] = mtab_coef(fm, j);
-  tab[(size_t)iv * 2 * kMtabN + kMtabN + j] = mtab_coef(fg, j);
+  row[j] = mtab_coef(fm, j);
+  row[kMtabN + j] = mtab_coef(fg, j);
 }
 
 __device__ __forceinline__ double mtab_clenshaw(const double* cf, double t) {
@@ -334,6 +336,104 @@ __device__ __forceinline__ void matern_table_Mg(const double* tab, int elo, doub
   const double ex = exp(-c);
   M = ex * mtab_clenshaw(cf, t);
   g = want_g ? ex * mtab_clenshaw(cf + kMtabN, t) : 0.0;
+}
+
+// The same interval as a polynomial in fixed point, for matern_table_fixed: cf
+// (shared, kMtabN) the Chebyshev coefficients of e^c M, or of e^c G (negated,
+// so that both are positive); thread j writes word j of row.  Their
+// magnitudes' sum s sets the exponent, s < 2 2^ex; the Chebyshev coefficients
+// are rounded to Q58 of 2^ex, and what they sum to in powers of t is exact
+// (the functions vary slowly on an interval: the powers' coefficients shrink
+// sixfold a term, the last is below 2^-26 of the scale).
+__device__ inline void mtab_fix_interval(const double* cf, double sign, double* sm, int64_t* row) {
+  const int j = threadIdx.x;
+  // coefficient of t^j in T_i, by the recurrence T_(i+1) = 2 t T_i - T_(i-1)
+  long long w[kMtabN], a[kMtabN] = {1}, b[kMtabN] = {0, 1};
+#pragma unroll
+  for (int i = 0; i < kMtabN; ++i) {
+    long long pick = 0;
+#pragma unroll
+    for (int k = 0; k < kMtabN; ++k) pick = k == j ? a[k] : pick;
+    w[i] = pick;
+#pragma unroll
+    for (int k = kMtabN - 1; k >= 0; --k) {
+      const long long nx = (k > 0 ? 2 * b[k - 1] : 0) - a[k];
+      a[k] = nx;
+    }
+#pragma unroll
+    for (int k = 0; k < kMtabN; ++k) {
+      const long long x = a[k];
+      a[k] = b[k];
+      b[k] = x;
+    }
+  }
+  double s = 0.0;
+  for (int i = 0; i < kMtabN; ++i) s = fma((double)w[i], cf[i], s);
+  sm[j] = fabs(s);
+  __syncthreads();
+  s = 0.0;
+  for (int i = 0; i < kMtabN; ++i) s += sm[i];
+  int ex;
+  frexp(s, &ex);
+  --ex;
+  long long v = 0;
+  for (int i = 0; i < kMtabN; ++i) v += w[i] * llrint(ldexp(sign * cf[i], 58 - ex));
+  if (j == kMtabN - 1) v = (long long)((unsigned long long)ex << 48) | (v & 0xffffffffffffll);
+  row[j] = v;
+  __syncthreads();
+}
+
+__device__ __forceinline__ uint64_t mtab_horner(const int64_t* row, Fx2 t, int& ex) {
+  const longlong2* r2 = reinterpret_cast<const longlong2*>(row);
+  longlong2 c = __ldg(r2 + kMtabN / 2 - 1);
+  ex = (int)(c.y >> 48);
+  int64_t v = (int64_t)((uint64_t)c.y << 16) >> 16;
+#pragma unroll
+  for (int k = kMtabN / 2 - 1; k >= 0; --k) {
+    if (k < kMtabN / 2 - 1) {
+      c = __ldg(r2 + k);
+      v = fx_mul(t, fx_split(v)) + c.y;
+    }
+    v = fx_mul(t, fx_split(v)) + c.x;
+  }
+  return v > 0 ? (uint64_t)v : 0;
+}
+
+// matern_table_Mg from the fixed-point form of the tables.  In float64 an
+// entry takes 32 (with g 64) dependent multiply-adds and an exponential on a
+// pipe of 64 cycles per warp instruction; here it is integer multiply-adds,
+// with absolute errors of a few 2^-58 of the interval's largest value, where
+// float64's are a few 2^-53.  The results keep float64's exponent range.
+__device__ __forceinline__ void matern_table_fixed(const double* tab, int elo, double s2n, double nu,
+                                                   double log_coef, double r, double& M, double& g,
+                                                   bool want_g) {
+  if (r < kRFloor) {
+    M = 1.0;
+    g = 0.0;
+    return;
+  }
+  const double c = s2n * r;
+  const long long b = __double_as_longlong(c);
+  const int e = (int)(b >> 52) - 1023;
+  if (e < elo || e >= kMtabEhi) {
+    double G;
+    matern_general_MG_c(c, nu, log_coef, M, G);
+    g = want_g ? G : 0.0;
+    return;
+  }
+  const uint64_t f = (uint64_t)b & 0x000FFFFFFFFFFFFFull;
+  const bool up = (long long)f >= (kMtabSqrt2Bits & 0x000FFFFFFFFFFFFFLL);
+  const Fx2 t = fx_split(fx_tab_t(f, up));
+  const int64_t* row = (const int64_t*)tab + (size_t)(2 * (e - elo) + (up ? 1 : 0)) * (2 * kMtabN);
+  int n, ex;
+  const uint64_t em = fx_exp_neg(f, e, kFxExp2, n);
+  const uint64_t P = mtab_horner(row, t, ex);
+  M = fx_to_double(fx_mulhi(em, P << 3), ex - n - 59);
+  g = 0.0;
+  if (want_g) {
+    const uint64_t G = mtab_horner(row + kMtabN, t, ex);
+    g = -fx_to_double(fx_mulhi(em, G << 3), ex - n - 59);
+  }
 }
 
 #endif

@@ -46,6 +46,7 @@ __device__ inline void pred_params(const PredArgs& A, PredPrm* prm) {
     mm.nu_p = mm.nu_m = mm.lc_p = mm.lc_m = 0.0;
     mm.inv2h = 0.0;
     mm.tab = A.closed < 0 ? A.tab : nullptr;
+    mm.tab_fixed = 0;
     mm.tab_elo = mm.tab ? mtab_elo(A.nu) : 0;
     mm.s2n = sqrt(2.0 * A.nu);
     mm.tab_p = mm.tab_m = nullptr;

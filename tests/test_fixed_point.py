@@ -151,3 +151,34 @@ def test_prediction_against_dense(m, d, nu, lo, precision):
         w = np.linalg.solve(S, k)
         assert abs(var[i] - (1.3 - w @ k)) <= tol * 1.3
         assert abs(mu[i] - w @ y[nb]) <= tol * max(1.0, np.abs(y).max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nu", [0.05, 1.0, 5.0, 9.99])
+@pytest.mark.parametrize("lam", [1e-3, 1.0, 1e6])
+def test_tables_against_bessel(nu, lam):
+    """The general smoothness' tables in fixed point against the Bessel routine
+    in every entry, from the smallest tabulated distances (ranges of 1e6) to
+    those beyond the table (ranges of 1e-3).  Both forms' entries are within
+    6e-15 of the variance; a block of 13 points and a nugget of 0.05 multiply
+    that by 13 / 0.05 = 260 at most."""
+    import pyscaledvecchia_gb300 as sv
+    from pyscaledvecchia_gb300.batched import BatchedLikelihood, BatchProblem
+    from pyscaledvecchia_gb300.likelihood import DeviceProblem
+    from pyscaledvecchia_gb300.ordering import _nn_groups
+    rng = np.random.default_rng(17)
+    X = rng.random((300, 2))
+    X[:40] = X[40:80] + 1e-6 * rng.standard_normal((40, 2))
+    y = rng.standard_normal(300)
+    theta = np.concatenate([[0.2], np.log([lam, 3 * lam]), [math.log(0.05)]])
+    groups = _nn_groups(sv.find_ordered_nn(X / lam, 12), 12)
+    BL = BatchedLikelihood([BatchProblem(X, y, None, groups, nu=nu)], matern_tables=False)
+    st, *ref = BL.evaluate([theta])[0]
+    if st:  # a rough field and distances on both sides of the floor: no covariance at all
+        with pytest.raises(np.linalg.LinAlgError):
+            DeviceProblem(X, y, None, groups).evaluate(theta, nu)
+        return
+    got = DeviceProblem(X, y, None, groups).evaluate(theta, nu)
+    assert abs(got[0] - ref[0]) <= 260 * 6e-15 * 300
+    for a, b in zip(got[1:3], ref[1:3]):
+        np.testing.assert_allclose(a, b, rtol=0, atol=2 * 260 * 6e-15 * max(300.0, np.abs(b).max()))
