@@ -648,6 +648,7 @@ __host__ __device__ inline int red_parts_n(int64_t nblk) {
 // partition per CTA leaves all but a few SMs idle below 100,000 blocks:
 // n = 5,000 took 90 us in k_reduce1 and 51 us in k_reduce2)
 constexpr int kRedCl = 8;
+constexpr int kRedWide = 4;  // warps of a CTA of k_reduce2 at most
 
 // the blocks [b0, b1) of CTA `rank` of partition `part`
 __device__ __forceinline__ void red_range(const ProbInfo& PI, int parts, int part, int rank, int64_t& b0,
@@ -815,7 +816,11 @@ __global__ void k_final1(RedArgs R) {
 }
 
 // Pass-2 sums of one partition: z_K^2 and the score terms, a thread per block.
-// PR: parameters whose sums are held in registers (a runtime count puts them
+// A lane's blocks are every 32nd of the CTA's run, in order, then the lanes
+// are added up: by one warp, or with a warp for each of up to kRedWide blocks
+// of a lane, whose terms then meet in the same order.  The width depends on
+// the launch, so the bits must not depend on the width, nor on PR (every
+// operation is written out).  PR: parameters whose sums are held in registers (a runtime count puts them
 // into local memory: 131 us instead of 111 at 200,000 blocks)
 template <int PR>
 __global__ void __cluster_dims__(kRedCl, 1, 1) k_reduce2(RedArgs R) {
@@ -823,7 +828,8 @@ __global__ void __cluster_dims__(kRedCl, 1, 1) k_reduce2(RedArgs R) {
   const int rank = (int)cl.block_rank();
   __shared__ double sbeta[kMaxQ];
   __shared__ double tot[kMaxP + 1];
-  __shared__ double red[kRedThreads / 32][PR + 1];
+  constexpr bool kWide = PR <= 16;  // (what the shared memory holds)
+  __shared__ double red[kWide ? kRedWide : 1][kWide ? PR + 1 : 1][32];
   const int p = blockIdx.y;
   const ProbInfo& PI = R.probs[p];
   if (PI.skip) return;
@@ -841,9 +847,9 @@ __global__ void __cluster_dims__(kRedCl, 1, 1) k_reduce2(RedArgs R) {
   for (int64_t b = b0 + threadIdx.x; b < b1; b += blockDim.x) {
     const double* c = R.cache + b * R.CS;
     double zK = c[2 + q];
-    for (int i = 0; i < q; ++i) zK -= c[3 + q + i] * sbeta[i];
-    const double zz = zK * zK;
-    acc[0] += zz;
+    for (int i = 0; i < q; ++i) zK = fma(-c[3 + q + i], sbeta[i], zK);
+    const double zz = __dmul_rn(zK, zK), z1 = __dadd_rn(1.0, zz), z2 = -2.0 * zK;
+    acc[0] = __dadd_rn(acc[0], zz);
     if (R.need_grad) {
       const double* wK = c + 3 + 2 * q;
       const double* wzy = wK + P;
@@ -852,25 +858,30 @@ __global__ void __cluster_dims__(kRedCl, 1, 1) k_reduce2(RedArgs R) {
       for (int pp = 0; pp < PR; ++pp)
         if (pp < P) {
           double wz = wzy[pp];
-          for (int i = 0; i < q; ++i) wz -= wzZ[pp * q + i] * sbeta[i];
-          acc[1 + pp] -= 0.5 * (wK[pp] * (1.0 + zz) - 2.0 * zK * wz);
+          for (int i = 0; i < q; ++i) wz = fma(-wzZ[pp * q + i], sbeta[i], wz);
+          acc[1 + pp] = fma(-0.5, fma(z2, wz, __dmul_rn(wK[pp], z1)), acc[1 + pp]);
         }
     }
   }
-  // fixed-order block reduction
-  const int w = threadIdx.x >> 5, ln = threadIdx.x & 31;
+  const int w = threadIdx.x >> 5, nw = blockDim.x >> 5, ln = threadIdx.x & 31;
+  auto lanes = [&](double v, int i) {
+    for (int o = 16; o > 0; o >>= 1) v = __dadd_rn(v, __shfl_down_sync(0xffffffffu, v, o));
+    if (ln == 0) tot[i] = v;
+  };
+  if (!kWide || nw == 1) {
 #pragma unroll
-  for (int i = 0; i <= PR; ++i)
-    if (i <= np) {
-      double v = acc[i];
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-      if (ln == 0) red[w][i] = v;
+    for (int i = 0; i <= PR; ++i)
+      if (i <= np) lanes(acc[i], i);
+  } else if constexpr (kWide) {
+#pragma unroll
+    for (int i = 0; i <= PR; ++i)
+      if (i <= np) red[w][i][ln] = acc[i];
+    __syncthreads();
+    for (int i = w; i <= np; i += nw) {
+      double v = red[0][i][ln];
+      for (int k = 1; k < nw; ++k) v = __dadd_rn(v, red[k][i][ln]);
+      lanes(v, i);
     }
-  __syncthreads();
-  for (int i = threadIdx.x; i <= np; i += blockDim.x) {
-    double s = 0.0;
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) s += red[k][i];
-    tot[i] = s;
   }
   cl.sync();
   if (rank == 0)
@@ -1287,13 +1298,14 @@ int run_eval(const EvalCall& C, cudaStream_t st, const ShardStage* sh = nullptr)
     k_final1<<<(unsigned)S.nprob, kRedThreads, 0, st>>>(R);
     SV_CUDA_TRY(cudaGetLastError());
     if (npart > 0) {
-      // a thread per block of a CTA's run while the CTAs do not fill the SMs;
+      // a thread per block of a CTA's run while the CTAs do not fill the SMs
+      // (runs of at most 128 blocks; beyond 8,192 blocks they have 114 to 128);
       // beyond that one warp, four blocks a thread: the sums over a warp are
       // most of the float64 work
-      const int64_t per = (S.nblk_max + parts - 1) / parts;
-      const int64_t run = (per + kRedCl - 1) / kRedCl;
-      int thr = (int64_t)npart * kRedCl * S.nprob > 2 * sv_num_sms() ? 32 : (int)((run + 31) / 32 * 32);
-      thr = std::max(32, std::min(thr, kRedThreads));
+      const int64_t run = S.nblk_max > 8192 ? 128 : (S.nblk_max + 8 * kRedCl - 1) / (8 * kRedCl);
+      const bool wide = (int64_t)npart * kRedCl * S.nprob <= 2 * sv_num_sms() &&
+                        S.nblk_max <= 4096 * 1024 && S.Pmax <= 16;
+      const int thr = wide ? std::max(32, (int)((run + 31) / 32 * 32)) : 32;
       if (S.Pmax <= 8)
         k_reduce2<8><<<rgrid, thr, 0, st>>>(R);
       else if (S.Pmax <= 16)

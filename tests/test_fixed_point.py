@@ -182,3 +182,25 @@ def test_tables_against_bessel(nu, lam):
     assert abs(got[0] - ref[0]) <= 260 * 6e-15 * 300
     for a, b in zip(got[1:3], ref[1:3]):
         np.testing.assert_allclose(a, b, rtol=0, atol=2 * 260 * 6e-15 * max(300.0, np.abs(b).max()))
+
+
+@pytest.mark.gpu
+def test_sums_do_not_depend_on_the_launch():
+    """Six problems of up to 5,000 blocks together (reductions of one warp per
+    CTA) and one by one (a warp per block of a lane): the same bits."""
+    import pyscaledvecchia_gb300 as sv
+    from pyscaledvecchia_gb300.batched import BatchedLikelihood, BatchProblem
+    from pyscaledvecchia_gb300.likelihood import DeviceProblem
+    from pyscaledvecchia_gb300.ordering import _nn_groups
+    rng = np.random.default_rng(3)
+    probs, thetas = [], []
+    for n, d, m in ((5000, 3, 10), (4097, 9, 5), (700, 2, 20), (3000, 12, 18), (2500, 1, 4), (4999, 6, 8)):
+        X, y, lam = rng.random((n, d)), rng.standard_normal(n), np.exp(rng.uniform(-1.0, 1.0, d))
+        probs.append((X, y, np.ones((n, 1)), _nn_groups(sv.find_ordered_nn(X / lam, m), m)))
+        thetas.append(np.concatenate([[0.1], np.log(lam), [math.log(1e-2)]]))
+    together = BatchedLikelihood([BatchProblem(*p, nu=2.5) for p in probs]).evaluate(thetas)
+    for p, th, r in zip(probs, thetas, together):
+        one = DeviceProblem(*p).evaluate(th, 2.5)
+        assert r[0] == 0 and r[1] == one[0]
+        for a, b in zip(r[2:], one[1:]):
+            np.testing.assert_array_equal(a, b)
