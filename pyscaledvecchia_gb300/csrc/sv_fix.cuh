@@ -168,6 +168,9 @@ SV_FX uint64_t fx_shr(uint64_t x, int k) {
 #endif
 }
 
+// 2^k, 0 beyond 63
+SV_FX uint64_t fx_shl1(int k) { return k > 63 ? 0 : 1ull << k; }
+
 // For m 2^-63 in [1/4, 1): the float32 reciprocal square root y0 (Q29),
 // g0 = m y0 (Q60), and t with 1/sqrt = y0 (1 + t), sqrt = g0 (1 + t): one
 // third-order step t = e/2 + 3 e^2 / 8 (Q61), e = 1 - m y0^2 (|e| < 2^-20; the
@@ -181,7 +184,7 @@ SV_FX int64_t fx_rsqrt_step(uint64_t m, uint32_t& y0, uint64_t& g0) {
 #endif
   y0 = (uint32_t)(yf * 536870912.0f);                                   // exact
   g0 = fx_mul32(m, y0);                                                 // Q60
-  const int64_t e = (int64_t)((1ull << 61) - (fx_mul32(g0, y0) << 4));  // Q57, in units of Q61
+  const int64_t e = (int64_t)((1ull << 61) - 8 - (fx_mul32(g0, y0) << 4));  // Q57, in units of Q61; 8: the mean of what the products drop
   const int32_t e10 = (int32_t)(e >> 10);                               // Q51
   const uint32_t ee = (uint32_t)((uint64_t)((int64_t)e10 * e10) >> 32); // Q70
   return (e >> 1) + ((3 * ee) >> 12);
@@ -214,10 +217,10 @@ SV_FX uint64_t fx_exp_tail(uint64_t z) {
   // z^2 from the top 32 bits and their cross product with the rest: Q80
   const uint64_t z2 = (uint64_t)zt * zt + (((uint64_t)zt * (uint32_t)(((uint32_t)z & 0x3fffffffu) << 2)) >> 31);
   const uint32_t z2t = (uint32_t)(z2 >> 32);   // Q48
-  const uint32_t z3 = fx_mulhi32(z2t, zt);     // Q56
+  const uint32_t z3 = 2 * fx_mulhi32(z2t, zt) + 1;  // Q57, with the mean of what is dropped
   // 1/6 - z/24 + z^2/120, Q34
   const uint32_t c3 = 2863311531u - fx_mulhi32(zt, 2796203u) + fx_mulhi32(z2t, 2185u);
-  return (1ull << 63) - (z >> 7) + (z2 >> 18) - (((uint64_t)z3 * c3) >> 27);
+  return (1ull << 63) - (z >> 7) + (z2 >> 18) - (((uint64_t)z3 * c3) >> 28);
 }
 
 // Matern 3/2 (code 1) and 5/2 (code 2) of a squared distance s (Q62) in units
@@ -227,7 +230,9 @@ SV_FX uint64_t fx_exp_tail(uint64_t z) {
 // a few 2^-59. exp(-c) = 2^-t, t = c log2 e: the integer part shifts, the
 // next 8 bits index the table of 2^(-i/256) (Tang's table-driven method), the
 // rest takes the Taylor polynomial of degree 5 of e^-z, z < 2^-8 ln 2. c and
-// its powers keep their own exponent until they meet e^-c.
+// its powers keep their own exponent until they meet e^-c. The mean errors
+// are below 2^-61: a common shift of all entries, 2^-58 say, would reach a
+// small pivot of every block with the same sign, and add up over the blocks.
 template <int CODE>
 SV_FX void fx_matern(uint64_t s, int es, const uint64_t* T, uint64_t& M, uint64_t& g) {
   s = s > 0 ? s : 1;  // r = 0: M and g come out as 1 less the rounding below
@@ -238,16 +243,16 @@ SV_FX void fx_matern(uint64_t s, int es, const uint64_t* T, uint64_t& M, uint64_
   const int64_t st = fx_rsqrt_step(m, y0, q);
   q = (q << 2) + (uint64_t)(fx_scale_step(q, st) * 4);  // sqrt(m), Q62
   const int E = es + 1 - h2 / 2;                        // sqrt(s) = q 2^E
-  const uint64_t t0 = fx_mulhi(q << 1, CODE == 1 ? kFxK3 : kFxK5);  // Q60
+  const uint64_t t0 = fx_mulhi(q << 1, CODE == 1 ? kFxK3 : kFxK5) + 2;  // Q60; 2: the mean of what is dropped
   // t in Q57; beyond 79 (E > 5) the results are below 2^-70
   const int sh = 3 - E;
-  const uint64_t t = sh >= 0 ? fx_shr(t0, sh) : t0 << (E > 5 ? 0 : -sh);
+  const uint64_t t = sh >= 0 ? fx_shr(t0 + (fx_shl1(sh) >> 1), sh) : t0 << (E > 5 ? 0 : -sh);
   const uint32_t th = (uint32_t)(t >> 32);
   const int n = E > 5 ? 128 : (int)(th >> 25);
   const uint64_t rem = t & ((1ull << 49) - 1);
   const uint64_t e = fx_mulhi(fx_exp_tail(fx_mulhi(rem << 14, kFxLn2)), T[(th >> 17) & 255]);  // Q62
   const uint64_t c = fx_mulhi(q << 1, CODE == 1 ? kFxA3 : kFxA5);  // c = this 2^E, Q60
-  const uint64_t F = fx_mulhi(c << 1, e << 1);                     // c e^-c, Q60 before the shift
+  const uint64_t F = fx_mulhi(c << 1, e << 1) + 1;                 // c e^-c, Q60 before the shift
   const uint64_t e0 = fx_shr(e, n + 1);
   const int kf = n - E - 1;  // -1 only at c < 1: the shift up by one
   const uint64_t eF = e0 + (kf < 0 ? F << 1 : fx_shr(F, kf));
@@ -255,9 +260,9 @@ SV_FX void fx_matern(uint64_t s, int es, const uint64_t* T, uint64_t& M, uint64_
     M = eF;
     g = e0;
   } else {
-    const uint64_t G = fx_mulhi(fx_mulhi(c << 1, F << 1) << 2, kFxThird);  // c^2 e^-c / 3, Q59
+    const uint64_t G = fx_mulhi(fx_mulhi(c << 1, F << 1) << 2, kFxThird) + 1;  // c^2 e^-c / 3, Q59
     const int kg = n - 2 * E - 2;
-    M = eF + (kg < 0 ? G << -kg : fx_shr(G, kg));
+    M = eF + (kg < 0 ? G << -kg : fx_shr(G, kg)) + 1;
     g = eF;
   }
 }

@@ -8,7 +8,7 @@
 // (sv_fix.cuh). k_block_warp is bound by the float64 pipe (64 cycles per warp
 // instruction and scheduler, 2,310 of them per block of 31); here the pipe is
 // left with the coordinate differences and the conversion of the results, and
-// the work is on the integer multiply-adds (2 cycles each).
+// the work is on the integer multiply-adds (4 cycles each).
 //
 //   * coordinates centred on the block's own point, in units of 2^es, 8 times
 //     the block's largest coordinate: r^2 = n_i + n_j - 2 U_i . U_j with an
@@ -28,10 +28,10 @@
 // Measured at n = 200,000, d = 10, m = 30: 10.2 ms, where k_block_warp takes
 // 27.3 ms; the integer multiply pipe is 65 % busy, the float64 pipe 6 %
 // (3 warps per scheduler, one block of 18 KB of shared memory each). Errors
-// against 113-bit arithmetic at n = 500, m = 30 (float64 kernels in brackets):
-// tau = 1e-4, d = 8: log-likelihood 1e-17 (1.9e-14), score 2e-15 (3e-14),
-// Fisher 3e-16 (5e-15); tau = 1e-8, d = 3: 9e-11 (1.4e-9), 1.2e-10 (1.6e-9),
-// 1.3e-11 (1.4e-10).
+// against 64-bit-mantissa long double at n = 4,000, m = 30 (float64 kernels in
+// brackets): tau = 1e-4, d = 4: log-likelihood 2e-14 (1.6e-13), score 3e-14
+// (1.9e-13), Fisher 4e-15 (5e-14); tau = 1e-8, d = 3: 4e-12 (7e-10), 2e-11
+// (1.4e-9), 1.5e-11 (4.7e-10).
 //
 // What has no such bound goes to the float64 kernels: a block with a pivot
 // below 2^-34 of the diagonal (its jitter ladder is theirs), coordinates
