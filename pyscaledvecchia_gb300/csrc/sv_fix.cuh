@@ -1,12 +1,13 @@
-// Fixed-point arithmetic of the likelihood blocks (sv_loglik_fix.cu): numbers
+// Fixed-point arithmetic of the likelihood and prediction blocks
+// (sv_loglik_fix.cu, sv_predict_fix.cu) and of the Matern tables: numbers
 // of magnitude at most 1 as 64-bit integers in units of 2^-58 ("Q58"), split
 // for products into two 30-bit limbs, x = h 2^30 + l with |l| <= 2^29.
 //
 // GB300 issues a float64 warp instruction every 64 cycles per scheduler and a
-// 32 x 32 + 64 bit integer multiply-add every 2 (both measured). A product of
+// 32 x 32 + 64 bit integer multiply-add every 4 (both measured). A product of
 // two split numbers accumulated over a sum takes three of the latter: h h'
 // into one 64-bit accumulator, h l' + l h' into another (l l' lies below
-// 2^-60 and is left out). So a multiply-add costs 6 cycles instead of 64, its
+// 2^-60 and is left out). So a multiply-add costs 12 cycles instead of 64, its
 // accumulation is exact, and the one rounding per sum, 2^-58 of the scale, is
 // 32 times finer than float64's at that scale. Correlations, their Cholesky
 // factor and the whitened columns are bounded by construction, so the scale is
