@@ -317,7 +317,9 @@ class DeviceProblem:
             self._ws = _lib.workspace(torch, nbytes)
         nout = 1 + P + P * P + self.q
         if self.out is None or self.out.numel() != nout:
-            self.out = torch.empty(nout, dtype=torch.float64, device="cuda")
+            # results and status words in one buffer, read back by one copy
+            self._res = torch.zeros(nout + 2, dtype=torch.float64, device="cuda")
+            self.out, self.info = self._res[:nout], self._res[nout:].view(torch.int32)
         chunk = self.chunk_tensor(P if need_grad else 1) if chunked else None
         st = stream if stream is not None else _lib.stream_handle(torch)
         rc = lib.sv_vecchia_loglik(D, _lib.ptr(theta_dev), _lib.ptr(self.X), _lib.ptr(self.y),
@@ -339,9 +341,9 @@ class DeviceProblem:
         th = _lib.to_dev(torch, theta[:P], np.float64)
         self.launch(th, P, nu, estimate_nu, need_grad, var_penalty, log_var_target, chunked,
                     precision=precision, team_lanes=team_lanes)
-        res = torch.cat([self.out, self.info.to(torch.float64)]).cpu().numpy()
+        res = self._res.cpu().numpy()
         nout = 1 + P + P * P + self.q
-        self.last_info = res[nout:].astype(np.int64)
+        self.last_info = res[nout:].view(np.int32).astype(np.int64)
         _lib.check_info(self.lib, self.last_info, "sv_vecchia_loglik")
         ll = float(res[0])
         beta = res[1 + P + P * P:nout].copy() if self.has_Z else np.zeros(0)
