@@ -819,7 +819,7 @@ __global__ void k_final1(RedArgs R) {
 // A lane's blocks are every 32nd of the CTA's run, in order, then the lanes
 // are added up: by one warp, or with a warp for each of up to kRedWide blocks
 // of a lane, whose terms then meet in the same order.  The width depends on
-// the launch, so the bits must not depend on the width, nor on PR (every
+// the launch's largest problem, so the bits must not depend on the width, nor on PR (every
 // operation is written out).  PR: parameters whose sums are held in registers (a runtime count puts them
 // into local memory: 131 us instead of 111 at 200,000 blocks)
 template <int PR>
@@ -1298,13 +1298,11 @@ int run_eval(const EvalCall& C, cudaStream_t st, const ShardStage* sh = nullptr)
     k_final1<<<(unsigned)S.nprob, kRedThreads, 0, st>>>(R);
     SV_CUDA_TRY(cudaGetLastError());
     if (npart > 0) {
-      // a thread per block of a CTA's run while the CTAs do not fill the SMs
-      // (runs of at most 128 blocks; beyond 8,192 blocks they have 114 to 128);
-      // beyond that one warp, four blocks a thread: the sums over a warp are
-      // most of the float64 work
+      // a thread per block of a CTA's run (at most 128 blocks; beyond 8,192
+      // blocks they have 114 to 128): one warp with four blocks a thread took
+      // 150 us at 200,000 blocks, this 55 (a CTA of 256 per partition 79)
       const int64_t run = S.nblk_max > 8192 ? 128 : (S.nblk_max + 8 * kRedCl - 1) / (8 * kRedCl);
-      const bool wide = (int64_t)npart * kRedCl * S.nprob <= 2 * sv_num_sms() &&
-                        S.nblk_max <= 4096 * 1024 && S.Pmax <= 16;
+      const bool wide = S.nblk_max <= 4096 * 1024 && S.Pmax <= 16;
       const int thr = wide ? std::max(32, (int)((run + 31) / 32 * 32)) : 32;
       if (S.Pmax <= 8)
         k_reduce2<8><<<rgrid, thr, 0, st>>>(R);
