@@ -819,9 +819,10 @@ __global__ void k_final1(RedArgs R) {
 // A lane's blocks are every 32nd of the CTA's run, in order, then the lanes
 // are added up: by one warp, or with a warp for each of up to kRedWide blocks
 // of a lane, whose terms then meet in the same order.  The width depends on
-// the launch's largest problem, so the bits must not depend on the width, nor on PR (every
-// operation is written out).  PR: parameters whose sums are held in registers (a runtime count puts them
-// into local memory: 131 us instead of 111 at 200,000 blocks)
+// the launch's largest problem, so the bits must not depend on the width, nor
+// on PR (every operation is written out).  PR: parameters whose sums are held
+// in registers (a runtime count puts them into local memory: 131 us instead of
+// 111 at 200,000 blocks, before the lanes' sums were shared)
 template <int PR>
 __global__ void __cluster_dims__(kRedCl, 1, 1) k_reduce2(RedArgs R) {
   cg::cluster_group cl = cg::this_cluster();
