@@ -150,8 +150,14 @@ class DeviceProblem:
         del pending
         self._chunks = {}
         self._ws = None
+        # the status words between the results without and with an estimated
+        # nu, so that either comes to the host with them in one copy; laid out
+        # here, since launch() may be given a stream that is ahead of this one
+        self._n0, self._n1 = (1 + P + P * P + self.q for P in (self.d + 2, self.d + 3))
+        self._res = torch.empty(self._n0 + 2 + self._n1, dtype=torch.float64, device="cuda")
         self.out = None
-        self.info = _lib.new_info(torch)
+        self.info = self._res[self._n0:self._n0 + 2].view(torch.int32)
+        self.info.zero_()
 
     def _pack_on_device(self, groups):
         """Enqueue the block table of ``pack_groups`` built on the device
@@ -315,11 +321,7 @@ class DeviceProblem:
         nbytes = lib.sv_loglik_workspace_bytes(D)
         if self._ws is None or self._ws.numel() < nbytes:
             self._ws = _lib.workspace(torch, nbytes)
-        nout = 1 + P + P * P + self.q
-        if self.out is None or self.out.numel() != nout:
-            # results and status words in one buffer, read back by one copy
-            self._res = torch.zeros(nout + 2, dtype=torch.float64, device="cuda")
-            self.out, self.info = self._res[:nout], self._res[nout:].view(torch.int32)
+        self.out = self._res[self._n0 + 2:] if estimate_nu else self._res[:self._n0]
         chunk = self.chunk_tensor(P if need_grad else 1) if chunked else None
         st = stream if stream is not None else _lib.stream_handle(torch)
         rc = lib.sv_vecchia_loglik(D, _lib.ptr(theta_dev), _lib.ptr(self.X), _lib.ptr(self.y),
@@ -341,9 +343,14 @@ class DeviceProblem:
         th = _lib.to_dev(torch, theta[:P], np.float64)
         self.launch(th, P, nu, estimate_nu, need_grad, var_penalty, log_var_target, chunked,
                     precision=precision, team_lanes=team_lanes)
-        res = self._res.cpu().numpy()
         nout = 1 + P + P * P + self.q
-        self.last_info = res[nout:].view(np.int32).astype(np.int64)
+        if estimate_nu:
+            res = self._res[self._n0:].cpu().numpy()
+            inf, res = res[:2], res[2:]
+        else:
+            res = self._res[:self._n0 + 2].cpu().numpy()
+            inf = res[nout:]
+        self.last_info = inf.view(np.int32).astype(np.int64)
         _lib.check_info(self.lib, self.last_info, "sv_vecchia_loglik")
         ll = float(res[0])
         beta = res[1 + P + P * P:nout].copy() if self.has_Z else np.zeros(0)
