@@ -224,27 +224,67 @@ SV_FX uint64_t fx_exp_tail(uint64_t z) {
   return (1ull << 63) - (z >> 7) + (z2 >> 18) - (((uint64_t)z3 * c3) >> 28);
 }
 
-// Matern 3/2 (code 1) and 5/2 (code 2) of a squared distance s (Q62) in units
-// of 2^(2 es): the correlation M, and the factor of its
+// The squared distance of two points whose coordinates are split integers
+// below 2^59: per input the square of the difference dh 2^30 + dl, exactly, as
+// three sums at 2^60, 2^31 and 1. Differences first, so that a close pair keeps
+// its relative accuracy however far both lie from the origin, and equal rows
+// come out at 0 (|x|^2 + |y|^2 - 2 x.y is off by a unit of the whole extent's
+// square: 31 ranges from the origin that reached 2^-46 of the variance, and
+// had one sign for replicates). The limbs' differences are as many multiply-adds.
+struct FxSq {
+  uint64_t hh, ll;  // sums of 12 squares below 2^60
+  int64_t hl;
+};
+SV_FX void fx_sqdiff(FxSq& a, Fx2 x, Fx2 y) {
+  const int32_t dh = x.h - y.h, dl = x.l - y.l;  // |dh| <= 2^30, |dl| < 2^30
+  a.hh += (uint64_t)((int64_t)dh * dh);
+  a.hl += (int64_t)dh * dl;
+  a.ll += (uint64_t)((int64_t)dl * dl);
+}
+// after 8 terms: room for 4 more in the middle sum, which is at most
+// 2^30 sqrt(8 hh) (below 64 it needs none, and hh might go below 0)
+SV_FX void fx_sqcarry(FxSq& a) {
+  const int64_t t = a.hh >= 64 ? a.hl >> 29 : 0;
+  a.hh += (uint64_t)t;
+  a.hl -= (int64_t)((uint64_t)t << 29);
+}
+// The sum as s 2^(2 E) with s in [1/4, 1), Q64 (truncated), for coordinates in
+// Q61 of 2^es; a sum of 0 reads as s = 1/4, E = es - 92 (es <= 7: it correlates
+// by 1)
+SV_FX uint64_t fx_sqnorm(const FxSq& a, int es, int& E) {
+  const uint64_t l0 = a.hh << 60, l1 = (uint64_t)a.hl << 31;
+  uint64_t lo = l0 + l1, hi = (a.hh >> 4) + (uint64_t)(a.hl >> 33) + (lo < l0 ? 1 : 0);
+  lo += a.ll;
+  hi += lo < a.ll ? 1 : 0;
+  const bool low = hi == 0;
+  hi = low ? lo : hi;
+  lo = low ? 0 : lo;
+  const bool none = hi == 0;
+  hi |= none ? 1 : 0;
+  const int z = fx_clz(hi) & ~1;
+  E = es + 3 - z / 2 - (low ? 32 : 0) - (none ? 32 : 0);
+  return hi << z | (lo >> 1) >> (63 - z);
+}
+
+// Matern 3/2 (code 1) and 5/2 (code 2) of a squared distance s 2^(2 E), s in
+// [1/4, 1) (Q64): the correlation M, and the factor of its
 // derivative, g = e^-c (3/2: M'(r)/r = -3 g) or (1 + c) e^-c (5/2:
 // M'(r)/r = -5/3 g), c = sqrt(3) r or sqrt(5) r; both in Q61, absolute error
-// a few 2^-59. exp(-c) = 2^-t, t = c log2 e: the integer part shifts, the
+// a few 2^-59. SCALED: g 2^(2 E) instead (below 1.5, since 2^E < 2 r), to
+// which squared differences in units of 2^E belong. exp(-c) = 2^-t,
+// t = c log2 e: the integer part shifts, the
 // next 8 bits index the table of 2^(-i/256) (Tang's table-driven method), the
 // rest takes the Taylor polynomial of degree 5 of e^-z, z < 2^-8 ln 2. c and
 // its powers keep their own exponent until they meet e^-c. The mean errors
 // are below 2^-61: a common shift of all entries, 2^-58 say, would reach a
 // small pivot of every block with the same sign, and add up over the blocks.
-template <int CODE>
-SV_FX void fx_matern(uint64_t s, int es, const uint64_t* T, uint64_t& M, uint64_t& g) {
-  s = s > 0 ? s : 1;  // r = 0: M and g come out as 1 less the rounding below
-  const int h2 = fx_clz(s) & ~1;
-  const uint64_t m = s << h2 >> 1;  // Q63
+template <int CODE, bool SCALED>
+SV_FX void fx_matern_norm(uint64_t s, int E, const uint64_t* T, uint64_t& M, uint64_t& g) {
   uint32_t y0;
   uint64_t q;
-  const int64_t st = fx_rsqrt_step(m, y0, q);
-  q = (q << 2) + (uint64_t)(fx_scale_step(q, st) * 4);  // sqrt(m), Q62
-  const int E = es + 1 - h2 / 2;                        // sqrt(s) = q 2^E
-  const uint64_t t0 = fx_mulhi(q << 1, CODE == 1 ? kFxK3 : kFxK5) + 2;  // Q60; 2: the mean of what is dropped
+  const int64_t st = fx_rsqrt_step(s >> 1, y0, q);
+  q = (q << 2) + (uint64_t)(fx_scale_step(q, st) * 4);  // sqrt(s), Q62
+  const uint64_t t0 = fx_mulhi(q << 1, CODE == 1 ? kFxK3 : kFxK5) + 2;  // Q60; 2: the mean of what the products drop
   // t in Q57; beyond 79 (E > 5) the results are below 2^-70
   const int sh = 3 - E;
   const uint64_t t = sh >= 0 ? fx_shr(t0 + (fx_shl1(sh) >> 1), sh) : t0 << (E > 5 ? 0 : -sh);
@@ -259,13 +299,22 @@ SV_FX void fx_matern(uint64_t s, int es, const uint64_t* T, uint64_t& M, uint64_
   const uint64_t eF = e0 + (kf < 0 ? F << 1 : fx_shr(F, kf));
   if (CODE == 1) {
     M = eF;
-    g = e0;
+    g = SCALED ? fx_shr(e, n + 1 - 2 * E) : e0;
   } else {
     const uint64_t G = fx_mulhi(fx_mulhi(c << 1, F << 1) << 2, kFxThird) + 1;  // c^2 e^-c / 3, Q59
     const int kg = n - 2 * E - 2;
     M = eF + (kg < 0 ? G << -kg : fx_shr(G, kg)) + 1;
-    g = eF;
+    const int ks = kf - 2 * E;
+    g = SCALED ? fx_shr(e, n + 1 - 2 * E) + (ks < 0 ? F << -ks : fx_shr(F, ks)) : eF;
   }
+}
+// the same of s in Q62 of 2^(2 es); r = 0: M and g come out as 1 less the
+// rounding
+template <int CODE>
+SV_FX void fx_matern(uint64_t s, int es, const uint64_t* T, uint64_t& M, uint64_t& g) {
+  s = s > 0 ? s : 1;
+  const int z = fx_clz(s) & ~1;
+  fx_matern_norm<CODE, false>(s << z, es + 1 - z / 2, T, M, g);
 }
 
 // x 2^n, rounded to nearest (ties up) where bits are lost; the result fits

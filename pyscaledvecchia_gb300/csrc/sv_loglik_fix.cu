@@ -10,9 +10,9 @@
 // left with the coordinate differences and the conversion of the results, and
 // the work is on the integer multiply-adds (4 cycles each).
 //
-//   * coordinates centred on the block's own point, in units of 2^es, 8 times
-//     the block's largest coordinate: r^2 = n_i + n_j - 2 U_i . U_j with an
-//     absolute error of about 2^-61 of the unit's square;
+//   * coordinates centred on the block's own point, in units of 2^-61 of 4 to
+//     8 times the block's largest coordinate; r^2 as the exact sum of the
+//     squared differences, with an exponent of its own;
 //   * the covariance is scaled by its own variance and a power of two,
 //     Sigma = s2 2^ek (M 2^-ek + tau 2^-ek I), so that its diagonal lies in
 //     (1/2, 1] and its Cholesky factor's entries are below 1 whatever the
@@ -20,9 +20,12 @@
 //     the diagonal, where float64's is about K 2^-53;
 //   * the factor's inverse T comes with it (fix_factor): its last row is
 //     a = C^-T e_K, and the solves W = C^-1 V are products with T;
-//   * dSigma_l a as one matrix product with the pairs' g: for every input,
-//     sum_j g_ij (U_i - U_j)^2 a_j = U_i^2 (G a)_i - 2 U_i (G aU)_i +
-//     (G aU^2)_i, U in units of the input's own extent in the block;
+//   * dSigma_l a = sum_j g_ij (U_i - U_j)^2 a_j from the differences as well,
+//     every pair's in units of the pair's own distance 2^E (their square
+//     joins g, which is bounded however far the points): errors of 2^-58 of
+//     the variance at any extent. (As three matrix products, U_i^2 (G a)_i -
+//     2 U_i (G aU)_i + (G aU^2)_i, they were 2^-58 of the extent's square, and
+//     it takes as many multiply-adds);
 //   * rows of T, right-hand sides and solutions carry power-of-two scales.
 //
 // Measured at n = 200,000, d = 10, m = 30: 10.2 ms, where k_block_warp takes
@@ -43,7 +46,8 @@
 namespace sv {
 
 constexpr int kFixThreads = 384;
-constexpr int kFixV = 4;  // inputs per pass over the pairs' g
+constexpr int kFixV = 6;  // inputs per pass over the pairs' g at most
+constexpr int kFixEsMin = -27;  // smallest unit of the coordinates (pairs' exponents are bytes)
 
 __device__ __forceinline__ double pow2(int n) {
   return n < -1022 ? 0.0 : __longlong_as_double((long long)(min(n, 1023) + 1023) << 52);
@@ -57,27 +61,25 @@ __host__ __device__ inline int fix_g_words(int G, int kcap, int ncol) {
   const int g = kcap * (kcap - 1) / 2, w = (G + 1) * ncol;  // pairs' g, then the solutions
   return ((g > w ? g : w) + 1) & ~1;
 }
-// products of kFixV inputs with a, then the columns' scales and last rows
-__host__ __device__ inline int fix_p_words(int kcap) {
-  return 2 * kFixV * kcap > 2 * kFixCols ? 2 * kFixV * kcap : 2 * kFixCols;
-}
+// exponents of the pairs' distances (at most 496 bytes), then the columns'
+// scales and last rows
+constexpr int kFixPWords = 2 * kFixCols;
 __host__ __device__ inline int fix_slot_words(int G, int kcap, int ncol, int rs) {
   int s = kcap * (G + 2);            // M
   s += fix_g_words(G, kcap, ncol);
   s += rs * kcap;                    // coordinates, then right-hand sides
-  s += fix_p_words(kcap);
-  s += 2 * G;                        // a, norms
+  s += kFixPWords;
+  s += G;                            // a
   return (s + 1) & ~1;
 }
 
 template <int G>
 struct FixSlot {
   Fx2* M;
-  Fx2* Gp;   // g of the pairs i > j at i(i-1)/2 + j; then the solutions (column stride kCs)
+  Fx2* Gp;   // g 2^(2 E) of the pairs i > j at i(i-1)/2 + j; then the solutions (column stride kCs)
+  signed char* Ep;  // their E
   Fx2* cv;   // [point][rs]
-  Fx2* Pm;
   Fx2* us;
-  int64_t* nrm;
   int rs;
 };
 
@@ -95,9 +97,8 @@ __device__ __forceinline__ void fix_assemble(int K, int d, int tl, int es, int e
 #pragma unroll
       for (int l = g; l < g + 4; ++l) ui[l] = S.cv[tl * S.rs + l];
     }
-  const int64_t ni = S.nrm[tl];
   for (int r = 1; 2 * r <= K; r += 2) {
-    int jj[2];
+    int jj[2], E[2];
     uint64_t s[2], m[2], g[2];
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
@@ -106,31 +107,27 @@ __device__ __forceinline__ void fix_assemble(int K, int d, int tl, int es, int e
       if (2 * (r + t) > K || (2 * (r + t) == K && tl >= r + t)) j = tl;  // no such pair
       jj[t] = j;
       const Fx2* uj = S.cv + j * S.rs;
-      int64_t hh = 0, cr = 0;
+      FxSq q = {0, 0, 0};
 #pragma unroll
       for (int g4 = 0; g4 < kFixMaxD; g4 += 4)
         if (g4 < d) {
           Fx2 v[4];
           load4(uj + g4, v);
+          if (g4 == 8) fx_sqcarry(q);
 #pragma unroll
-          for (int l = 0; l < 4; ++l) {
-            hh += (int64_t)ui[g4 + l].h * v[l].h;
-            cr += (int64_t)ui[g4 + l].h * v[l].l;
-            cr += (int64_t)ui[g4 + l].l * v[l].h;
-          }
+          for (int l = 0; l < 4; ++l) fx_sqdiff(q, ui[g4 + l], v[l]);
         }
-      // in [0, 3) 2^62; what rounds below 0 reads as close to 2^64
-      const uint64_t x = (uint64_t)(ni + S.nrm[j]) - ((uint64_t)hh << 1) - (uint64_t)((cr + (1ll << 28)) >> 29);
-      s[t] = x > ~0xfffffull ? 0 : x;
+      s[t] = fx_sqnorm(q, es, E[t]);
     }
 #pragma unroll
-    for (int t = 0; t < 2; ++t) fx_matern<CODE>(s[t], es, T, m[t], g[t]);
+    for (int t = 0; t < 2; ++t) fx_matern_norm<CODE, true>(s[t], E[t], T, m[t], g[t]);
 #pragma unroll
     for (int t = 0; t < 2; ++t)
       if (jj[t] != tl) {
         const int lo = min(tl, jj[t]), hi = max(tl, jj[t]);
         *(int64_t*)(S.M + lo * St + hi) = (int64_t)((m[t] + (4ull << ek)) >> (3 + ek));
         S.Gp[hi * (hi - 1) / 2 + lo] = fx_split((int64_t)((g[t] + 4) >> 3));
+        S.Ep[hi * (hi - 1) / 2 + lo] = (signed char)E[t];
       }
   }
 }
@@ -144,70 +141,73 @@ __device__ __forceinline__ int fix_put_rhs(int64_t x, int E, bool own, Fx2* p) {
   return f;
 }
 
-// dSigma_l a for NV inputs l0 .. l0 + NV - 1, in place of their coordinates;
-// fc[l] their scales. FIRST also takes G a. Returns false when a sum does not
-// fit.
-template <int G, int NV, bool FIRST>
-__device__ __forceinline__ bool fix_dsig(int K, int d, int l0, int tl, int es, int E, const FixSlot<G>& S, Fx2 usi,
-                                         int& fc, int64_t& A0) {
+// dSigma_l a for NV inputs l0 .. l0 + NV - 1, in place of their coordinates
+// (plain Q61 integers here); fc[l] their scales. Each unordered pair is met
+// once, as in fix_assemble: lane i squares the difference to i + r, and lane
+// i + r has the square from it by a shuffle. The square in units of the pair's
+// 2^(2 E) is at most 1 (Q62; 2: the mean of what is dropped below it, 0 for equal
+// rows), its weight g 2^(2 E) a_j below 0.75 (Q58)
+template <int G, int NV>
+__device__ __forceinline__ void fix_dsig(int K, int Kw, int d, int l0, int tl, int es, int E, const FixSlot<G>& S,
+                                         int& fc) {
   const bool own = tl < K;
-  Fx2* cv = S.cv + tl * S.rs;
-  Fx2 U[NV];
-  int ex[NV];
+  const int i = own ? tl : 0;
+  Fx2* cv = S.cv + i * S.rs;
+  int64_t U[NV];
 #pragma unroll
-  for (int t = 0; t < NV; ++t) {
-    const int l = l0 + t;
-    const int64_t x = (own && l < d) ? fx_join(cv[l]) : 0;
-    const int len = team_max<G>(fx_bits(x));
-    const int sh = len > 0 ? 58 - len : 0;  // |x| < 2^59
-    ex[t] = es - 3 - sh;
-    U[t] = fx_split(fx_scale2(x, sh));
-    const Fx2 p1 = fx_split(fx_mul(usi, U[t]));
-    const Fx2 p2 = fx_split(fx_mul(p1, U[t]));
-    if (own) {
-      S.Pm[2 * NV * tl + 2 * t] = p1;
-      S.Pm[2 * NV * tl + 2 * t + 1] = p2;
+  for (int t = 0; t < NV; ++t) U[t] = *(const int64_t*)(cv + l0 + t);
+  int64_t ah[NV], am[NV];  // Q58, Q88
+#pragma unroll
+  for (int t = 0; t < NV; ++t) ah[t] = am[t] = 0;
+#pragma unroll 1
+  for (int r = 1; 2 * r <= Kw; ++r) {
+    const bool fwd = own && 2 * r <= K, rev = own && 2 * r < K;
+    int j = i + r, jr = i - r;
+    if (j >= K) j -= K;
+    if (jr < 0) jr += K;
+    if (!fwd) j = i;
+    if (!rev) jr = i;
+    const int hi = max(i, j), at = fwd ? hi * (hi - 1) / 2 + min(i, j) : 0;
+    const int hr = max(i, jr), ar = rev ? hr * (hr - 1) / 2 + min(i, jr) : 0;
+    const Fx2 w = fx_keep(fx_split(fx_mul(S.Gp[at], S.us[j])), fwd ? -1 : 0);
+    const Fx2 wr = fx_keep(fx_split(fx_mul(S.Gp[ar], S.us[jr])), rev ? -1 : 0);
+    const int k = es + 2 - S.Ep[at];
+    const Fx2* uj = S.cv + j * S.rs + l0;
+#pragma unroll
+    for (int t = 0; t < NV; t += 2) {
+      const longlong2 v = *(const longlong2*)(uj + t);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int64_t D = (int64_t)((uint64_t)(U[t + u] - (u ? v.y : v.x)) << (k & 63));  // Q63
+        const int h = (int)(D >> 32), l = (int)((uint32_t)D >> 1);
+        const int64_t q = (int64_t)h * h + 2 + (((int64_t)h * l) >> 30);
+        const int qh = (int)(q >> 32), ql = (int)((uint32_t)q >> 2);
+        const int rh = __shfl_sync(kFull, qh, jr, G), rl = __shfl_sync(kFull, ql, jr, G);
+        ah[t + u] += (int64_t)w.h * qh;
+        ah[t + u] += (int64_t)wr.h * rh;
+        am[t + u] += (int64_t)w.h * ql;
+        am[t + u] += (int64_t)w.l * qh;
+        am[t + u] += (int64_t)wr.h * rl;
+        am[t + u] += (int64_t)wr.l * rh;
+      }
+    }
+    if ((r & 3) == 3) {  // the middle sums hold 9 pairs' at least
+#pragma unroll
+      for (int t = 0; t < NV; ++t) {
+        ah[t] += am[t] >> 30;
+        am[t] &= (1ll << 30) - 1;
+      }
     }
   }
   __syncwarp();
-  FxAcc a0 = {0, 0}, a[2 * NV];
-#pragma unroll
-  for (int t = 0; t < 2 * NV; ++t) a[t] = {0, 0};
-  const int i = own ? tl : 0;
-  const Fx2* pj = S.Pm;
-  const Fx2* row = S.Gp + i * (i - 1) / 2;
-  int off = 0;  // j (j - 1) / 2
-#pragma unroll 2
-  for (int j = 0; j < K; ++j, pj += 2 * NV) {
-    Fx2 g = j > i ? S.Gp[off + i] : row[j < i ? j : 0];
-    if (j == i) g = {0, 0};
-    off += j;
-    if (FIRST) fx_mac(a0, g, S.us[j]);
-#pragma unroll
-    for (int t = 0; t < 2 * NV; t += 4) {
-      Fx2 p[4];
-      load4(pj + t, p);
-#pragma unroll
-      for (int w = 0; w < 4; ++w) fx_mac(a[t + w], g, p[w]);
-    }
-  }
-  if (FIRST) A0 = fx_val(a0);
-  int64_t mx = A0 < 0 ? -A0 : A0;
-  const Fx2 A0s = fx_split(A0);
 #pragma unroll
   for (int t = 0; t < NV; ++t)
     if (l0 + t < kFixMaxD) {
-      const int64_t a1 = fx_val(a[2 * t]), a2 = fx_val(a[2 * t + 1]);
-      mx |= (a1 < 0 ? -a1 : a1) | (a2 < 0 ? -a2 : a2);
-      // U (U A0 - 2 a1) + a2
-      const int64_t in = fx_mul(U[t], A0s) - 2 * a1;
-      const int64_t v = a2 + fx_mul(U[t], fx_split(in));
       const bool put = own && l0 + t < d;
-      const int f = fix_put_rhs<G>(v, E, put, cv + l0 + t);
-      if (tl == l0 + t) fc = f + 2 * ex[t];
+      const int f = fix_put_rhs<G>(ah[t] + ((am[t] + (1ll << 29)) >> 30), E, put, cv + l0 + t);
+      if (tl == l0 + t) fc = f;
     }
   __syncwarp();
-  return !own || mx < (1ll << 59);
 }
 
 template <int G>
@@ -223,11 +223,10 @@ __global__ void __launch_bounds__(kFixThreads, 1) k_block_fix(LikArgs A, int wpc
   S.M = (Fx2*)(smem + 256 + (int64_t)(warp * NB + tm) * fix_slot_words(G, kcap, ncap, rs));
   S.Gp = S.M + kcap * St;
   S.cv = S.Gp + fix_g_words(G, kcap, ncap);
-  S.Pm = S.cv + rs * kcap;
-  S.us = S.Pm + fix_p_words(kcap);
-  S.nrm = (int64_t*)(S.us + G);
+  double* scg = (double*)(S.cv + rs * kcap);  // column scales and last rows, after dSigma a
+  S.Ep = (signed char*)scg;
+  S.us = (Fx2*)scg + kFixPWords;
   S.rs = rs;
-  double* scg = (double*)S.Pm;   // column scales and last rows, after dSigma a
   double* wkd = scg + kFixCols;  // w_K of the parameters, then z_K of y and Z
 
   const int64_t nb = A.b1 - A.b0;
@@ -286,8 +285,8 @@ __global__ void __launch_bounds__(kFixThreads, 1) k_block_fix(LikArgs A, int wpc
         bad = true;
         exm = 2046;
       }
-      // Q61 with |U| < 1/4; n = |U|^2 in Q62
-      int64_t hh = 0, cr = 0, ll = 0;
+      exm = max(exm, kFixEsMin + 1023 - 3);
+      // Q61 with |U| < 1/4
 #pragma unroll
       for (int g = 0; g < kFixMaxD; g += 4)
         if (g < d) {
@@ -295,12 +294,8 @@ __global__ void __launch_bounds__(kFixThreads, 1) k_block_fix(LikArgs A, int wpc
           for (int l = g; l < g + 4; ++l) {
             const Fx2 u = fx_split(fx_from_bits<6>(dbits(v[l]), exm));
             if (own) S.cv[tl * rs + l] = u;
-            hh += (int64_t)u.h * u.h;
-            cr += (int64_t)u.h * u.l;
-            ll += (int64_t)u.l * u.l;
           }
         }
-      S.nrm[tl] = hh + ((2 * cr + (ll >> 30) + (1ll << 29)) >> 30);
     }
     const int es = bad ? 0 : exm - 1023 + 3;  // |u| 2^-es < 1/4
     if (own) *(int64_t*)(S.M + tl * St + tl) = PI.fix_diag;
@@ -327,15 +322,20 @@ __global__ void __launch_bounds__(kFixThreads, 1) k_block_fix(LikArgs A, int wpc
     int fc = 0, fc2 = 0;
     Fx2* cv = S.cv + tl * rs;
     if (A.need_grad) {
-      int64_t A0 = 0;
       const int dw = __reduce_max_sync(kFull, active ? d : 0);
-      if (!fix_dsig<G, kFixV, true>(K, d, 0, tl, es, E, S, usi, fc, A0)) bad = true;
-      int l0 = kFixV;
+      if (own) {
+#pragma unroll
+        for (int l = 0; l < kFixMaxD; ++l)
+          if (l < ((d + 3) & ~3)) *(int64_t*)(cv + l) = fx_join(cv[l]);
+      }
+      __syncwarp();
+      int l0 = 0;
 #pragma unroll 1
-      for (; l0 + 2 < dw; l0 += kFixV)
-        if (!fix_dsig<G, kFixV, false>(K, d, l0, tl, es, E, S, usi, fc, A0)) bad = true;
-      if (l0 < dw)
-        if (!fix_dsig<G, 2, false>(K, d, l0, tl, es, E, S, usi, fc, A0)) bad = true;
+      for (; l0 + 4 < dw; l0 += kFixV) fix_dsig<G, kFixV>(K, Kw, d, l0, tl, es, E, S, fc);
+      if (l0 + 2 < dw)
+        fix_dsig<G, 4>(K, Kw, d, l0, tl, es, E, S, fc);
+      else if (l0 < dw)
+        fix_dsig<G, 2>(K, Kw, d, l0, tl, es, E, S, fc);
       const int f = fix_put_rhs<G>(fx_join(usi), E, own, cv + d);  // nugget: s2 tau a
       if (tl == d) fc = f;
     }

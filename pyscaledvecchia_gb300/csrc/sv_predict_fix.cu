@@ -6,7 +6,7 @@
 // distance, a square root and an exponential per entry. Here the block's
 // covariance is scaled to a diagonal in (1/2, 1] (its Cholesky factor is then
 // bounded by 1) and factored in integers, three 2-cycle multiply-adds for one
-// of float64's; the entries come from fx_matern (float64 form, nu = 3/2 and
+// of float64's; the entries come from fx_matern_norm (float64 form, nu = 3/2 and
 // 5/2) or, as before, from the float32 deficits (split form).
 //
 // One CTA per block, 16 rows per warp, two lanes per row: lanes t and t + 16
@@ -48,7 +48,7 @@ __host__ __device__ inline int64_t pf_matrix_words(int K8) {
 __host__ __device__ inline int pf_rs(int d) { return d <= 4 ? 10 : ((d + 3) & ~3) + 2; }
 __host__ __device__ inline int64_t pf_words(int kt, int d) {
   const int64_t K8 = (kt + 7) & ~7;
-  // matrix, coordinates, norms, reciprocal roots and exponents, weights, exponents
+  // matrix, coordinates, pivot thresholds, reciprocal roots and exponents, weights, exponents
   const int64_t fix = pf_matrix_words((int)K8) + K8 * pf_rs(d) + K8 + K8 + K8 / 2 + K8 + K8 / 2 + 4;
   const int64_t old = pred_team_doubles(kt, d);
   return (fix > old ? fix : old) + 2;
@@ -205,14 +205,13 @@ __global__ void __launch_bounds__(NT, MINB) k_pred_fix(PredArgs A) {
     const int k = s_k, K = k + 1, K8 = (K + 7) & ~7;
     Fx2* M = (Fx2*)region;
     Fx2* cv = M + pf_matrix_words(K8);
-    int64_t* nrm = (int64_t*)(cv + K8 * rs);
-    Fx2* ivy = (Fx2*)(nrm + K8);
+    int64_t* thr = (int64_t*)(cv + K8 * rs);  // pivot thresholds
+    Fx2* ivy = (Fx2*)(thr + K8);
     int* ive = (int*)(ivy + K8);
     Fx2* us = (Fx2*)(ive + K8);
     int* Te = (int*)(us + K8);
     int64_t* last = (int64_t*)(Te + K8);   // pivot and C_KK of the last row
     Fx2* Tp = cv;                          // panels' inverse blocks, once the entries are there
-    int64_t* thr = nrm;                    // pivot thresholds, likewise
     const bool own = !boss && i < K;
     const int row = own ? (i < k ? A.nbr[b * A.ldnbr + i] : A.tgt[b]) : 0;
     // gp.py:263-265, 336-339: nugget on observations only (a prior draw keeps
@@ -253,22 +252,11 @@ __global__ void __launch_bounds__(NT, MINB) k_pred_fix(PredArgs A) {
           if (threadIdx.x == 0) s_bad = 1;
           exm = 2046;
         }
-        int64_t hh = 0, cr = 0, ll = 0;
 #pragma unroll
         for (int t = 0; t < kFixMaxD / 2; ++t) {
           const int l = 2 * t + half;
-          if (l < ((d + 3) & ~3)) {
-            const Fx2 u = fx_split(fx_from_bits<6>(dbits(v[t]), exm));
-            if (own) cv[i * rs + l] = u;
-            hh += (int64_t)u.h * u.h;
-            cr += (int64_t)u.h * u.l;
-            ll += (int64_t)u.l * u.l;
-          }
+          if (l < ((d + 3) & ~3) && own) cv[i * rs + l] = fx_split(fx_from_bits<6>(dbits(v[t]), exm));
         }
-        hh += __shfl_xor_sync(kFull, (long long)hh, 16);
-        cr += __shfl_xor_sync(kFull, (long long)cr, 16);
-        ll += __shfl_xor_sync(kFull, (long long)ll, 16);
-        if (own) nrm[i] = hh + ((2 * cr + (ll >> 30) + (1ll << 29)) >> 30);
       }
     }
     if (own && half == 0) *(int64_t*)(M + pf_col(i, K8) + i) = diag;
@@ -306,33 +294,28 @@ __global__ void __launch_bounds__(NT, MINB) k_pred_fix(PredArgs A) {
 #pragma unroll
             for (int l = g; l < g + 4; ++l) ui[l] = cv[i * rs + l];
           }
-        const int64_t ni = nrm[i];
         for (int r = 1 + half; 2 * r <= K; r += 2) {
           if (2 * r == K && i >= r) break;
           int j = i + r;
           if (j >= K) j -= K;
           const Fx2* uj = cv + j * rs;
-          int64_t hh = 0, cr = 0;
+          FxSq q = {0, 0, 0};
 #pragma unroll
           for (int g4 = 0; g4 < kFixMaxD; g4 += 4)
             if (g4 < d) {
               Fx2 w[4];
               load4(uj + g4, w);
+              if (g4 == 8) fx_sqcarry(q);
 #pragma unroll
-              for (int l = 0; l < 4; ++l) {
-                hh += (int64_t)ui[g4 + l].h * w[l].h;
-                cr += (int64_t)ui[g4 + l].h * w[l].l;
-                cr += (int64_t)ui[g4 + l].l * w[l].h;
-              }
+              for (int l = 0; l < 4; ++l) fx_sqdiff(q, ui[g4 + l], w[l]);
             }
-          // in [0, 3) 2^62; what rounds below 0 reads as close to 2^64
-          uint64_t s = (uint64_t)(ni + nrm[j]) - ((uint64_t)hh << 1) - (uint64_t)((cr + (1ll << 28)) >> 29);
-          s = s > ~0xfffffull ? 0 : s;
+          int E;
           uint64_t m, g;
+          const uint64_t s = fx_sqnorm(q, es, E);
           if (A.closed == 1)
-            fx_matern<1>(s, es, T, m, g);
+            fx_matern_norm<1, false>(s, E, T, m, g);
           else
-            fx_matern<2>(s, es, T, m, g);
+            fx_matern_norm<2, false>(s, E, T, m, g);
           const int lo = min(i, j), hi = max(i, j);
           *(int64_t*)(M + pf_col(lo, K8) + hi) = (int64_t)((m + (4ull << ek)) >> (3 + ek));
         }
