@@ -346,15 +346,18 @@ SV_FX double fx_to_double(uint64_t v, int ex) {
 constexpr uint64_t kFxTabS0 = 0x4d413cccfe779921ull;  // 2 (1 + sqrt 2), Q60
 constexpr uint64_t kFxTabS1 = 0x36a09e667f3bcc90ull;  // 2 + sqrt 2, Q60
 constexpr int64_t kFxTabO1 = 0x09a827999fcef324ll;    // 1 + sqrt 2, Q58
-constexpr uint64_t kFxLog2e = 0x5c551d94ae0bf85dull;  // log2 e, Q62
+constexpr uint64_t kFxLog2e = 0x5c551d94ae0bf85eull;  // log2 e, Q62
 // t in [-1, 1] (Q58) of the mantissa fraction f (52 bits) on the lower
 // ([1, sqrt2)) or upper ([sqrt2, 2)) half of an octave
 SV_FX int64_t fx_tab_t(uint64_t f, bool upper) {
   const uint64_t p = fx_mulhi(f << 11, upper ? kFxTabS1 : kFxTabS0);  // Q59
   return (int64_t)(p >> 1) - (upper ? kFxTabO1 : 1ll << 58);
 }
-// e^-c for c = (1 + f 2^-52) 2^e, e < 9: the result (Q62) times 2^-n.  t = c log2 e
-// in Q54 here, for c up to 2^9.
+// e^-c for c = (1 + f 2^-52) 2^e, -40 <= e < 9: the result (Q62) times 2^-n.
+// t = c log2 e, its fraction in Q57: rounded to nearest below c = 8 (e^-c is
+// within 2 units of 2^-58, and low or high by a third of one in the mean: an
+// error common to all near pairs adds up), truncated above, where e^-c is
+// small (the integer part must not take a carry)
 SV_FX uint64_t fx_exp_neg(uint64_t f, int e, const uint64_t* T, int& n) {
   const uint64_t m = (1ull << 62) + (f << 10);
 #if defined(__CUDA_ARCH__)
@@ -363,10 +366,11 @@ SV_FX uint64_t fx_exp_neg(uint64_t f, int e, const uint64_t* T, int& n) {
   const unsigned __int128 q = (unsigned __int128)m * kFxLog2e;
   const uint64_t p = (uint64_t)(q >> 64), pl = (uint64_t)q;
 #endif
-  const uint64_t t = e > 6 ? p << (e - 6) | pl >> (70 - e) : fx_shr(p + (e < 6 ? fx_shr(1ull << 5, e) : 0), 6 - e);
-  n = (int)(t >> 54);
-  const uint64_t rem = t & ((1ull << 46) - 1);
-  return fx_mulhi(fx_exp_tail(fx_mulhi(rem << 17, kFxLn2)), T[(t >> 46) & 255]);
+  const int sh = 3 - e;
+  const uint64_t t = sh > 0 ? (p + (1ull << (sh - 1))) >> sh : p << -sh | (pl >> 1) >> (63 + sh);
+  n = (int)(sh > 0 ? t >> 57 : p >> (57 + sh));
+  const uint64_t rem = t & ((1ull << 49) - 1);
+  return fx_mulhi(fx_exp_tail(fx_mulhi(rem << 14, kFxLn2)), T[(t >> 49) & 255]);
 }
 
 // mantissa and sign of a float64 (bits) as an integer in units of the power
