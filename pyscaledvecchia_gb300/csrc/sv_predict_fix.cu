@@ -29,9 +29,10 @@
 namespace sv {
 
 constexpr int kPfW = 8;     // columns per panel
-// weights |a_j| < 2^(kPfShift - 1) / C_KK, then (where one does not fit)
-// 2^(kPfShift2 - 1) / C_KK
-constexpr int kPfShift = 3, kPfShift2 = 12;
+// weights |a_j| < 2^(shift - 1) / C_KK, shift = 3 first; where one does not fit,
+// two bits more than it needs, up to 12: the column's unit stays below float64's
+// for its largest weight
+constexpr int kPfShift = 3, kPfShiftMax = 12;
 
 // column j's rows start at row 8 (j / 8); two words of padding keep the
 // columns' 16-byte loads apart
@@ -124,10 +125,7 @@ __device__ __forceinline__ void pf_diag(int K, int k0, int r, bool writer, Fx2* 
       if (writer) {
         ivy[c] = Y;
         ive[c] = e;
-        if (c == K - 1) {
-          last[0] = dv;
-          last[1] = x;
-        }
+        if (c == K - 1) *last = dv;
       }
       E = e + kFixHead;
       x = Yq >> kFixHead;
@@ -210,7 +208,7 @@ __global__ void __launch_bounds__(NT, MINB) k_pred_fix(PredArgs A) {
     int* ive = (int*)(ivy + K8);
     Fx2* us = (Fx2*)(ive + K8);
     int* Te = (int*)(us + K8);
-    int64_t* last = (int64_t*)(Te + K8);   // pivot and C_KK of the last row
+    int64_t* last = (int64_t*)(Te + K8);   // pivot of the last row
     Fx2* Tp = cv;                          // panels' inverse blocks, once the entries are there
     const bool own = !boss && i < K;
     const int row = own ? (i < k ? A.nbr[b * A.ldnbr + i] : A.tgt[b]) : 0;
@@ -406,10 +404,14 @@ __global__ void __launch_bounds__(NT, MINB) k_pred_fix(PredArgs A) {
 
     // ---- a = C^-T e_K, panels from the last to the first: the panel's 8 rows
     //      by the inverse of its diagonal block, then every earlier row its
-    //      terms (the two lanes of a row four each).  a = us 2^sa
-    int sa = ive[K - 1] + kPfShift;
+    //      terms (the two lanes of a row four each).  a = us 2^sa.  The sums
+    //      keep 2^-86 of the scale, since the inverse's entries magnify what
+    //      they lose: with one rounding to 2^-58 (and the products of low limbs
+    //      left out) a row's error was 8 2^-57 / C_jj, more than float64's
+    int shift = kPfShift;
     Fx2 ui = {0, 0};
-    for (int wide = 0; wide < 2; ++wide) {
+    for (;;) {
+      const int sa = ive[K - 1] + shift;
       FxAcc acc = {0, 0};
       for (int k0 = K8 - kPfW; k0 >= 0; k0 -= kPfW) {
         if (!boss && warp == (k0 >> 4)) {
@@ -417,13 +419,19 @@ __global__ void __launch_bounds__(NT, MINB) k_pred_fix(PredArgs A) {
           FxAcc tot = acc;
           tot.h += __shfl_xor_sync(kFull, (long long)acc.h, 16);
           tot.m += __shfl_xor_sync(kFull, (long long)acc.m, 16);
-          int64_t r = mine && own ? -fx_val(tot) : 0;
-          if (mine && i == K - 1) r += 1ll << (58 - sa);
+          const bool first = s_bad == 0;  // (behind a column that does not fit come meaningless ones)
+          // r 2^28 + lo in Q86
+          int64_t r = 0, lo = 0;
+          if (mine && own) {
+            lo = -tot.m & ((1ll << 28) - 1);
+            r = (-tot.m >> 28) - (int64_t)((uint64_t)tot.h << 2);
+            if (i == K - 1) r += 1ll << (58 - sa);
+          }
           const int g = 57 - team_max<32>(fx_bits(r));  // the panel's largest below 2^57
-          const Fx2 rs2 = fx_split(fx_scale2(r, g));
+          const Fx2 rs2 = fx_split(fx_scale2(r, g) + (g >= 28 ? lo << (g - 28) : g > 0 ? lo >> (28 - g) : 0));
           const Fx2* t = Tp + 8 * k0 + (i & 7);
           FxAcc u = {0, 0};
-  #pragma unroll
+#pragma unroll
           for (int w = 0; w < kPfW; ++w) {
             Fx2 o;
             o.h = __shfl_sync(kFull, rs2.h, (k0 & 15) + w);
@@ -434,7 +442,7 @@ __global__ void __launch_bounds__(NT, MINB) k_pred_fix(PredArgs A) {
             const int64_t x = fx_val(u);
             int sh = Te[i] - g;
             if (own && fx_bits(x) + sh > 57 && x != 0) {
-              s_bad = 1;
+              if (first) atomicMax(&s_bad, fx_bits(x) + sh - 57);
               sh = 0;
             }
             ui = fx_split(own ? fx_scale2(x, sh) : 0);
@@ -446,15 +454,20 @@ __global__ void __launch_bounds__(NT, MINB) k_pred_fix(PredArgs A) {
           Fx2 c4[4], u4[4];
           load4(M + pf_col(i, K8) + k0 + 4 * half, c4);
           load4(us + k0 + 4 * half, u4);
-  #pragma unroll
-          for (int w = 0; w < 4; ++w) fx_mac(acc, c4[w], u4[w]);
+          int64_t low = 1ll << 29;
+#pragma unroll
+          for (int w = 0; w < 4; ++w) {
+            fx_mac(acc, c4[w], u4[w]);
+            low += (int64_t)c4[w].l * u4[w].l;
+          }
+          acc.m += low >> 30;
         }
       }
       __syncthreads();
-      if (!s_bad || wide) break;
+      if (!s_bad || shift >= kPfShiftMax) break;
+      shift = min(shift + s_bad + 2, kPfShiftMax);
       __syncthreads();
       if (threadIdx.x == 0) s_bad = 0;
-      sa = ive[K - 1] + kPfShift2;
       __syncthreads();
     }
     if (s_bad) {
@@ -463,8 +476,8 @@ __global__ void __launch_bounds__(NT, MINB) k_pred_fix(PredArgs A) {
       break;
     }
 
-    // ---- Sigma = sig^2 C C^T: mean = -(a.r) C_KK, var = sig^2 d_K, the
-    //      column of U a / sig
+    // ---- Sigma = sig^2 C C^T: mean = -(a.r) / a_K, a_K = 1 / C_KK = Y 2^e,
+    //      var = sig^2 d_K, the column of U a / sig
     const double uq = (double)fx_join(ui) * 0x1p-58;
     double sm = 0.0;
     if (!boss && half == 0 && i < k && row < A.nobs && A.resid) sm = uq * A.resid[row];
@@ -474,10 +487,10 @@ __global__ void __launch_bounds__(NT, MINB) k_pred_fix(PredArgs A) {
     __syncthreads();
     sm = 0.0;
     for (int w = 0; 16 * w < K; ++w) sm += s_red[w];
-    const double sc = ldexp(s2, ek), p2 = (double)(1 << sa);
+    const double sc = ldexp(s2, ek), p2 = (double)(1 << (ive[K - 1] + shift));
     if (threadIdx.x == 0) {
-      if (A.mean) A.mean[b] = -sm * p2 * ((double)last[1] * 0x1p-58);
-      if (A.var) A.var[b] = sc * ((double)last[0] * 0x1p-58);
+      if (A.mean) A.mean[b] = -sm * (double)(1 << shift) / ((double)fx_join(ivy[K - 1]) * 0x1p-58);
+      if (A.var) A.var[b] = sc * ((double)*last * 0x1p-58);
     }
     if (A.rhs || A.acol) {
       const double rs1 = p2 / sqrt(sc);
