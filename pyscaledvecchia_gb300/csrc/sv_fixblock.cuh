@@ -146,8 +146,11 @@ __device__ __forceinline__ int64_t fix_factor(int K, int Kw, int tl, Fx2* M, int
         fx_mac(acc[w2], c, b);
       }
     }
+    // nothing left but blocks that are not kept
+    if (__all_sync(kFull, dmin < (1ll << (58 - kFixPivotShift)) || k0 + kFixPanel >= K)) break;
     __syncwarp();
   }
+  __syncwarp();
   return dmin;
 }
 

@@ -260,6 +260,14 @@ __global__ void __launch_bounds__(kFixThreads, 1) k_block_fix(LikArgs A, int wpc
     if (Kw == 0) continue;
     const int d = PI.d, q = PI.q, P = PI.P;
     bool bad = false;  // to the float64 kernels
+    auto leave = [&](bool redo) {
+      if (active && tl == 0) {
+        A.level[b] = 0;
+        A.redo[b] = redo ? 1 : 0;
+        if (redo) A.flags[1] = 1;
+      }
+      __syncwarp();
+    };
     const int ek = PI.fix_ek;
     const bool own = tl < K;
 
@@ -297,6 +305,13 @@ __global__ void __launch_bounds__(kFixThreads, 1) k_block_fix(LikArgs A, int wpc
           }
         }
     }
+    // no work on blocks that are not kept: 100,000 of them beyond 32 ranges,
+    // each computed twice in full, took 13.2 ms where the float64 kernels alone
+    // take 9.2, now 9.5; with pivots below the limit 13.1, now 10.3
+    if (__all_sync(kFull, bad || !active)) {
+      leave(bad);
+      continue;
+    }
     const int es = bad ? 0 : exm - 1023 + 3;  // |u| 2^-es < 1/4
     if (own) *(int64_t*)(S.M + tl * St + tl) = PI.fix_diag;
     __syncwarp();
@@ -314,6 +329,10 @@ __global__ void __launch_bounds__(kFixThreads, 1) k_block_fix(LikArgs A, int wpc
     int64_t cd;
     const int64_t dmin = fix_factor<G>(K, Kw, tl, S.M, cd, E);
     bad |= dmin < (1ll << (58 - kFixPivotShift));
+    if (__all_sync(kFull, bad || !active)) {
+      leave(bad);
+      continue;
+    }
     Fx2 usi;
     bad |= !fix_last_row<G>(K, Kw, tl, S.M, cd, E, S.us, su, usi);
 
@@ -488,12 +507,7 @@ __global__ void __launch_bounds__(kFixThreads, 1) k_block_fix(LikArgs A, int wpc
       }
     }
     const unsigned badm = __ballot_sync(kFull, bad) & (G == 32 ? kFull : 0xffffu << (16 * tm));
-    if (active && tl == 0) {
-      A.level[b] = 0;
-      A.redo[b] = badm ? 1 : 0;
-      if (badm) A.flags[1] = 1;
-    }
-    __syncwarp();
+    leave(badm != 0);
   }
 }
 
