@@ -284,11 +284,15 @@ typedef struct sv_batch_desc {
   int32_t dmax, qmax, kmax, ldnbr;
   int32_t need_grad, any_estimate_nu, chunked, precision, team_lanes;
   int32_t theta_stride, out_stride;
-  int32_t general_nu;   /* 1: some problem has a fixed nu outside {0.5, 1.5, */
-                        /*    2.5} or an estimated nu; the workspace then    */
-                        /*    holds Matern tables per problem (as the        */
+  int32_t general_nu;   /* bit 0: some problem has a fixed nu outside {0.5,  */
+                        /*    1.5, 2.5} or an estimated nu; the workspace    */
+                        /*    then holds Matern tables per problem (as the   */
                         /*    one-problem call builds for such a nu), so     */
                         /*    results match it bit for bit                   */
+                        /* bit 1: no problem has a fixed nu of 1.5 or 2.5,   */
+                        /*    d <= 12 and d + 2 + q <= 32: the kernel for    */
+                        /*    these is not launched (set for one that has,   */
+                        /*    it is evaluated by the general kernels)        */
   double split_rho_min;
   int64_t nblk_max;     /* blocks of the largest problem (sizes the reductions) */
 } sv_batch_desc;

@@ -158,6 +158,10 @@ class BatchedLikelihood:
         # check of the tables)
         self.general_nu = matern_tables and any(
             pr.estimate_nu or float(pr.nu) not in (0.5, 1.5, 2.5) for pr in problems)
+        # whether the float64 form has a problem for its fixed-point kernel
+        self.fixed_point = any(
+            not pr.estimate_nu and float(pr.nu) in (1.5, 2.5) and self.d[i] <= 12 and self.d[i] + 2 + self.q[i] <= 32
+            for i, pr in enumerate(problems))
         self.Pmax = self.dmax + 2 + (1 if self.any_est else 0)
         self.ostride = 1 + self.Pmax + self.Pmax * self.Pmax + self.qmax
 
@@ -255,7 +259,7 @@ class BatchedLikelihood:
             Bd.need_grad, Bd.any_estimate_nu, Bd.chunked = int(self.need_grad), int(self.any_est), int(self.chunked)
             Bd.precision, Bd.team_lanes = _PRECISION[prec], self._lanes[prec]
             Bd.theta_stride, Bd.out_stride = self.Pmax, self.ostride
-            Bd.general_nu = int(self.general_nu)
+            Bd.general_nu = int(self.general_nu) | (0 if self.fixed_point else 2)
             Bd.split_rho_min = self.split_rho_min
             Bd.nblk_max = int(self.nblk.max())
             wsb = max(wsb, int(lib.sv_loglik_batched_workspace_bytes(Bd)))

@@ -1359,8 +1359,11 @@ EvalShape batch_shape(const sv_batch_desc* B) {
   S.need_grad = B->need_grad;
   S.any_est = B->any_estimate_nu;
   S.precision = B->precision;
-  S.tabs = B->general_nu ? 1 : 0;
-  S.fix = 1;  // decided per problem on the device
+  S.tabs = (B->general_nu & 1) ? 1 : 0;
+  // decided per problem on the device; the caller may know that there is none
+  // (64 problems of 300 rows, nu = 1/2: 0.78 ms with the launches in vain, 0.68
+  // without)
+  S.fix = (B->general_nu & 2) ? 0 : 1;
   return S;
 }
 
