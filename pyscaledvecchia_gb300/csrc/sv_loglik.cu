@@ -643,14 +643,17 @@ __host__ __device__ inline int red_parts_n(int64_t nblk) {
   return (int)parts;
 }
 
-// CTAs per partition: a thread-block cluster, its CTAs the partition's blocks
-// in runs, added up through distributed shared memory in CTA order (a
+// A partition's blocks in 8 runs, whose sums are added up in order: by the
+// CTAs of a thread-block cluster, through distributed shared memory (a
 // partition per CTA leaves all but a few SMs idle below 100,000 blocks:
-// n = 5,000 took 90 us in k_reduce1 and 51 us in k_reduce2)
+// n = 5,000 took 90 us in k_reduce1 and 51 us in k_reduce2), or, in a batch with
+// partitions enough to fill the SMs, by the warps of one CTA (64 problems of 300
+// rows: 512 clusters take 109 and 32 us, 512 CTAs 25 and 23; of 3,500: 234 and
+// 124, 150 and 57).  Either way the operations of a sum are the same.
 constexpr int kRedCl = 8;
 constexpr int kRedWide = 4;  // warps of a CTA of k_reduce2 at most
 
-// the blocks [b0, b1) of CTA `rank` of partition `part`
+// the blocks [b0, b1) of run `rank` of partition `part`
 __device__ __forceinline__ void red_range(const ProbInfo& PI, int parts, int part, int rank, int64_t& b0,
                                           int64_t& b1) {
   const int64_t per = (PI.nblk + parts - 1) / parts;
@@ -660,6 +663,20 @@ __device__ __forceinline__ void red_range(const ProbInfo& PI, int parts, int par
   b0 = min(p1, p0 + rank * run);
   b1 = min(p1, b0 + run);
 }
+
+// pass-1 field f of the block with record c and log L_KK lgj
+__device__ __forceinline__ double red1_field(const double* c, int q, int foff, int f, double lgj) {
+  if (f == 0) return lgj;
+  if (f < 1 + q) return c[2 + (f - 1)] * c[1];
+  if (f < 1 + q + q * q) {
+    const int e = f - 1 - q;
+    const int i = e / q, jj = e - (e / q) * q;
+    return c[2 + i] * c[2 + jj];
+  }
+  return c[foff + (f - 1 - q - q * q)];
+}
+constexpr int kRedFr = 4;  // fields of a lane in registers
+constexpr int kRb = 4;     // blocks whose fields are loaded before they are added
 
 __global__ void __cluster_dims__(kRedCl, 1, 1) k_reduce1(RedArgs R) {
   extern __shared__ double racc[];  // [nwarp][nfmax]
@@ -677,24 +694,13 @@ __global__ void __cluster_dims__(kRedCl, 1, 1) k_reduce1(RedArgs R) {
   int64_t b0, b1;
   red_range(PI, parts, part, rank, b0, b1);
   double* acc = racc + (int64_t)w * R.nfmax;
-  const int foff = 3 + 2 * q + P * (2 + q);
   // the (warp, field) sums, one owner lane each: fields lane + 32 r < 128 in
   // registers a[r], the rest (large d) in shared memory
-  constexpr int kFr = 4;
-  double a[kFr];
+  double a[kRedFr];
 #pragma unroll
-  for (int r = 0; r < kFr; ++r) a[r] = 0.0;
-  for (int f = lane + 32 * kFr; f < nf; f += 32) acc[f] = 0.0;
-  auto field = [&](const double* c, int f, double lgj) -> double {
-    if (f == 0) return lgj;
-    if (f < 1 + q) return c[2 + (f - 1)] * c[1];
-    if (f < 1 + q + q * q) {
-      const int e = f - 1 - q;
-      const int i = e / q, jj = e - (e / q) * q;
-      return c[2 + i] * c[2 + jj];
-    }
-    return c[foff + (f - 1 - q - q * q)];
-  };
+  for (int r = 0; r < kRedFr; ++r) a[r] = 0.0;
+  for (int f = lane + 32 * kRedFr; f < nf; f += 32) acc[f] = 0.0;
+  const int foff = 3 + 2 * q + P * (2 + q);
   for (int64_t base = b0 + w; base < b1; base += 32 * (int64_t)nwarp) {
     // log L_KK of the warp's next 32 blocks, one per lane (a float64 warp
     // instruction costs the same with one lane as with 32)
@@ -703,35 +709,34 @@ __global__ void __cluster_dims__(kRedCl, 1, 1) k_reduce1(RedArgs R) {
     const int nj = (int)min((int64_t)32, (b1 - base + nwarp - 1) / nwarp);
     // kRb blocks' register fields are loaded before they are added (in
     // block order, so the sums are those of one block at a time)
-    constexpr int kRb = 4;
     for (int j0 = 0; j0 < nj; j0 += kRb) {
-      double v[kRb][kFr];
+      double v[kRb][kRedFr];
 #pragma unroll
       for (int u = 0; u < kRb; ++u) {
         const int j = j0 + u < nj ? j0 + u : nj - 1;
         const double lgj = __shfl_sync(0xffffffffu, lg, j);
         const double* c = R.cache + (base + (int64_t)j * nwarp) * R.CS;
 #pragma unroll
-        for (int r = 0; r < kFr; ++r) {
+        for (int r = 0; r < kRedFr; ++r) {
           const int f = lane + 32 * r;
-          v[u][r] = f < nf ? field(c, f, lgj) : 0.0;
+          v[u][r] = f < nf ? red1_field(c, q, foff, f, lgj) : 0.0;
         }
       }
 #pragma unroll
       for (int u = 0; u < kRb; ++u) {
         if (j0 + u >= nj) break;
 #pragma unroll
-        for (int r = 0; r < kFr; ++r)
+        for (int r = 0; r < kRedFr; ++r)
           if (lane + 32 * r < nf) a[r] += v[u][r];
         const int j = j0 + u;
         const double lgj = __shfl_sync(0xffffffffu, lg, j);
         const double* c = R.cache + (base + (int64_t)j * nwarp) * R.CS;
-        for (int f = lane + 32 * kFr; f < nf; f += 32) acc[f] += field(c, f, lgj);
+        for (int f = lane + 32 * kRedFr; f < nf; f += 32) acc[f] += red1_field(c, q, foff, f, lgj);
       }
     }
   }
 #pragma unroll
-  for (int r = 0; r < kFr; ++r)
+  for (int r = 0; r < kRedFr; ++r)
     if (lane + 32 * r < nf) acc[lane + 32 * r] = a[r];
   __syncthreads();
   for (int f = threadIdx.x; f < nf; f += blockDim.x) {
@@ -752,7 +757,99 @@ __global__ void __cluster_dims__(kRedCl, 1, 1) k_reduce1(RedArgs R) {
   cl.sync();  // the others' shared memory stays until it has been read
 }
 
-constexpr int kFinSl = 8;  // slices of the partitions summed side by side
+// The same with a warp per run, which takes the parts of the cluster form's
+// eight warps one after the other (at most 32 kRedFr fields)
+__global__ void __launch_bounds__(kRedThreads) k_reduce1_cta(RedArgs R) {
+  static_assert(kRedThreads == 32 * kRedCl && kRb * (kRedThreads / 32) == 32, "a warp per run, of up to 128 blocks");
+  extern __shared__ double racc[];  // [kRedCl][nfmax]
+  const int p = blockIdx.y;
+  const ProbInfo& PI = R.probs[p];
+  if (PI.skip) return;
+  const int q = PI.q, P = PI.P;
+  const int nf = nfield1(q, P, R.need_grad);
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int parts = red_parts_n(PI.nblk);
+  const int part = R.pbeg + (int)blockIdx.x;
+  if (part >= parts) return;
+  int64_t b0, b1;
+  red_range(PI, parts, part, w, b0, b1);
+  const int foff = 3 + 2 * q + P * (2 + q);
+  double lg[kRedWide];  // the run's log L_KK, one per lane
+#pragma unroll
+  for (int c = 0; c < kRedWide; ++c) {
+    const int64_t b = b0 + 32 * c + lane;
+    lg[c] = b < b1 ? log(R.cache[b * R.CS]) : 0.0;
+  }
+  double s[kRedFr];
+#pragma unroll
+  for (int r = 0; r < kRedFr; ++r) s[r] = 0.0;
+  constexpr int kW = kRedThreads / 32;
+  // the fields of the run's blocks first + stride u, u < min(kRb, left)
+  auto load = [&](double (&v)[kRb][kRedFr], double lgc, int first, int stride, int left) {
+#pragma unroll
+    for (int u = 0; u < kRb; ++u) {
+      const int at = first + stride * min(u, left - 1);
+      const double lgj = __shfl_sync(0xffffffffu, lgc, at & 31);
+      const double* rec = R.cache + (b0 + at) * R.CS;
+#pragma unroll
+      for (int r = 0; r < kRedFr; ++r) {
+        const int f = lane + 32 * r;
+        v[u][r] = f < nf ? red1_field(rec, q, foff, f, lgj) : 0.0;
+      }
+    }
+  };
+  const int len = (int)(b1 - b0);
+  if (len <= kW) {  // a block each
+    for (int k = 0; k < len; k += kRb) {
+      double v[kRb][kRedFr];
+      load(v, lg[0], k, 1, len - k);
+#pragma unroll
+      for (int u = 0; u < kRb; ++u)
+        if (k + u < len) {
+#pragma unroll
+          for (int r = 0; r < kRedFr; ++r)
+            if (32 * r < nf) s[r] += v[u][r];
+        }
+    }
+  } else {
+    for (int k = 0; k < kW; ++k) {
+      double a[kRedFr];
+#pragma unroll
+      for (int r = 0; r < kRedFr; ++r) a[r] = 0.0;
+      const int nj = (len - k + kW - 1) / kW;
+#pragma unroll
+      for (int c = 0; c < kRedWide; ++c) {  // (32 blocks of the run, kRb of them this part's)
+        if (kRb * c >= nj) break;
+        double v[kRb][kRedFr];
+        load(v, lg[c], 32 * c + k, kW, nj - kRb * c);
+#pragma unroll
+        for (int u = 0; u < kRb; ++u)
+          if (kRb * c + u < nj) {
+#pragma unroll
+            for (int r = 0; r < kRedFr; ++r)
+              if (32 * r < nf) a[r] += v[u][r];
+          }
+      }
+#pragma unroll
+      for (int r = 0; r < kRedFr; ++r)
+        if (32 * r < nf) s[r] += a[r];
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < kRedFr; ++r)
+    if (lane + 32 * r < nf) racc[w * R.nfmax + lane + 32 * r] = s[r];
+  __syncthreads();
+  double* partv = R.part1 + ((int64_t)p * R.parts + part) * R.nfmax;
+  for (int f = threadIdx.x; f < nf; f += blockDim.x) {
+    double t = 0.0;
+#pragma unroll
+    for (int c = 0; c < kRedCl; ++c) t += racc[c * R.nfmax + f];
+    partv[f] = t;
+  }
+}
+
+constexpr int kFinSl = 8;  // slices of the partitions summed side by side,
+constexpr int kFinThreads = 1024;  // for up to 128 fields at a time
 
 __global__ void k_final1(RedArgs R) {
   const int p = blockIdx.x;
@@ -763,8 +860,8 @@ __global__ void k_final1(RedArgs R) {
   double* sums = R.sums + (int64_t)p * R.nfmax;
   const int parts = red_parts_n(PI.nblk);
   // kFinSl slices of the partitions side by side, added in slice order
-  __shared__ double sl[kFinSl][kRedThreads / kFinSl];
-  constexpr int kF = kRedThreads / kFinSl;
+  __shared__ double sl[kFinSl][kFinThreads / kFinSl];
+  const int kF = blockDim.x / kFinSl;
   const int ps = (parts + kFinSl - 1) / kFinSl;
   for (int f0 = 0; f0 < nf; f0 += kF) {
     const int f = f0 + threadIdx.x % kF, z = threadIdx.x / kF;
@@ -816,25 +913,56 @@ __global__ void k_final1(RedArgs R) {
 }
 
 // Pass-2 sums of one partition: z_K^2 and the score terms, a thread per block.
-// A lane's blocks are every 32nd of the CTA's run, in order, then the lanes
+// A lane's blocks are every 32nd of the run, in order, then the lanes
 // are added up: by one warp, or with a warp for each of up to kRedWide blocks
 // of a lane, whose terms then meet in the same order.  The width depends on
 // the launch's largest problem, so the bits must not depend on the width, nor
 // on PR (every operation is written out).  PR: parameters whose sums are held
-// in registers (a runtime count puts them into local memory: 131 us instead of
-// 111 at 200,000 blocks, before the lanes' sums were shared)
+// in registers at a time (a runtime count puts them into local memory: 131 us
+// instead of 111 at 200,000 blocks, before the lanes' sums were shared; room
+// for all 66 takes 252 registers: 217 us at d = 20 and 200,000 blocks, 16 at a time 113)
+template <int PR>
+__device__ __forceinline__ void red2_sum(const RedArgs& R, int q, int P, int p0, const double* sbeta, int64_t b,
+                                         int64_t b1, int step, double (&acc)[PR + 1]) {
+#pragma unroll
+  for (int i = 0; i <= PR; ++i) acc[i] = 0.0;
+  for (; b < b1; b += step) {
+    const double* c = R.cache + b * R.CS;
+    double zK = c[2 + q];
+    for (int i = 0; i < q; ++i) zK = fma(-c[3 + q + i], sbeta[i], zK);
+    const double zz = __dmul_rn(zK, zK), z1 = __dadd_rn(1.0, zz), z2 = -2.0 * zK;
+    acc[0] = __dadd_rn(acc[0], zz);
+    if (R.need_grad) {
+      const double* wK = c + 3 + 2 * q + p0;
+      const double* wzy = wK + P;
+      const double* wzZ = c + 3 + 2 * q + 2 * P + p0 * q;
+#pragma unroll
+      for (int pp = 0; pp < PR; ++pp)
+        if (p0 + pp < P) {
+          double wz = wzy[pp];
+          for (int i = 0; i < q; ++i) wz = fma(-wzZ[pp * q + i], sbeta[i], wz);
+          acc[1 + pp] = fma(-0.5, fma(z2, wz, __dmul_rn(wK[pp], z1)), acc[1 + pp]);
+        }
+    }
+  }
+}
+// the sum over the lanes, of which those from 2 o on hold 0
+__device__ __forceinline__ double red2_lanes(double v, int o = 16) {
+  for (; o > 0; o >>= 1) v = __dadd_rn(v, __shfl_down_sync(0xffffffffu, v, o));
+  return v;
+}
+
 template <int PR>
 __global__ void __cluster_dims__(kRedCl, 1, 1) k_reduce2(RedArgs R) {
   cg::cluster_group cl = cg::this_cluster();
   const int rank = (int)cl.block_rank();
   __shared__ double sbeta[kMaxQ];
   __shared__ double tot[kMaxP + 1];
-  constexpr bool kWide = PR <= 16;  // (what the shared memory holds)
-  __shared__ double red[kWide ? kRedWide : 1][kWide ? PR + 1 : 1][32];
+  __shared__ double red[kRedWide][PR + 1][32];
   const int p = blockIdx.y;
   const ProbInfo& PI = R.probs[p];
   if (PI.skip) return;
-  const int q = PI.q, P = PI.P, np = R.need_grad ? P : 0;
+  const int P = PI.P, q = PI.q, np = R.need_grad ? P : 0;
   for (int i = threadIdx.x; i < q; i += blockDim.x) sbeta[i] = R.beta[(int64_t)p * (R.qmax + 1) + i];
   __syncthreads();
   const int parts = red_parts_n(PI.nblk);
@@ -842,46 +970,31 @@ __global__ void __cluster_dims__(kRedCl, 1, 1) k_reduce2(RedArgs R) {
   if (part >= parts) return;
   int64_t b0, b1;
   red_range(PI, parts, part, rank, b0, b1);
-  double acc[PR + 1];
-#pragma unroll
-  for (int i = 0; i <= PR; ++i) acc[i] = 0.0;
-  for (int64_t b = b0 + threadIdx.x; b < b1; b += blockDim.x) {
-    const double* c = R.cache + b * R.CS;
-    double zK = c[2 + q];
-    for (int i = 0; i < q; ++i) zK = fma(-c[3 + q + i], sbeta[i], zK);
-    const double zz = __dmul_rn(zK, zK), z1 = __dadd_rn(1.0, zz), z2 = -2.0 * zK;
-    acc[0] = __dadd_rn(acc[0], zz);
-    if (R.need_grad) {
-      const double* wK = c + 3 + 2 * q;
-      const double* wzy = wK + P;
-      const double* wzZ = wzy + P;
-#pragma unroll
-      for (int pp = 0; pp < PR; ++pp)
-        if (pp < P) {
-          double wz = wzy[pp];
-          for (int i = 0; i < q; ++i) wz = fma(-wzZ[pp * q + i], sbeta[i], wz);
-          acc[1 + pp] = fma(-0.5, fma(z2, wz, __dmul_rn(wK[pp], z1)), acc[1 + pp]);
-        }
-    }
-  }
   const int w = threadIdx.x >> 5, nw = blockDim.x >> 5, ln = threadIdx.x & 31;
-  auto lanes = [&](double v, int i) {
-    for (int o = 16; o > 0; o >>= 1) v = __dadd_rn(v, __shfl_down_sync(0xffffffffu, v, o));
-    if (ln == 0) tot[i] = v;
-  };
-  if (!kWide || nw == 1) {
+  for (int p0 = 0; p0 == 0 || p0 < np; p0 += PR) {
+    double acc[PR + 1];
+    red2_sum<PR>(R, q, P, p0, sbeta, b0 + threadIdx.x, b1, blockDim.x, acc);
+    // acc[1 + t] is parameter p0 + t, acc[0] the sum of z_K^2 (first time)
+    const int i0 = p0 ? 1 : 0, i1 = min(PR, np - p0);
+    if (nw == 1) {
 #pragma unroll
-    for (int i = 0; i <= PR; ++i)
-      if (i <= np) lanes(acc[i], i);
-  } else if constexpr (kWide) {
+      for (int i = 0; i <= PR; ++i)
+        if (i >= i0 && i <= i1) {
+          const double v = red2_lanes(acc[i]);
+          if (ln == 0) tot[p0 + i] = v;
+        }
+    } else {
+      if (p0) __syncthreads();
 #pragma unroll
-    for (int i = 0; i <= PR; ++i)
-      if (i <= np) red[w][i][ln] = acc[i];
-    __syncthreads();
-    for (int i = w; i <= np; i += nw) {
-      double v = red[0][i][ln];
-      for (int k = 1; k < nw; ++k) v = __dadd_rn(v, red[k][i][ln]);
-      lanes(v, i);
+      for (int i = 0; i <= PR; ++i)
+        if (i >= i0 && i <= i1) red[w][i][ln] = acc[i];
+      __syncthreads();
+      for (int i = i0 + w; i <= i1; i += nw) {
+        double v = red[0][i][ln];
+        for (int k = 1; k < nw; ++k) v = __dadd_rn(v, red[k][i][ln]);
+        v = red2_lanes(v);
+        if (ln == 0) tot[p0 + i] = v;
+      }
     }
   }
   cl.sync();
@@ -893,6 +1006,41 @@ __global__ void __cluster_dims__(kRedCl, 1, 1) k_reduce2(RedArgs R) {
       R.part2[((int64_t)p * R.parts + part) * (R.Pmax + 1) + i] = s;
     }
   cl.sync();  // the others' shared memory stays until it has been read
+}
+
+// The same with a warp per run
+template <int PR>
+__global__ void __launch_bounds__(kRedThreads) k_reduce2_cta(RedArgs R) {
+  __shared__ double sbeta[kMaxQ];
+  __shared__ double tot[kRedCl][PR + 1];
+  const int p = blockIdx.y;
+  const ProbInfo& PI = R.probs[p];
+  if (PI.skip) return;
+  const int P = PI.P, q = PI.q, np = R.need_grad ? P : 0;
+  for (int i = threadIdx.x; i < q; i += blockDim.x) sbeta[i] = R.beta[(int64_t)p * (R.qmax + 1) + i];
+  __syncthreads();
+  const int parts = red_parts_n(PI.nblk);
+  const int part = R.pbeg + (int)blockIdx.x;
+  if (part >= parts) return;
+  const int w = threadIdx.x >> 5, ln = threadIdx.x & 31;
+  int64_t b0, b1;
+  red_range(PI, parts, part, w, b0, b1);
+  double acc[PR + 1];
+  red2_sum<PR>(R, q, P, 0, sbeta, b0 + ln, b1, 32, acc);
+  const int o = b1 - b0 > 16 ? 16 : b1 - b0 > 8 ? 8 : 4;
+#pragma unroll
+  for (int i = 0; i <= PR; ++i)
+    if (i <= np) {
+      const double v = red2_lanes(acc[i], o);
+      if (ln == 0) tot[w][i] = v;
+    }
+  __syncthreads();
+  for (int i = threadIdx.x; i <= np; i += blockDim.x) {
+    double s = 0.0;
+#pragma unroll
+    for (int c = 0; c < kRedCl; ++c) s += tot[c][i];
+    R.part2[((int64_t)p * R.parts + part) * (R.Pmax + 1) + i] = s;
+  }
 }
 
 __global__ void k_final2(RedArgs R) {
@@ -1283,34 +1431,37 @@ int run_eval(const EvalCall& C, cudaStream_t st, const ShardStage* sh = nullptr)
   R.parts = parts;
   R.pbeg = sh ? sh->pb : 0;
   const int npart = sh ? sh->pe - sh->pb : parts;
-  const dim3 rgrid((unsigned)(npart > 0 ? npart * kRedCl : 1), (unsigned)S.nprob);
+  // a batch's partitions, two to an SM at least
+  const bool cta = S.nprob > 1 && S.Pmax <= 16 && W.nfmax <= 32 * kRedFr &&
+                   (int64_t)npart * S.nprob >= 2LL * sv_num_sms() && S.nblk_max <= 4096 * 1024;
+  const dim3 rgrid((unsigned)(npart > 0 ? npart * (cta ? 1 : kRedCl) : 1), (unsigned)S.nprob);
   if (stage == 0 || stage == 2) {
     int rwarps = kRedThreads / 32;
     while (rwarps > 1 && sizeof(double) * (size_t)rwarps * W.nfmax > (size_t)max_smem_optin()) --rwarps;
     const size_t rsmem = sizeof(double) * (size_t)rwarps * W.nfmax;
     if (rsmem > (size_t)max_smem_optin()) return SV_EINVAL;
     if (npart > 0) {
-      SV_CUDA_TRY(cudaFuncSetAttribute(k_reduce1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsmem));
-      k_reduce1<<<rgrid, 32 * rwarps, rsmem, st>>>(R);
+      auto kern = cta ? k_reduce1_cta : k_reduce1;
+      SV_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsmem));
+      kern<<<rgrid, 32 * rwarps, rsmem, st>>>(R);
       SV_CUDA_TRY(cudaGetLastError());
     }
   }
   if (stage == 0 || stage == 3) {
-    k_final1<<<(unsigned)S.nprob, kRedThreads, 0, st>>>(R);
+    const int fthr = std::min(kFinThreads, kFinSl * ((W.nfmax + 31) / 32 * 32));
+    k_final1<<<(unsigned)S.nprob, fthr, 0, st>>>(R);
     SV_CUDA_TRY(cudaGetLastError());
     if (npart > 0) {
       // a thread per block of a CTA's run (at most 128 blocks; beyond 8,192
       // blocks they have 114 to 128): one warp with four blocks a thread took
-      // 150 us at 200,000 blocks, this 55 (a CTA of 256 per partition 79)
+      // 150 us at 200,000 blocks (d = 20: 250), this 55 (113; a CTA of 256 per
+      // partition 79, 114)
       const int64_t run = S.nblk_max > 8192 ? 128 : (S.nblk_max + 8 * kRedCl - 1) / (8 * kRedCl);
-      const bool wide = S.nblk_max <= 4096 * 1024 && S.Pmax <= 16;
-      const int thr = wide ? std::max(32, (int)((run + 31) / 32 * 32)) : 32;
-      if (S.Pmax <= 8)
-        k_reduce2<8><<<rgrid, thr, 0, st>>>(R);
-      else if (S.Pmax <= 16)
-        k_reduce2<16><<<rgrid, thr, 0, st>>>(R);
-      else
-        k_reduce2<kMaxP><<<rgrid, thr, 0, st>>>(R);
+      const bool wide = S.nblk_max <= 4096 * 1024;
+      const int thr = cta ? kRedThreads : wide ? std::max(32, (int)((run + 31) / 32 * 32)) : 32;
+      auto kern = cta ? (S.Pmax <= 8 ? k_reduce2_cta<8> : k_reduce2_cta<16>)
+                      : S.Pmax <= 8 ? k_reduce2<8> : k_reduce2<16>;
+      kern<<<rgrid, thr, 0, st>>>(R);
       SV_CUDA_TRY(cudaGetLastError());
     }
   }
