@@ -102,7 +102,16 @@ struct KnnArgs {
   int64_t b0;
   int ldnbr;
   int wq_cap, wq_sort;  // large k: superset capacity and sort width per warp
+  // the choice between tree and screens, made on the device: tiles that sampled
+  // queries would visit, and all; null where there is none
+  const unsigned* sel;
+  unsigned sel_max;     // the tree where at most sel_max / 256 of them are visited
+  int sel_tree;         // the launch belongs to that choice (else to the other)
 };
+
+__device__ __forceinline__ bool kt_left_out(const KnnArgs& A) {
+  return A.sel && (256ull * A.sel[0] <= (unsigned long long)A.sel_max * A.sel[1]) != (A.sel_tree != 0);
+}
 
 __device__ __forceinline__ float knn_thr(double s64k, float Bi, int d) {
   const double t = (sqrt(s64k) * (1.0 + (double)(d + 4) * 0x1p-53) + (double)Bi) * (1.0 + 0x1p-40);
@@ -241,6 +250,7 @@ __device__ __forceinline__ void knn_tile(const KnnArgs& A, int64_t qt, unsigned 
 template <int DP>
 __global__ void __launch_bounds__(kKnnQ) k_knn(KnnArgs A) {
   extern __shared__ unsigned char smraw[];
+  if (kt_left_out(A)) return;
   const int64_t ntile = (A.nq + kKnnQ - 1) / kKnnQ;
   // largest tiles first (ordered search work grows with the row index)
   const int64_t qt = A.ordered ? (ntile - 1 - blockIdx.x) : blockIdx.x;
@@ -550,6 +560,7 @@ __device__ __forceinline__ void knn_wq_tile(const KnnArgs& A, int64_t qt, unsign
 template <int DP>
 __global__ void __launch_bounds__(256) k_knn_wq(KnnArgs A) {
   extern __shared__ __align__(16) unsigned char smraw[];
+  if (kt_left_out(A)) return;
   const int nw = blockDim.x >> 5;
   const int64_t ntile = (A.nq + nw - 1) / nw;
   // ordered searches: largest rows first (their work grows with the row index)
@@ -691,9 +702,67 @@ __device__ __forceinline__ float kt_box2(const float (&qv)[DP], const float* lo,
   return s;
 }
 
+// How much of the tree an ordered search would visit: for kKtSamples rows, the
+// k-th smallest distance to the earlier rows of their own super-tile bounds the
+// search's; out[0] += the tiles within it, out[1] += the row's share of all.
+constexpr int kKtSamples = 128;
+template <int DP>
+__global__ void __launch_bounds__(256) k_kt_sample(KnnTree R, int k, unsigned* out) {
+  const int64_t pos = (2 * (int64_t)blockIdx.x + 1) * R.n / (2 * kKtSamples);
+  const int i = R.id[pos];
+  float qv[DP];
+#pragma unroll
+  for (int l = 0; l < DP; ++l) qv[l] = R.v[pos * DP + l];
+  const int64_t home = (((pos + 1) * R.ntile - 1) / R.n) / kKtSuper;
+  const int64_t p0 = home * kKtSuper * R.n / R.ntile, p1 = (home + 1) * kKtSuper * R.n / R.ntile;
+  constexpr int kPer = kKtTile * kKtSuper / 256;
+  unsigned key[kPer];  // of the distances, as bits; all ones: no such row
+#pragma unroll
+  for (int e = 0; e < kPer; ++e) {
+    const int64_t p = p0 + threadIdx.x + 256 * e;
+    key[e] = 0xffffffffu;
+    if (p < p1 && R.id[p] < i) {
+      float s = 0.0f;
+#pragma unroll
+      for (int l = 0; l < DP; ++l) {
+        const float df = qv[l] - R.v[p * DP + l];
+        s = fmaf(df, df, s);
+      }
+      key[e] = __float_as_uint(s);
+    }
+  }
+  unsigned kth = 0;  // the smallest bits that at least k keys do not exceed
+  for (int bit = 31; bit >= 0; --bit) {
+    const unsigned mid = kth + (1u << bit) - 1;
+    int below = 0;
+#pragma unroll
+    for (int e = 0; e < kPer; ++e) below += key[e] <= mid ? 1 : 0;
+    int n = __reduce_add_sync(0xffffffffu, below);
+    __shared__ int s_n[2];
+    if (threadIdx.x < 2 && bit == 31) s_n[threadIdx.x] = 0;
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) atomicAdd(&s_n[bit & 1], n);
+    __syncthreads();
+    n = s_n[bit & 1];
+    if (threadIdx.x == 0) s_n[(bit & 1) ^ 1] = 0;
+    if (n < k) kth += 1u << bit;
+  }
+  const float B = R.B[pos];
+  const float T = kth >= 0x7f800000u ? __int_as_float(0x7f800000) : sqrtf(__uint_as_float(kth)) + 3.0f * B;
+  int vis = 0;
+  for (int t = threadIdx.x; t < R.ntile; t += blockDim.x) {
+    const float tb = T + R.tB[t];
+    if (R.tmin[t] < i && !(kt_box2<DP>(qv, R.lo + (int64_t)t * DP, R.hi + (int64_t)t * DP) > tb * tb)) ++vis;
+  }
+  vis = __reduce_add_sync(0xffffffffu, vis);
+  if ((threadIdx.x & 31) == 0) atomicAdd(out, (unsigned)vis);
+  if (threadIdx.x == 0) atomicAdd(out + 1, (unsigned)((int64_t)i * R.ntile / R.n));
+}
+
 template <int DP>
 __global__ void __launch_bounds__(256) k_knn_tree(KnnArgs A, KnnTree R) {
   extern __shared__ __align__(16) unsigned char smraw[];
+  if (kt_left_out(A)) return;
   const int nw = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned full = 0xffffffffu;
   WqSmem S;
@@ -928,8 +997,7 @@ static int launch_knn(const KnnArgs& A, int DP, int64_t grid, size_t smem, cudaS
 // ---- tree search: scratch, build and launch
 static size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// rows from which the tree search is taken (below, the screens of all rows
-// take less than building the tree)
+// rows from which a tree is built (below, the screens of all rows take less)
 constexpr int64_t kKtMinRows = 16384;
 
 static int kt_levels(int64_t n) {
@@ -937,21 +1005,54 @@ static int kt_levels(int64_t n) {
   while (((n + ((int64_t)1 << L) - 1) >> L) > kKtTile) ++L;
   return L;
 }
-// and the queries from which it is, for smaller sets: the screens take one pass
-// over the rows while every query has a warp of its own (16 to an SM). Measured
-// at d = 6, k = 140: 1,500 queries of 60,000 rows 1.33 ms by the tree, 1.36 by
-// the screens (of 30,000: 1.04, 0.85), 4,000 queries 1.35, 2.60 (1.11, 1.60);
-// 50 of 100,000 1.45, 1.81. 200,000 ordered rows, d = 10, m = 30: 8.4, 134 ms;
-// 20,000 queries of 100,000: 2.2, 15.8 ms; no slower where every input counts
-// (100,000 ordered rows, d = 10, no range above 0.1: 25.7, 55 ms)
-static bool kt_use(int k, int64_t n, int64_t nq, int DP) {
-  return n >= kKtMinRows && n <= 0x7fffffffLL && (n >= 65536 || nq > 16LL * sv_num_sms()) &&
-         wq_plan(k, DP, nullptr, nullptr);
+// Which search a call takes.  The tree's cost follows the rows it visits, and
+// those the number of inputs that matter, which only the data tell.  Measured
+// over evenly spread rows with the same range in every input, its worst case
+// (screens / tree, ms; with ranges from 0.05 to 50 the tree is 1.5 to 20 times
+// faster at every size and d):
+//   ordered, 20,000 rows: m = 5, d = 10 4.8 / 4.6, d = 12 5.1 / 5.7; m = 30, d = 8
+//     2.3 / 2.7, d = 10 2.6 / 4.1
+//   40,000, m = 30: d = 8 7.3 / 5.3, d = 10 8.3 / 9.9
+//   200,000: m = 5, d = 9 39 / 32, d = 10 39 / 47, d = 16 51 / 254; m = 30, d = 9
+//     122 / 59, d = 12 134 / 159, d = 16 162 / 279
+//   queries, k = 140: 2,400 of 100,000 rows, d = 4 as long, d = 8 to 16 by the tree
+//     1.4 to 1.8 times longer; 2,500 of 65,535 rows 1.1 to 1.7 times shorter, 20,000
+//     of 16,384 1.35 to 2.8 times
+// So up to 8 to 10 inputs the tree is taken as it is, beyond that an ordered
+// search of 32,768 rows and more builds it, and samples decide (1 to 1.5 ms when
+// they are against it); smaller ones keep the screens.
+enum KtUse { kKtNo, kKtYes, kKtAsk };
+
+// kKtAsk: build the tree, and let the sampled rows tell (k_kt_sample).
+// sel_max: visited share, of 256, up to which the tree is faster then
+static KtUse kt_ordered(int m, int64_t n, int64_t nq, int d, unsigned* sel_max) {
+  const int DP = pad_dim(d);
+  if (m < 1 || n < kKtMinRows || n > 0x7fffffffLL || !wq_plan(m, DP, nullptr, nullptr)) return kKtNo;
+  const bool wq = use_wq(m, n, DP);
+  if (nq <= 16LL * sv_num_sms() && (wq || n < 65536)) return kKtNo;  // (as for queries)
+  if (n < 32768) return d <= (wq ? 8 : 10) ? kKtYes : kKtNo;
+  if (d <= (wq ? 8 : 9)) return kKtYes;
+  // a warp's screens cost what visits to 0.7 to 1 times the earlier rows do (an estimate: the
+  // samples' bounds are wide), a thread's what some 12,000 to 60,000 rows' do, whatever
+  // n is, most of it insertions
+  *sel_max = wq ? (n < 50000 ? 180 : n < 150000 ? 256 : 192)
+                : (unsigned)min((int64_t)256, 512 * (6000 + 900 * (int64_t)m + 32 * (int64_t)m * m) / n);
+  return kKtAsk;
+}
+
+static bool kt_query(int k, int64_t n, int64_t nq, int d) {
+  const int DP = pad_dim(d);
+  if (n < kKtMinRows || n > 0x7fffffffLL || !wq_plan(k, DP, nullptr, nullptr)) return false;
+  const int64_t waves = (nq + 16LL * sv_num_sms() - 1) / (16LL * sv_num_sms());
+  // a thread per query: slower than the tree from 65,536 rows or a wave on
+  if (!use_wq(k, n, DP)) return n >= 65536 || waves > 1;
+  // a warp per query passes over all rows once per wave of 16 warps an SM
+  return waves * n >= (waves > 1 && d <= 6 ? 50000 : 100000) && (waves > 1 || d <= 6);
 }
 static size_t kt_bytes(int64_t n, int d, int DP) {
   if (n < kKtMinRows || DP > 16) return 0;
   const size_t S = (size_t)1 << kt_levels(n), N = (size_t)n;
-  return 2 * al256(8 * N) + 2 * al256(4 * N) + 2 * al256(4 * S * d) + al256(kd_sort_reserve(n)) +
+  return 256 + 2 * al256(8 * N) + 2 * al256(4 * N) + 2 * al256(4 * S * d) + al256(kd_sort_reserve(n)) +
          al256(4 * N * DP) + al256(4 * N) + 2 * al256(4 * S * DP) + 2 * al256(4 * S) +
          2 * al256(4 * (S / kKtSuper) * DP) + 2 * al256(4 * (S / kKtSuper));
 }
@@ -969,6 +1070,7 @@ static int kt_run(const KnnArgs& A0, int warps, char* ws, cudaStream_t st) {
     ws += al256(bytes);
     return p;
   };
+  unsigned* sel = (unsigned*)take(256);
   unsigned long long* keys0 = (unsigned long long*)take(8 * (size_t)n);
   unsigned long long* keys1 = (unsigned long long*)take(8 * (size_t)n);
   int* ids0 = (int*)take(4 * (size_t)n);
@@ -1003,6 +1105,13 @@ static int kt_run(const KnnArgs& A0, int warps, char* ws, cudaStream_t st) {
   SV_CUDA_TRY(cudaGetLastError());
   KnnTree R = {v, B, ids, lo, hi, tB, tmin, slo, shi, sB, smin, n, S, ns};
   KnnArgs A = A0;
+  if (A.sel_max) {
+    SV_CUDA_TRY(cudaMemsetAsync(sel, 0, 8, st));
+    k_kt_sample<DP><<<kKtSamples, 256, 0, st>>>(R, A.k, sel);
+    SV_CUDA_TRY(cudaGetLastError());
+    A.sel = sel;
+    A.sel_tree = 1;
+  }
   A.wq_cap = kt_cap(A.k);
   A.wq_sort = wq_sort(A.wq_cap);
   size_t smem = 0;
@@ -1192,14 +1301,24 @@ extern "C" int sv_ordered_knn(const double* X, int64_t n, int32_t d, int32_t m, 
   A.nbr = nullptr;
   A.b0 = 0;
   A.ldnbr = 0;
-  const bool tree = m > 0 && kt_use(m, n, n - A.start, DP);
-  if (tree) {
+  A.sel = nullptr;
+  A.sel_max = 0;
+  A.sel_tree = 0;
+  const KtUse use = kt_ordered(m, n, n - A.start, d, &A.sel_max);
+  if (use != kKtNo) {
+    char* tws = (char*)B + al256(sizeof(float) * (size_t)n);
+    int rc = launch_knn_tree(A, DP, tws, st);
+    if (rc != SV_OK) return rc;
+    if (use == kKtAsk) {  // (the samples' sums are first in the tree's scratch)
+      A.sel = (const unsigned*)tws;
+      A.sel_tree = 1;
+    }
     // the first rows have few earlier ones, spread over all of the tree
     A.nq = A.nr = kKtHead;
-    const int rc = launch_knn(A, DP, (kKtHead + kKnnQ - 1) / kKnnQ, smem, st);
-    if (rc != SV_OK) return rc;
+    rc = launch_knn(A, DP, (kKtHead + kKnnQ - 1) / kKnnQ, smem, st);
+    if (rc != SV_OK || use == kKtYes) return rc;
     A.nq = A.nr = n;
-    return launch_knn_tree(A, DP, (char*)B + al256(sizeof(float) * (size_t)n), st);
+    A.sel_tree = 0;
   }
   const int64_t ntile = (n + kKnnQ - 1) / kKnnQ;
   return launch_knn(A, DP, ntile, smem, st);
@@ -1260,7 +1379,10 @@ extern "C" int sv_knn_query(const double* Xref, int64_t nref, const double* Xq, 
   A.nbr = nullptr;
   A.b0 = 0;
   A.ldnbr = 0;
-  if (kt_use(k, nref, nq, DP)) return launch_knn_tree(A, DP, (char*)Br + al256(sizeof(float) * (size_t)nref), st);
+  A.sel = nullptr;
+  A.sel_max = 0;
+  A.sel_tree = 0;
+  if (kt_query(k, nref, nq, d)) return launch_knn_tree(A, DP, (char*)Br + al256(sizeof(float) * (size_t)nref), st);
   const int64_t ntile = (nq + kKnnQ - 1) / kKnnQ;
   return launch_knn(A, DP, ntile, smem, st);
 }
