@@ -1238,14 +1238,20 @@ int launch_knn_batched(int DP, const KnnBatchProb* probs, const int2* tiles, int
 
 using namespace sv;
 
-extern "C" size_t sv_ordered_knn_workspace_bytes(int64_t n, int32_t d) {
+// centre, images and bounds of one set of rows
+static size_t knn_set_bytes(int64_t n, int d) {
   const int DP = pad_dim(d > 0 ? d : 1);
   return al256(sizeof(double) * 64) + al256(sizeof(float) * (size_t)(n > 0 ? n : 1) * DP) +
-         al256(sizeof(float) * (size_t)(n > 0 ? n : 1)) + kt_bytes(n, d > 0 ? d : 1, DP);
+         al256(sizeof(float) * (size_t)(n > 0 ? n : 1));
+}
+
+// (the tree is over the reference rows, which are an ordered search's own)
+extern "C" size_t sv_ordered_knn_workspace_bytes(int64_t n, int32_t d) {
+  return knn_set_bytes(n, d) + kt_bytes(n, d > 0 ? d : 1, pad_dim(d > 0 ? d : 1));
 }
 
 extern "C" size_t sv_knn_query_workspace_bytes(int64_t nref, int64_t nq, int32_t d) {
-  return sv_ordered_knn_workspace_bytes(nref, d) + sv_ordered_knn_workspace_bytes(nq, d);
+  return sv_ordered_knn_workspace_bytes(nref, d) + knn_set_bytes(nq, d);
 }
 
 static int knn_smem_ok(int DP, int k, size_t* smem) {
