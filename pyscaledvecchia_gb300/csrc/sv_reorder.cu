@@ -288,11 +288,8 @@ __device__ __forceinline__ void mc_screen(const McSmem& M, const float* Un, cons
 #pragma unroll
       for (int x = 0; x < 4; ++x)
         for (unsigned m = bits[x]; m; m &= m - 1, ++at) {
-          const unsigned e = (unsigned)(r0 + g + 8 * x) << 5 | (unsigned)(__ffs(m) - 1);
-          if (at < kMcQueue)
-            queue[at] = e;
-          else
-            mc_update(M, slot, e, Sc, d, growth);  // the queue is full
+          if (at < kMcQueue)  // (else the pass takes all pairs)
+            queue[at] = (unsigned)(r0 + g + 8 * x) << 5 | (unsigned)(__ffs(m) - 1);
         }
     }
   }
@@ -313,9 +310,20 @@ __device__ __forceinline__ void mc_apply(const McSmem& M, const float* Un, const
   else
     mc_screen<4>(M, Un, Ue, slot, qn, k, S, Sc, d, growth);
   __syncthreads();
-  const int nq = min(*qn, kMcQueue);
-  const unsigned* queue = reinterpret_cast<const unsigned*>(M.pairS);
-  for (int e = threadIdx.x; e < nq; e += blockDim.x) mc_update(M, slot, queue[e], Sc, d, growth);
+  const int nq = *qn;
+  if (nq <= kMcQueue) {
+    const unsigned* queue = reinterpret_cast<const unsigned*>(M.pairS);
+    for (int e = threadIdx.x; e < nq; e += blockDim.x) mc_update(M, slot, queue[e], Sc, d, growth);
+  } else {
+    // images that bf16 cannot tell apart, or the first passes: every pair meets
+    // the float32 screen, a thread its points (one lane's pairs at a time, where
+    // the queue was full, took 4.9 ms for 5,000 rows of a cluster and 52 rows
+    // 1e6 times further out, this 3.5)
+    for (int p = threadIdx.x; p < S; p += blockDim.x) {
+      if (__double_as_longlong(M.dist[p]) < 0) continue;  // ordered
+      for (int t = 0; t < k; ++t) mc_update(M, slot, (unsigned)p << 5 | (unsigned)t, Sc, d, growth);
+    }
+  }
   __syncthreads();
 }
 
