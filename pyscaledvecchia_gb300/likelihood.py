@@ -255,19 +255,22 @@ class DeviceProblem:
         cta = self.nblk > self.nblk_warp
         split = (precision in _SPLIT and split_nu(nu, estimate_nu)
                  and self.d + 3 + self.q <= 32)
-        n = (1 if warp else 0) + (1 if cta else 0)
-        if (not split and warp and not estimate_nu and float(nu) in (1.5, 2.5) and self.d <= 12
-                and self.d + 2 + self.q <= 32):
-            n += 1  # the fixed-point kernel, then the float64 kernels over what it flagged
+        # descriptor, status, parameters; the four reduction kernels
+        n = 3 + 4
         if estimate_nu or matern_table_nu(nu):
             n += 2 if split else 1  # the Matern tables: float64, and float32 for the split kernels
-        if split and warp:
-            n += 1  # coordinate pre-pass
-        if chunked:
-            n += 1 + (1 if warp else 0) + (1 if cta else 0)
-        if split and warp:
-            n += 1  # float64 re-evaluation of flagged blocks
-        return n + 2 + 4  # status/parameter set-up, then the four reduction kernels
+        if warp:
+            n += 2  # the float64 kernels, a half and a whole warp per block: all blocks, or those flagged
+            if split:
+                n += 2  # coordinate pre-pass, split kernel
+            elif (not estimate_nu and float(nu) in (1.5, 2.5) and self.d <= 12
+                    and self.d + 2 + self.q <= 32):
+                n += 1  # the fixed-point kernel
+        if cta:
+            n += 1
+        if chunked and self.nblk:
+            n += 1 + (1 if warp else 0) + (1 if cta else 0)  # chunks' jitter levels, their re-evaluation
+        return n
 
     def chunk_tensor(self, Pc):
         """Chunk of every block (chunk_ids), computed on the device from the
