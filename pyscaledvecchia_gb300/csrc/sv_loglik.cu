@@ -952,7 +952,9 @@ __device__ __forceinline__ double red2_lanes(double v, int o = 16) {
   return v;
 }
 
-template <int PR>
+// ALL: more than PR parameters, PR at a time (a kernel of its own: the loop
+// costs 10 us at 200,000 blocks, d = 10)
+template <int PR, bool ALL>
 __global__ void __cluster_dims__(kRedCl, 1, 1) k_reduce2(RedArgs R) {
   cg::cluster_group cl = cg::this_cluster();
   const int rank = (int)cl.block_rank();
@@ -971,7 +973,7 @@ __global__ void __cluster_dims__(kRedCl, 1, 1) k_reduce2(RedArgs R) {
   int64_t b0, b1;
   red_range(PI, parts, part, rank, b0, b1);
   const int w = threadIdx.x >> 5, nw = blockDim.x >> 5, ln = threadIdx.x & 31;
-  for (int p0 = 0; p0 == 0 || p0 < np; p0 += PR) {
+  for (int p0 = 0; p0 == 0 || (ALL && p0 < np); p0 += PR) {
     double acc[PR + 1];
     red2_sum<PR>(R, q, P, p0, sbeta, b0 + threadIdx.x, b1, blockDim.x, acc);
     // acc[1 + t] is parameter p0 + t, acc[0] the sum of z_K^2 (first time)
@@ -1460,7 +1462,8 @@ int run_eval(const EvalCall& C, cudaStream_t st, const ShardStage* sh = nullptr)
       const bool wide = S.nblk_max <= 4096 * 1024;
       const int thr = cta ? kRedThreads : wide ? std::max(32, (int)((run + 31) / 32 * 32)) : 32;
       auto kern = cta ? (S.Pmax <= 8 ? k_reduce2_cta<8> : k_reduce2_cta<16>)
-                      : S.Pmax <= 8 ? k_reduce2<8> : k_reduce2<16>;
+                      : S.Pmax <= 8 ? k_reduce2<8, false>
+                      : S.Pmax <= 16 ? k_reduce2<16, false> : k_reduce2<16, true>;
       kern<<<rgrid, thr, 0, st>>>(R);
       SV_CUDA_TRY(cudaGetLastError());
     }
