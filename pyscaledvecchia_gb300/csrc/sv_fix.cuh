@@ -6,10 +6,12 @@
 // GB300 issues a float64 warp instruction every 64 cycles per scheduler and a
 // 32 x 32 + 64 bit integer multiply-add every 4 (both measured). A product of
 // two split numbers accumulated over a sum takes three of the latter: h h'
-// into one 64-bit accumulator, h l' + l h' into another (l l' lies below
-// 2^-60 and is left out). So a multiply-add costs 12 cycles instead of 64, its
-// accumulation is exact, and the one rounding per sum, 2^-58 of the scale, is
-// 32 times finer than float64's at that scale. Correlations, their Cholesky
+// into one 64-bit accumulator, h l' + l h' into another; l l', at most 2^-58 and
+// a third of that in the root mean square, is left out (where that adds up with one
+// sign or is magnified it is not: pivots, distances, back substitutions). So a
+// multiply-add costs 12 cycles instead of 64, the rest of its accumulation is
+// exact, and a sum of K products is off by some sqrt(K) / 3 units of 2^-58 of
+// the scale and one rounding, where float64 rounds every term to 2^-53 of it. Correlations, their Cholesky
 // factor and the whitened columns are bounded by construction, so the scale is
 // known; what is not is rescaled or left to the float64 kernels.
 //

@@ -1320,7 +1320,7 @@ int run_eval(const EvalCall& C, cudaStream_t st, const ShardStage* sh = nullptr)
   if (split && lanes != 4 && lanes != 8 && lanes != 16 && lanes != 32) return SV_EINVAL;
 
   // float64 form: the fixed-point kernel first where a problem may be its
-  // (10.2 ms against 27.3 ms for the float64 kernels, measured at 200,000
+  // (11.2 ms against 27.3 ms for the float64 kernels, measured at 200,000
   // blocks of 31, d = 10), then the float64 kernels over the blocks it flagged
   const bool fix = !split && S.fix;
 

@@ -28,13 +28,18 @@
 //     it takes as many multiply-adds);
 //   * rows of T, right-hand sides and solutions carry power-of-two scales.
 //
-// Measured at n = 200,000, d = 10, m = 30: 10.2 ms, where k_block_warp takes
-// 27.3 ms; the integer multiply pipe is 65 % busy, the float64 pipe 6 %
-// (3 warps per scheduler, one block of 18 KB of shared memory each). Errors
-// against 64-bit-mantissa long double at n = 4,000, m = 30 (float64 kernels in
-// brackets): tau = 1e-4, d = 4: log-likelihood 2e-14 (1.6e-13), score 3e-14
-// (1.9e-13), Fisher 4e-15 (5e-14); tau = 1e-8, d = 3: 4e-12 (7e-10), 2e-11
-// (1.4e-9), 1.5e-11 (4.7e-10).
+// Measured at n = 200,000, d = 10, m = 30: 11.2 ms (d = 8: 9.6, d = 12: 11.8), where
+// k_block_warp takes 27.3 ms; the integer multiply pipe is 61 to 65 % busy, the
+// float64 pipe 6 % (3 warps per scheduler, one block of 17 KB of shared memory
+// each; at 200,000 blocks a tenth of the warps' waits are for instructions).
+//
+// Errors against binary128 (float64 kernels in brackets), n = 240, m = 30, rows
+// evenly spread, in clusters of six 0.02 ranges across, or three times each,
+// reaching 0.5 to 30 ranges, tau = 1e-8 to 0.1, d = 3 and 8: log-likelihood, score
+// and Fisher as close as the float64 kernels' or closer, but for single results
+// of 1e-16 to 1e-15; clusters, d = 3, 10 ranges, tau = 1e-8: log-likelihood 1e-13
+// (3e-12), score 2e-12 (3e-11), Fisher 3e-12 (7e-11). n = 200,000, d = 10, tau =
+// 3e-3: log-likelihood 4e-17 (4e-15).
 //
 // What has no such bound goes to the float64 kernels: a block with a pivot
 // below 2^-34 of the diagonal (its jitter ladder is theirs), coordinates

@@ -286,10 +286,14 @@ extern "C" int sv_predict_blocks(const sv_pred_desc* D, const double* theta, con
   cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   const size_t prm = (sizeof(PredPrm) + 7) / 8 * 8;
   const int nsm = sv_num_sms();
-  // the fixed-point kernel takes nu = 3/2 and 5/2 and every split call (20,000
-  // blocks of 141, d = 6: 17.9 ms against k_pred_cta's 37.0; 9,001 split blocks
-  // of 141, d = 7: 7.2 against 10.6), beyond 32 points a block: 20,000 calls of
-  // 21 points take 5.3 ms with a warp each and 5.6 with a CTA each
+  // the fixed-point kernel takes nu = 3/2 and 5/2, and split calls whose pivot
+  // guard is at least 1e-9, of 33 to 208 points a block, d <= 12 and what shared
+  // memory holds (20,000 blocks of 141, d = 6: 18.6 ms against k_pred_cta's 37.0;
+  // 9,001 split blocks of 141, d = 7: 7.2 against 10.6; 3,000 of 36, d = 6: 0.37
+  // against 0.58, split 0.30 against 0.47). Up to two blocks per SM of fewer than
+  // 60 points take 5 to 20 us longer than there, so that a block's bits do not
+  // depend on how many there are. 20,000 calls of 21 points take 5.3 ms
+  // with a warp each and 5.6 with a CTA each
   A.kt = D->k + 1;
   if (pred_fix_takes(A, maxsm)) return launch_pred_fix(A, maxsm, st);
   if (D->k + 1 <= 32) {

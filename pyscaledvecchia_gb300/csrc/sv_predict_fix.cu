@@ -5,7 +5,7 @@
 // scheduler): K^3/6 multiply-adds of the LDL^T and, in the float64 form, a
 // distance, a square root and an exponential per entry. Here the block's
 // covariance is scaled to a diagonal in (1/2, 1] (its Cholesky factor is then
-// bounded by 1) and factored in integers, three 2-cycle multiply-adds for one
+// bounded by 1) and factored in integers, three 4-cycle multiply-adds for one
 // of float64's; the entries come from fx_matern_norm (float64 form, nu = 3/2 and
 // 5/2) or, as before, from the float32 deficits (split form).
 //
