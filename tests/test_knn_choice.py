@@ -11,7 +11,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("ranges", ["one", "spread"])  # the screens, the tree
 @pytest.mark.parametrize("n,d,m,start", [(32768, 10, 5, 0), (33001, 16, 20, 0), (33000, 12, 50, 0), (32769, 9, 16, 0),
-                                         (66000, 11, 30, 60000), (33000, 13, 15, 32990)])
+                                         (66000, 11, 30, 60000), (33000, 13, 15, 32990),
+                                         (66000, 16, 20, 65900)])
 def test_ordered(oracle, ranges, n, d, m, start):
     from pyscaledvecchia_gb300 import find_ordered_nn
     rng = np.random.default_rng(n + d)
